@@ -479,8 +479,7 @@ static int run_doubling(Ctx* c, Work& w, uint32_t ndbl, cudaStream_t st, pssgpu_
     const uint64_t memb = (uint64_t)hc[C_DBL_MEMB] | ((uint64_t)hc[C_DBL_MEMB + 1] << 32);
     c->kstat[K_DBL].alg_bytes += 8ull * n + 16ull * memb;
     if (!*err && a.lb) {
-        const uint64_t nchunk = ((uint64_t)n + DBL_LCP_CHUNK - 1) / DBL_LCP_CHUNK;
-        k_dbl_lcp<<<(unsigned)std::min<uint64_t>((nchunk + 255) / 256, 148ull * 16), 256, 0, st>>>(
+        k_dbl_lcp<<<(unsigned)std::min<uint64_t>(((uint64_t)n + 255) / 256, 148ull * 16), 256, 0, st>>>(
             w.chars, w.nchars, w.perm, a.isa, a.lb, w.lcp, n);
         stats.kernel_launches += 1;
         c->kstat[K_DBL].launches += 1;
