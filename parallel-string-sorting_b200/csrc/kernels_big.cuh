@@ -40,12 +40,16 @@ __device__ __forceinline__ int find_tile_seg(const uint32_t* tile_start, int nbi
 
 __device__ __forceinline__ uint32_t tree_bits_for(const Work& w, uint32_t m)
 {
-    // a tuned value for this size class, else about 8 strings per '<'
-    // bucket; at most pS5's 10 tree levels
+    // a tuned value for this size class, else about 128 strings per '<'
+    // bucket, which the leaf sorters finish for less than finer splitting
+    // costs (64 Mi prefix sort: 7.63 ms at 8 strings, 7.51 at 64, 7.41 at
+    // 128, 7.48 at 256; 613-instance batch: 535, 496, 478, 478 us); a suffix
+    // set's buckets go on to rank doubling, at about 8. At most pS5's 10 tree
+    // levels.
     const int lg = 31 - __clz((int)m);
     const uint32_t tuned = w.tree_bits_by_size[lg];
     if (tuned) return min((uint32_t)MAX_TREE_BITS, tuned);
-    return (uint32_t)min(MAX_TREE_BITS, max(1, lg - 3));
+    return (uint32_t)min(MAX_TREE_BITS, max(1, lg - (w.suffix ? 3 : 7)));
 }
 
 __global__ void k_tile_scan(Work w, uint32_t nbig)
@@ -575,65 +579,6 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) k_scatter(Work w, uint32_t nb
     }
 }
 
-__device__ __forceinline__ void push_seg(Work& w, int nxt, Seg c)
-{
-    int cls;
-    if (c.size > SMALL_MAX) cls = L_BIG;
-    else if (c.size > 256) cls = L_SMALLB;
-    else if (c.size > WARP_GROUP_MAX) cls = L_SMALLA;
-    else cls = L_TINY;
-    const uint32_t at = atomicAdd(w.counters + C_PAR * nxt + cls, 1u);
-    if (at >= w.cap[cls]) {
-        set_error(w.counters + C_ERR, ERR_OVERFLOW);
-        return;
-    }
-    w.list[cls][nxt][at] = c;
-    if (cls == L_BIG) {
-        const uint32_t tiles = (c.size + TILE - 1) / TILE;
-        atomicAdd(w.counters + C_PAR * nxt + C_NTILES, tiles);
-        if (tiles > (uint32_t)CHUNK) atomicAdd(w.counters + C_MULTI + nxt, 1u);
-    } else {
-        atomicAdd(w.counters + C_PAR * nxt + C_NSTR + cls, c.size);
-    }
-}
-
-// push_seg for a whole warp: lanes with push set append c. One reservation
-// per class and warp, and the class's tile or string count added once (a
-// launch that pushes many segments would otherwise serialise on these few
-// counters).
-__device__ __forceinline__ void push_seg_warp(Work& w, int nxt, bool push, const Seg& c)
-{
-    const uint32_t lane = threadIdx.x & 31;
-    int cls = -1;
-    if (push)
-        cls = c.size > SMALL_MAX ? L_BIG : c.size > 256 ? L_SMALLB : c.size > WARP_GROUP_MAX ? L_SMALLA : L_TINY;
-#pragma unroll
-    for (int k = 0; k < L_NCLASS; ++k) {
-        const uint32_t m = __ballot_sync(0xffffffffu, cls == k);
-        if (!m) continue;
-        const int leader = __ffs(m) - 1;
-        const uint32_t tiles = cls == k && k == L_BIG ? (c.size + TILE - 1) / TILE : 0u;
-        const uint32_t amount = __reduce_add_sync(0xffffffffu, cls != k ? 0u : k == L_BIG ? tiles : c.size);
-        const uint32_t multi = __reduce_add_sync(0xffffffffu, tiles > (uint32_t)CHUNK ? 1u : 0u);
-        uint32_t base = 0;
-        if (lane == (uint32_t)leader) {
-            base = atomicAdd(w.counters + C_PAR * nxt + k, (uint32_t)__popc(m));
-            if (k == L_BIG) {
-                atomicAdd(w.counters + C_PAR * nxt + C_NTILES, amount);
-                if (multi) atomicAdd(w.counters + C_MULTI + nxt, multi);
-            } else {
-                atomicAdd(w.counters + C_PAR * nxt + C_NSTR + k, amount);
-            }
-        }
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (cls == k) {
-            const uint32_t at = base + __popc(m & ((1u << lane) - 1u));
-            if (at >= w.cap[k]) set_error(w.counters + C_ERR, ERR_OVERFLOW);
-            else w.list[k][nxt][at] = c;
-        }
-    }
-}
-
 // Children of each bucket, after the scatter has placed them (hpp:1492-1584):
 // '<' buckets keep their depth and keys, '=' buckets go 8 chars deeper or
 // are finished when their splitter ends the string. Behind a common-prefix
@@ -711,10 +656,7 @@ __global__ void __launch_bounds__(1024) k_children(Work w)
                     child = Seg{P, c, dj, (uint32_t)nbuf | META_VALID};
                 }
                 if (!inline_done) {
-                    if (c > SMALL_MAX) cls = L_BIG;
-                    else if (c > 256) cls = L_SMALLB;
-                    else if (c > WARP_GROUP_MAX) cls = L_SMALLA;
-                    else cls = L_TINY;
+                    cls = seg_class(w, c);
                     slot = atomicAdd(&lcnt[cls], 1u);
                     if (cls == L_BIG) {
                         const uint32_t tiles = (c + TILE - 1) / TILE;

@@ -1,4 +1,5 @@
-// kernels_block.cuh -- block sample sort for segments of 33..MAXN strings.
+// kernels_block.cuh -- block sample sort for segments of 33..MAXN strings: the
+// last phase of k_wave and the allocation-free entry point.
 //
 // One block runs pS5's sequential sample-sort step (SeqSampleSortStep,
 // src/parallel/bingmann-parallel_sample_sort.hpp:565-676) on its segment in
@@ -317,8 +318,6 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 64 ? 20 : 4) k_block(Work 
     block_sort_groups<MAXN, THREADS>(w, sm, begin, m, buf, wscratch, err);
 }
 
-#define K_BLOCK_A k_block<SMALL_A, SMALL_A_THREADS>
-#define K_BLOCK_B k_block<SMALL_MAX, SMALL_THREADS>
 // the allocation-free entry point's sorter: up to 2048 strings in one block
 #define K_BLOCK_NOALLOC k_block<2048, 256>
 

@@ -1,0 +1,758 @@
+// kernels_leaf.cuh -- finishing of the segments the sample-sort passes do not
+// split any further, at most SMALL_MAX strings, by sorting networks in
+// registers. The device counterpart of pS5's base cases on 8-byte caches
+// (sort_mkqs_cache / insertion_sort_cache, src/parallel/
+// bingmann-parallel_sample_sort.hpp:805-861, 1056-1178) and its sequential
+// sample sort (hpp:565-676).
+//
+// A string is one 64-bit word while it is sorted: its key, shifted left past
+// the bits that all keys of the segment share, over the string's index in the
+// segment. Words are distinct, their order is the key order, and the index
+// says where the string came from, so a compare-exchange moves one register
+// pair and no payload. When the shared bits leave no room for the index, the
+// word holds the first 7 (or 6) chars of the key only, and ties in those
+// continue at that depth.
+//
+//   k_tiny      2..32 strings: one thread per segment, Batcher's odd-even
+//               merge network over its 8, 16 or 32 registers
+//   k_segs<1>   33..256 strings: one warp per segment, 2, 4 or 8 words a lane
+//   k_segs<4>   257..1024 strings: a block of 4 warps
+//   k_segs<16>  1025..4096 strings: a block of 16 warps
+//
+// All are bound by instructions (12 to 17 warp instructions per string).
+// Measured in the 64 Mi prefix sort, 67 M strings: 27, 32, 32 and 62 ps per
+// string. Sample-sort steps in shared memory with a warp window per 32
+// strings took 30 ps (2..32 strings), 66 (33..256) and 67 (257..1024), and
+// segments of 1025..4096 strings one more sample-sort pass (about 42 ps)
+// before them: 9.29 -> 7.42 ms per sort; 100k-instance batch 3.86 -> 2.48 ms.
+//
+// Strings whose whole words tie and do not end go to warp windows
+// (kernels_small.cuh), up to 32 strings of several groups at a time; larger
+// tied groups are sorted again by their warp, behind their common prefix.
+#pragma once
+
+#include <utility>
+
+#include "kernels_small.cuh"
+
+namespace pssgpu {
+
+__device__ __forceinline__ void cmp_exchange(uint64_t& a, uint64_t& b)
+{
+    const bool s = b < a;
+    const uint64_t lo = s ? b : a;
+    b = s ? a : b;
+    a = lo;
+}
+
+__device__ __forceinline__ void cmp_exchange(uint32_t& a, uint32_t& b)
+{
+    const uint32_t lo = min(a, b);
+    b = max(a, b);
+    a = lo;
+}
+
+// Batcher's odd-even merge sorting network for N (a power of two) inputs:
+// 19 compare-exchanges for 8, 63 for 16, 191 for 32.
+template <int N>
+struct OddEvenNet {
+    int a[N * N / 4 + N] = {};
+    int b[N * N / 4 + N] = {};
+    int size = 0;
+    constexpr OddEvenNet()
+    {
+        for (int p = 1; p < N; p *= 2)
+            for (int k = p; k >= 1; k /= 2)
+                for (int j = k % p; j + k < N; j += 2 * k)
+                    for (int i = 0; i < k && i + j + k < N; ++i)
+                        if ((i + j) / (2 * p) == (i + j + k) / (2 * p)) {
+                            a[size] = i + j;
+                            b[size] = i + j + k;
+                            ++size;
+                        }
+    }
+};
+
+template <int N, int I>
+__device__ __forceinline__ void net_step(uint32_t (&x)[N])
+{
+    constexpr OddEvenNet<N> net{};
+    constexpr int a = net.a[I], b = net.b[I];
+    cmp_exchange(x[a], x[b]);
+}
+
+template <int N, int... I>
+__device__ __forceinline__ void net_run(uint32_t (&x)[N], std::integer_sequence<int, I...>)
+{
+    (net_step<N, I>(x), ...);
+}
+
+template <int N>
+__device__ __forceinline__ void net_sort(uint32_t (&x)[N])
+{
+    constexpr OddEvenNet<N> net{};
+    net_run<N>(x, std::make_integer_sequence<int, net.size>{});
+}
+
+// Barrier of the G warps that sort a segment together (G > 1: a whole block).
+template <int G>
+__device__ __forceinline__ void group_sync()
+{
+    if constexpr (G == 1) __syncwarp();
+    else __syncthreads();
+}
+
+// Ascending bitonic sort of 32 * E * G words held by G warps (G > 1: a block
+// of 32 * G threads), position t * E + e in x[e] of thread t afterwards.
+// Every merge starts by comparing positions with their mirror in the merged
+// block, so all compares are ascending. Partner distances below E stay
+// inside a thread, those inside a warp are shuffles, longer ones go through
+// xb (32 * E * G words of shared memory, G > 1 only).
+template <int E, int G>
+__device__ __forceinline__ void group_sort(uint64_t (&x)[E], uint64_t* xb)
+{
+    constexpr uint32_t T = 32 * G;
+    const uint32_t t = G == 1 ? threadIdx.x & 31 : threadIdx.x;
+    auto inner = [&](int j) {  // distances j, j/2, .., 1 inside the threads
+#pragma unroll
+        for (int d = E / 2; d > 0; d >>= 1) {
+            if (d > j) continue;
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+                if (!(e & d)) cmp_exchange(x[e], x[e + d]);
+        }
+    };
+    auto publish = [&]() {
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < E; ++e) xb[e * T + t] = x[e];
+        __syncthreads();
+    };
+#pragma unroll
+    for (int k = 2; k <= E; k <<= 1) {
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+            if (!(e & (k >> 1))) cmp_exchange(x[e], x[e ^ (k - 1)]);
+        inner(k / 4);
+    }
+    // merges of 2, 4, .. 32 * G threads
+#pragma unroll 1
+    for (uint32_t k = 2; k <= T; k <<= 1) {
+        const bool lower = (t & (k >> 1)) == 0;
+        if (G == 1 || k <= 32) {
+#pragma unroll
+            for (int e = 0; e < E / 2; ++e) {
+                const uint64_t y0 = __shfl_xor_sync(0xFFFFFFFFu, x[E - 1 - e], k - 1);
+                const uint64_t y1 = __shfl_xor_sync(0xFFFFFFFFu, x[e], k - 1);
+                if ((y0 < x[e]) == lower) x[e] = y0;
+                if ((y1 < x[E - 1 - e]) == lower) x[E - 1 - e] = y1;
+            }
+        } else {
+            publish();
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const uint64_t y = xb[(E - 1 - e) * T + (t ^ (k - 1))];
+                if ((y < x[e]) == lower) x[e] = y;
+            }
+        }
+        uint32_t j = k >> 2;
+        if (G > 1) {
+#pragma unroll 1
+            for (; j >= 32; j >>= 1) {
+                const bool low = (t & j) == 0;
+                publish();
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    const uint64_t y = xb[e * T + (t ^ j)];
+                    if ((y < x[e]) == low) x[e] = y;
+                }
+            }
+        }
+#pragma unroll 1
+        for (; j > 0; j >>= 1) {
+            const bool low = (t & j) == 0;
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const uint64_t y = __shfl_xor_sync(0xFFFFFFFFu, x[e], j);
+                if ((y < x[e]) == low) x[e] = y;
+            }
+        }
+        inner(E / 2);
+    }
+}
+
+// The words of a segment (or tied group): IB index bits below the key's
+// chars. x is the OR of its keys' differences from key0, not 0.
+template <int IB>
+struct WordForm {
+    uint64_t key0;
+    int cp;      // bits all keys share
+    int chars;   // chars of the key in the word: 8, or 7 / 6 when the index takes their place
+    __device__ __forceinline__ WordForm(uint64_t k0, uint64_t x) : key0(k0)
+    {
+        cp = __clzll((long long)x);
+        chars = cp >= IB ? 8 : IB <= 8 ? 7 : 6;
+        static_assert(IB <= 16, "6 chars leave 16 bits");
+    }
+    __device__ __forceinline__ uint64_t make(uint64_t key, uint32_t i) const
+    {
+        return ((key & (~0ull << (64 - 8 * chars))) << cp) | i;
+    }
+    // do two words hold the same chars?
+    __device__ __forceinline__ static bool same(uint64_t a, uint64_t b) { return ((a ^ b) >> IB) == 0; }
+    // chars shared by two words that differ
+    __device__ __forceinline__ uint32_t lcp(uint64_t a, uint64_t b) const
+    {
+        return (uint32_t)(cp + __clzll((long long)(a ^ b))) >> 3;
+    }
+    __device__ __forceinline__ uint64_t key(uint64_t word) const
+    {
+        return ((word & (~0ull << IB)) >> cp) | (cp ? key0 & (~0ull << (64 - cp)) & (~0ull << (64 - 8 * chars)) : 0ull);
+    }
+    // do strings with this key (key()'s value) end inside the word's chars?
+    __device__ __forceinline__ bool ended(uint64_t k) const { return ((k >> (64 - 8 * chars)) & 0xFF) == 0; }
+};
+
+// Runs of tied strings (at most 32 each) into warp windows of up to 32
+// strings. Each lane brings runs one after another: next(start, len) gives
+// its next one or returns false. fn(owner, start, gs) runs on every lane of a
+// window: the lane whose run the slot belongs to, the run's start and the
+// slot its run starts at (32: an unused slot). scratch: 32 words of the warp.
+template <typename Next, typename Fn>
+__device__ __forceinline__ void tie_windows(uint32_t* scratch, Next next, Fn fn)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t start = 0, len = 0;
+    bool has = next(start, len);
+    while (__any_sync(0xFFFFFFFFu, has)) {
+        const uint32_t end = warp_incl_sum(has ? len : 0u);
+        const bool take = has && end <= 32u;
+        const uint32_t at = end - len;
+        const uint32_t starts = __reduce_or_sync(0xFFFFFFFFu, take ? 1u << at : 0u);
+        const uint32_t used = __reduce_max_sync(0xFFFFFFFFu, take ? end : 0u);
+        if (take) scratch[at] = lane;
+        __syncwarp();
+        const bool real = lane < used;
+        const uint32_t gs = 31u - __clz(starts & (0xFFFFFFFFu >> (31 - lane)));
+        const uint32_t owner = scratch[gs];
+        __syncwarp();
+        fn(owner, __shfl_sync(0xFFFFFFFFu, start, owner), real ? gs : 32u);
+        if (take) has = next(start, len);
+    }
+}
+
+// ---- 2..32 strings ----------------------------------------------------------
+// A block takes up to TINY_THREADS list entries, orders them by network size so
+// that the threads of a warp run the same one, and each warp stages the keys
+// of its segments in shared memory (rows of 32 positions across segments,
+// coalesced), sorts one segment per thread, and writes perm and LCPs in rows
+// again. At most TINY_ROWS rows at a time: two halves of the warp in turn
+// when its segments hold more.
+//
+// The network runs on 32-bit words, the 27 bits behind the bits all keys of
+// the segment share over a 5-bit index: a compare-exchange is a min and a
+// max, and the three networks are small enough to stay in the instruction
+// cache (with 64-bit words they were not, and the registers halved the
+// warps: 1.8 ms instead of 0.85 ms for the 28 M strings of this class in the
+// 64 Mi prefix sort at 8 strings per bucket). Neighbours that tie in 27 bits
+// are put in order by their whole keys in shared memory.
+constexpr int TINY_THREADS = 256;
+constexpr int TINY_ROWS = 16;
+
+struct TinyWarp {
+    uint64_t key[32 * TINY_ROWS];
+    uint32_t lcp[32 * TINY_ROWS];
+    uint8_t idx[32 * TINY_ROWS];
+    uint4 seg[32];               // base, first row entry, meta, depth (then ties) per lane
+    uint32_t starts[TINY_ROWS];  // per row: positions where a segment starts
+    uint32_t scratch[32];
+};
+
+// The warp's segments, one per lane (sg.size 0: none; packed from lane
+// `first` on), `total` strings from row entries `off`; N the network. Sorts
+// and writes them.
+template <int N>
+__device__ __forceinline__ void tiny_warp_sort(const Work& w, TinyWarp& sm, const Seg& sg, uint32_t first,
+                                               uint32_t off, uint32_t total)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t base = sg.begin - off;  // row entry f of the segment: position base + f
+    sm.seg[lane] = make_uint4(base, off, sg.meta, sg.depth);
+    if (lane < TINY_ROWS) sm.starts[lane] = 0;
+    __syncwarp();
+    if (sg.size) atomicOr(&sm.starts[off >> 5], 1u << (off & 31));
+    __syncwarp();
+    const uint32_t mask = lane < TINY_ROWS ? sm.starts[lane] : 0u;
+    const uint32_t count = __popc(mask);
+    const uint32_t before = first + warp_incl_sum(count) - count;  // segments before row `lane`
+    // lane of the segment that row r's entry at this lane belongs to
+    auto row_seg = [&](uint32_t r) {
+        const uint32_t m = __shfl_sync(0xFFFFFFFFu, mask, r & 15);
+        const uint32_t b = __shfl_sync(0xFFFFFFFFu, before, r & 15);
+        return (b + __popc(m & (0xFFFFFFFFu >> (31 - lane))) - 1) & 31;
+    };
+    constexpr uint32_t U = 4;  // rows in flight
+    for (uint32_t r0 = 0; 32 * r0 < total; r0 += U) {
+        uint64_t v[U];
+        uint4 q[U];
+        bool stale = false;
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) {
+            const uint32_t f = 32 * (r0 + u) + lane;
+            q[u] = sm.seg[row_seg(r0 + u)];
+            if (f >= total) continue;
+            const int buf = q[u].z & META_BUF;
+            const bool cached = q[u].z & META_VALID;
+            v[u] = (cached ? w.keys[buf] : w.hnd[buf])[q[u].x + f];
+            stale = stale || !cached;
+        }
+        if (stale) {
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u)
+                if (32 * (r0 + u) + lane < total && !(q[u].z & META_VALID)) v[u] = h_key(w, v[u], q[u].w);
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) {
+            const uint32_t f = 32 * (r0 + u) + lane;
+            if (f < total) sm.key[f] = v[u];
+        }
+    }
+    __syncwarp();
+    const uint64_t* key = sm.key + off;
+    uint8_t* idx = sm.idx + off;
+    uint32_t x[N];
+    const uint64_t key0 = key[0];  // an unused lane reads an entry and drops it
+    uint64_t diff = 1;             // equal keys: any shift does
+#pragma unroll
+    for (int i = 1; i < N; ++i)
+        if ((uint32_t)i < sg.size) diff |= key[i] ^ key0;
+    const int cp = __clzll((long long)diff);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        x[i] = 0xFFFFFFFFu;  // a real word is smaller, or has index 31 and no unused slot beside it
+        if ((uint32_t)i < sg.size) x[i] = ((uint32_t)((key[i] << cp) >> 32) & ~31u) | i;
+    }
+    net_sort<N>(x);
+    uint32_t near = 0;  // bit i: string i ties with string i - 1 in the word
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        if ((uint32_t)i < sg.size) {
+            idx[i] = (uint8_t)(x[i] & 31u);
+            if (i) {
+                const uint32_t df = (x[i] ^ x[i - 1]) >> 5;
+                if (!df) near |= 1u << i;
+                else if (w.lcp) sm.lcp[off + i] = sg.depth + ((uint32_t)(cp + __clz(df) - 5) >> 3);
+            }
+        }
+    }
+    uint32_t ties = 0;  // bit i: equal keys that do not end
+    if (near) {
+        for (uint32_t m = near; m; m &= m - 1) {  // insert the tied strings in order
+            uint32_t i = __ffs(m) - 1;
+            const uint8_t me = idx[i];
+            const uint64_t k = key[me];
+            while ((near >> i) & 1u) {
+                const uint8_t o = idx[i - 1];
+                if (key[o] <= k) break;
+                idx[i--] = o;
+            }
+            idx[i] = me;
+        }
+        for (uint32_t m = near; m; m &= m - 1) {
+            const uint32_t i = __ffs(m) - 1;
+            const uint64_t a = key[idx[i - 1]], b = key[idx[i]];
+            if (a == b && !key_terminated(b)) ties |= 1u << i;
+            else if (w.lcp) sm.lcp[off + i] = sg.depth + (a != b ? lcp_key_type(a, b) : lcp_key_depth(b));
+        }
+    }
+    sm.seg[lane].w = ties;
+    __syncwarp();
+    for (uint32_t r0 = 0; 32 * r0 < total; r0 += U) {
+        uint64_t h[U];
+        uint4 q[U];
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) {
+            const uint32_t f = 32 * (r0 + u) + lane;
+            q[u] = sm.seg[row_seg(r0 + u)];
+            if (f < total) h[u] = w.hnd[q[u].z & META_BUF][q[u].x + q[u].y + sm.idx[f]];
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) {
+            const uint32_t f = 32 * (r0 + u) + lane;
+            if (f >= total) continue;
+            w.perm[q[u].x + f] = h_id(w, h[u]);
+            const uint32_t i = f - q[u].y;
+            if (w.lcp && i && !((q[u].w >> i) & 1u)) w.lcp[q[u].x + f] = sm.lcp[f];
+        }
+    }
+    if (!__any_sync(0xFFFFFFFFu, ties)) return;
+    __syncwarp();
+    tie_windows(
+        sm.scratch,
+        [&](uint32_t& start, uint32_t& len) {
+            if (!ties) return false;
+            const uint32_t i = __ffs(ties) - 1;  // >= 1
+            const uint32_t rest = ~(ties >> i);
+            const uint32_t ones = __ffs(rest) - 1;  // at most 31: bit 0 is never set
+            start = i - 1;
+            len = ones + 1;
+            ties &= i + ones >= 32 ? 0u : ~0u << (i + ones);
+            return true;
+        },
+        [&](uint32_t owner, uint32_t start, uint32_t gs) {
+            const bool real = gs < 32;
+            const uint32_t o = __shfl_sync(0xFFFFFFFFu, off, owner);
+            const uint32_t bo = __shfl_sync(0xFFFFFFFFu, base, owner);
+            const uint32_t meta = __shfl_sync(0xFFFFFFFFu, sg.meta, owner);
+            const uint32_t dep = __shfl_sync(0xFFFFFFFFu, sg.depth + 8, owner);
+            const uint32_t f = o + start + (lane - gs);
+            const uint32_t pos = bo + f;
+            const uint64_t h = real ? w.hnd[meta & META_BUF][bo + o + sm.idx[f]] : ~0ull;
+            const uint64_t r = warp_window(w, h, gs, dep, pos, false, 0ull, sm.scratch);
+            if (real) w.perm[pos] = h_id(w, r);
+        });
+}
+
+__global__ void __launch_bounds__(TINY_THREADS, 3) k_tiny(Work w, const Seg* list, uint32_t count, uint32_t per)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TinyWarp* warps = reinterpret_cast<TinyWarp*>(smem_raw);
+    __shared__ Seg segs[TINY_THREADS];
+    __shared__ uint32_t cnt[3 * TINY_THREADS / 32];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t here = per * (TINY_THREADS / 32);  // entries of this block
+    const uint32_t g = threadIdx.x < here ? blockIdx.x * here + threadIdx.x : count;
+    Seg sg{};
+    if (g < count) sg = list[g];
+    // stable order by network: 9..16 strings behind those up to 8, and so on;
+    // unused threads last
+    const uint32_t cls = g >= count ? 3 : sg.size <= 8 ? 0 : sg.size <= 16 ? 1 : 2;
+    uint32_t below = 0;  // entries of this class in earlier lanes
+#pragma unroll
+    for (uint32_t c = 0; c < 3; ++c) {
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, cls == c);
+        if (lane == 0) cnt[c * (TINY_THREADS / 32) + warp] = __popc(m);
+        if (cls == c) below = __popc(m & ((1u << lane) - 1u));
+    }
+    segs[threadIdx.x] = Seg{};
+    __syncthreads();
+    static_assert(3 * TINY_THREADS / 32 <= 32, "one lane per class and warp");
+    const uint32_t mine = lane < 3 * TINY_THREADS / 32 ? cnt[lane] : 0u;
+    const uint32_t ahead = warp_incl_sum(mine) - mine;
+    const uint32_t at = __shfl_sync(0xFFFFFFFFu, ahead, (cls * (TINY_THREADS / 32) + warp) & 31) + below;
+    if (cls < 3) segs[at] = sg;
+    __syncthreads();
+    sg = lane < per ? segs[warp * per + lane] : Seg{};
+    const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, sg.size);
+    if (most == 0) return;  // whole warp
+    const uint32_t all = __reduce_add_sync(0xFFFFFFFFu, sg.size);
+    const uint32_t turns = all <= 32 * TINY_ROWS ? 1 : 2;
+    for (uint32_t t = 0; t < turns; ++t) {
+        Seg part = sg;
+        if (turns == 2 && (lane >> 4) != t) part.size = 0;
+        const uint32_t end = warp_incl_sum(part.size);
+        const uint32_t total = __shfl_sync(0xFFFFFFFFu, end, 31);
+        if (!total) continue;
+        const uint32_t off = part.size ? end - part.size : 0u;
+        if (most <= 8) tiny_warp_sort<8>(w, warps[warp], part, 16 * t, off, total);
+        else if (most <= 16) tiny_warp_sort<16>(w, warps[warp], part, 16 * t, off, total);
+        else tiny_warp_sort<32>(w, warps[warp], part, 16 * t, off, total);
+        __syncwarp();
+    }
+}
+
+// Entries per warp: fewer than 32 when that leaves SMs idle (a warp takes its
+// entries' loads and ties one after another).
+inline uint32_t tiny_per(uint32_t count)
+{
+    uint32_t per = 32;
+    while (per > 4 && count < per * (TINY_THREADS / 32) * 296u) per >>= 1;
+    return per;
+}
+constexpr size_t TINY_SMEM = sizeof(TinyWarp) * (TINY_THREADS / 32);
+
+// ---- 33..SMALL_MAX strings ------------------------------------------------------
+// G warps per segment of at most 256 G strings. hnd holds the segment's
+// handles as they came, idx the current order of positions; groups are sorted
+// from a stack (the segment first, then tied groups of more than 32 strings).
+constexpr int SEG_E = 8;  // most words a thread holds
+template <int G>
+struct alignas(16) SegState {
+    static constexpr int N = 32 * SEG_E * G;
+    static constexpr int IDX = N + N / 16;  // padded (idx_at)
+    static constexpr int LCP = N + N / 32;  // padded (lcp_at)
+    // G > 1: the sort's exchange buffer and the LCP staging share one array
+    static constexpr int TAIL = G > 1 ? 8 * N : 4 * LCP;
+    uint64_t hnd[N];
+    uint64_t last[G], key0, diff;
+    uint16_t idx[IDX];
+    uint32_t tied[N / 32];    // bit i: the string at i ties with the one before
+    uint32_t scratch[G][32];
+    uint16_t g_start[N / 32], g_len[N / 32];
+    uint32_t g_dep[N / 32];
+    uint32_t ng, jump, ntied;
+};
+
+// dynamic shared memory of a block that sorts `segs` segments at a time
+template <int G>
+constexpr size_t segs_smem(int segs, bool lcp)
+{
+    return (size_t)segs * (sizeof(SegState<G>) + (G > 1 || lcp ? SegState<G>::TAIL : 0));
+}
+
+// padded positions: a thread's consecutive entries start on another bank than
+// its neighbours'
+__device__ __forceinline__ uint32_t idx_at(uint32_t i) { return i + ((i >> 5) << 1); }
+__device__ __forceinline__ uint32_t lcp_at(uint32_t i) { return i + (i >> 5); }
+
+// Ties per warp beyond which a group hands its tied runs to the next pass
+// instead of sorting them in warp windows, or (runs over 32 strings) by all
+// its warps, one after another. Runs over LEAF_WINDOW_TIES * G stay: the
+// group's warps are not too many for them.
+constexpr uint32_t LEAF_WINDOW_TIES = 48;
+constexpr uint32_t LEAF_TIED = 0xFFFFFFFFu;  // LCP staging: not known yet
+
+// Sort the group of c strings (c <= 32 E G) at offset s of the segment, depth
+// d; with the segment's cached keys when `cached` (then s is 0). Tied groups
+// of more than 32 strings go to the stack, smaller ones to warp windows.
+template <int E, int G>
+__device__ __forceinline__ void sort_group(const Work& w, SegState<G>& sm, unsigned char* tail, uint32_t begin,
+                                           int buf, uint32_t s, uint32_t c, uint32_t d, bool cached)
+{
+    constexpr uint32_t T = 32 * G;
+    constexpr int NMAX = 32 * E * G;
+    constexpr int IB = NMAX == 64 ? 6 : NMAX == 128 ? 7 : NMAX == 256 ? 8 : NMAX == 512 ? 9 : NMAX == 1024 ? 10
+                     : NMAX == 2048 ? 11 : NMAX == 4096 ? 12 : 13;
+    static_assert(NMAX <= 1 << IB && IB <= 13, "index bits");
+    const uint32_t lane = threadIdx.x & 31, warp = G == 1 ? 0u : threadIdx.x >> 5;
+    const uint32_t t = 32 * warp + lane;
+    uint32_t* slcp = reinterpret_cast<uint32_t*>(tail);
+    uint64_t x[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint32_t j = t + T * e;
+        x[e] = 0;
+        if (j < c)
+            x[e] = cached ? __ldg(w.keys[buf] + begin + j) : h_key(w, sm.hnd[sm.idx[idx_at(s + j)]], d);
+    }
+    uint64_t key0 = __shfl_sync(0xFFFFFFFFu, x[0], 0);
+    if constexpr (G > 1) {
+        if (t == 0) {
+            sm.key0 = key0;
+            sm.diff = 0;
+            sm.ntied = 0;
+        }
+        __syncthreads();
+        key0 = sm.key0;
+    }
+    uint64_t diff = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+        if (t + T * e < c) diff |= x[e] ^ key0;
+    diff = ((uint64_t)__reduce_or_sync(0xFFFFFFFFu, (uint32_t)(diff >> 32)) << 32) |
+           __reduce_or_sync(0xFFFFFFFFu, (uint32_t)diff);
+    if constexpr (G > 1) {
+        if (lane == 0 && diff) atomicOr((unsigned long long*)&sm.diff, (unsigned long long)diff);
+        __syncthreads();
+        diff = sm.diff;
+    }
+    if (diff == 0) {
+        if (key_terminated(key0)) {  // all equal: any order
+            for (uint32_t j = t; j < c; j += T) {
+                w.perm[begin + s + j] = h_id(w, sm.hnd[sm.idx[idx_at(s + j)]]);
+                if (w.lcp && j) w.lcp[begin + s + j] = d + lcp_key_depth(key0);
+            }
+            return;
+        }
+        // one tied group: its common prefix in chunks of 8 chars (at least 1)
+        if (t == 0) sm.jump = 0xFFFFFFFFu;
+        group_sync<G>();
+        const uint64_t first = sm.hnd[sm.idx[idx_at(s)]];
+        for (uint32_t j = 1 + t; j < c; j += T)
+            atomicMin(&sm.jump, chunks_equal(w, first, sm.hnd[sm.idx[idx_at(s + j)]], d, &sm.jump));
+        group_sync<G>();
+        if (t == 0) {
+            const uint32_t at = sm.ng++;
+            sm.g_start[at] = (uint16_t)s;
+            sm.g_len[at] = (uint16_t)c;
+            sm.g_dep[at] = d + 8u * sm.jump;
+        }
+        return;
+    }
+    const WordForm<IB> form(key0, diff);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint32_t j = t + T * e;
+        x[e] = j < c ? form.make(x[e], j) : ~0ull;
+    }
+    group_sort<E, G>(x, reinterpret_cast<uint64_t*>(tail));
+    // LCPs and ties, from each word and the one before
+    uint64_t up = __shfl_up_sync(0xFFFFFFFFu, x[E - 1], 1);
+    if constexpr (G > 1) {
+        if (lane == 31) sm.last[warp] = x[E - 1];
+        __syncthreads();  // and the exchange buffer is free
+        if (lane == 0 && warp) up = sm.last[warp - 1];
+    }
+    uint32_t tied = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint32_t i = t * E + e;
+        const uint64_t prev = e ? x[e > 0 ? e - 1 : 0] : up;
+        if (i == 0 || i >= c) continue;
+        uint32_t l = LEAF_TIED;
+        if (!WordForm<IB>::same(prev, x[e])) {
+            l = d + form.lcp(prev, x[e]);
+        } else {
+            const uint64_t k = form.key(x[e]);
+            if (form.ended(k)) l = d + lcp_key_depth(k);
+            else tied |= 1u << e;
+        }
+        if (w.lcp) slcp[lcp_at(i)] = l;
+    }
+    // the order, in terms of the handles as they came
+    uint16_t o[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint32_t j = (uint32_t)x[e] & ((1u << IB) - 1);
+        o[e] = t * E + e < c ? sm.idx[idx_at(s + j)] : (uint16_t)0;
+    }
+    uint32_t nt = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)__popc(tied));  // strings that tie with their predecessor
+    if constexpr (G > 1) {
+        if (lane == 0 && nt) atomicAdd(&sm.ntied, nt);
+        __syncthreads();
+        nt = sm.ntied;
+    } else {
+        __syncwarp();
+    }
+    const bool any = nt != 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+        if (t * E + e < c) sm.idx[idx_at(s + t * E + e)] = o[e];
+    if (any && t < E * G) sm.tied[t] = 0;
+    group_sync<G>();
+    if (tied) atomicOr(&sm.tied[(t * E) >> 5], tied << ((t * E) & 31));
+#pragma unroll 4
+    for (uint32_t j = t; j < c; j += T) {
+        w.perm[begin + s + j] = h_id(w, sm.hnd[sm.idx[idx_at(s + j)]]);
+        if (w.lcp && j) {
+            const uint32_t l = slcp[lcp_at(j)];
+            if (l != LEAF_TIED) w.lcp[begin + s + j] = l;
+        }
+    }
+    if (!any) return;
+    group_sync<G>();
+    // lane l < E of a warp takes the runs that start in positions
+    // [32 v, 32 v + 32), v = l G + warp
+    const uint32_t dep = d + form.chars;
+    const uint32_t v = lane * G + warp;
+    uint32_t starts = 0;
+    if (lane < E) {
+        const uint32_t m = sm.tied[v], nx = v + 1 < E * G ? sm.tied[v + 1] : 0u;
+        starts = ((m >> 1) | (nx << 31)) & ~m;
+    }
+    // runs over `most` strings stay with this group's warps
+    const bool pass_on = nt > LEAF_WINDOW_TIES * G;
+    const uint32_t most = pass_on ? LEAF_WINDOW_TIES * G : (uint32_t)WARP_GROUP_MAX;
+    auto next_run = [&](uint32_t& start, uint32_t& len) {
+            while (starts) {
+                start = 32 * v + __ffs(starts) - 1;
+                starts &= starts - 1;
+                len = 1;
+                for (uint32_t q = start + 1; q < c;) {  // ones from q on
+                    const uint32_t rest = ~(sm.tied[q >> 5] >> (q & 31));
+                    const uint32_t room = 32 - (q & 31);
+                    const uint32_t ones = rest ? min((uint32_t)(__ffs(rest) - 1), room) : 32u;
+                    len += ones;
+                    if (ones < room) break;
+                    q += ones;
+                }
+                if (len <= most) return true;
+                const uint32_t at = atomicAdd(&sm.ng, 1u);
+                sm.g_start[at] = (uint16_t)(s + start);
+                sm.g_len[at] = (uint16_t)len;
+                sm.g_dep[at] = dep;
+            }
+            return false;
+        };
+    if (pass_on) {
+        // many ties: the next pass sorts the runs as segments of their own
+        // size, from the segment's handles in the order reached here
+        for (uint32_t j = t; j < c; j += T) w.hnd[buf][begin + s + j] = sm.hnd[sm.idx[idx_at(s + j)]];
+        uint32_t start = 0, len = 0;
+        bool has = next_run(start, len);
+        while (__any_sync(0xFFFFFFFFu, has)) {
+            push_seg_warp(w, w.cur ^ 1, has, Seg{begin + s + start, len, dep, (uint32_t)buf});
+            has = has && next_run(start, len);
+        }
+        return;
+    }
+    uint64_t* const defer = w.deep[w.cur ^ 1] ? w.hnd[buf] : nullptr;
+    tie_windows(
+        sm.scratch[warp], next_run,
+        [&](uint32_t, uint32_t start, uint32_t gs) {
+            const bool real = gs < 32;
+            const uint32_t q = s + start + (lane - gs);
+            const uint64_t h = real ? sm.hnd[sm.idx[idx_at(q)]] : ~0ull;
+            const uint64_t r =
+                warp_window(w, h, gs, dep, begin + q, false, 0ull, sm.scratch[warp], defer, (uint32_t)buf);
+            if (real) w.perm[begin + q] = h_id(w, r);
+        });
+}
+
+// SEGS segments per block for G == 1, one for G > 1.
+template <int G, int SEGS, int BLOCKS>
+__global__ void __launch_bounds__(32 * G * SEGS, BLOCKS) k_segs(Work w, const Seg* list, uint32_t count)
+{
+    static_assert(G == 1 || SEGS == 1, "a block's barriers serve one segment");
+    constexpr uint32_t T = 32 * G;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const uint32_t t = threadIdx.x % T, sub = threadIdx.x / T;
+    SegState<G>& sm = reinterpret_cast<SegState<G>*>(smem_raw)[sub];
+    // behind the states: exchange buffer and LCP staging (G == 1: sorts with LCP output only)
+    unsigned char* tail = smem_raw + SEGS * sizeof(SegState<G>) + sub * (size_t)SegState<G>::TAIL;
+    const uint32_t g = blockIdx.x * SEGS + sub;
+    if (g >= count) return;  // whole group
+    const Seg sg = list[g];
+    const uint32_t m = sg.size, begin = sg.begin;
+    const int buf = sg.meta & META_BUF;
+    if (sg.meta & META_FINAL) {
+        for (uint32_t i = t; i < m; i += T) {
+            w.perm[begin + i] = h_id(w, w.hnd[buf][begin + i]);
+            if (w.lcp && i) w.lcp[begin + i] = sg.depth;
+        }
+        return;
+    }
+#pragma unroll 8
+    for (uint32_t i = t; i < m; i += T) {
+        sm.hnd[i] = __ldg(w.hnd[buf] + begin + i);
+        sm.idx[idx_at(i)] = (uint16_t)i;
+    }
+    if (t == 0) {
+        sm.ng = 1;
+        sm.g_start[0] = 0;
+        sm.g_len[0] = (uint16_t)m;
+        sm.g_dep[0] = sg.depth;
+    }
+    bool cached = sg.meta & META_VALID;
+    group_sync<G>();
+    while (true) {
+        const uint32_t n = sm.ng;
+        if (n == 0) break;
+        const uint32_t s = sm.g_start[n - 1], c = sm.g_len[n - 1], d = sm.g_dep[n - 1];
+        group_sync<G>();
+        if (t == 0) sm.ng = n - 1;
+        group_sync<G>();
+        if (c <= 64 * G) sort_group<2, G>(w, sm, tail, begin, buf, s, c, d, cached);
+        else if (c <= 128 * G) sort_group<4, G>(w, sm, tail, begin, buf, s, c, d, cached);
+        else sort_group<8, G>(w, sm, tail, begin, buf, s, c, d, cached);
+        cached = false;
+        group_sync<G>();
+    }
+}
+
+constexpr int SEGS_A_WARPS = 8;
+#define K_SEGS_A k_segs<1, SEGS_A_WARPS, 3>
+#define K_SEGS_B k_segs<4, 1, 6>
+#define K_SEGS_C k_segs<16, 1, 2>
+
+}  // namespace pssgpu

@@ -6,10 +6,8 @@
 // (src/sequential/inssort.hpp:63-95) and lcp_insertion_sort
 // (src/sequential/bingmann-lcp_inssort.hpp:38-189).
 //
-// Size classes (push_seg in kernels_big.cuh picks the list):
-//   k_tiny            <= 32 strings (several segments share one warp window)
-//   k_block<256,128>  <= 256 strings, one block (kernels_block.cuh)
-//   k_block<1024,256> <= 1024 strings, one block (kernels_block.cuh)
+// The leaf sorters (kernels_leaf.cuh) and the block sorter (kernels_block.cuh)
+// send it the groups whose cached keys tie.
 //
 // A warp window holds up to 32 strings from one or more independent groups.
 // Each lane owns one output slot (a position of the permutation); groups
@@ -272,36 +270,14 @@ __device__ __forceinline__ void warp_seg_windows(const Seg* __restrict__ L, uint
     }
 }
 
-// Segments of at most 32 strings: each warp takes TINY_PER_WARP consecutive
-// list entries and packs them into warp windows.
-constexpr int TINY_WARPS = 8;
-constexpr int TINY_PER_WARP = 8;
-__global__ void __launch_bounds__(32 * TINY_WARPS, 5) k_tiny(Work w, const Seg* list, uint32_t count)
-{
-    __shared__ uint32_t scratch[TINY_WARPS][32];
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t g0 = (blockIdx.x * TINY_WARPS + (threadIdx.x >> 5)) * TINY_PER_WARP;
-    if (g0 >= count) return;  // whole warp
-    const uint32_t ng = min((uint32_t)TINY_PER_WARP, count - g0);
-    warp_seg_windows(list + g0, ng, [&](const Seg& sg, uint32_t, uint32_t gs, bool real) {
-        const uint32_t mygrp = real ? gs : 32u;
-        const int buf = sg.meta & META_BUF;
-        const uint32_t pos = sg.begin + (lane - gs);
-        const uint64_t h = real ? w.hnd[buf][pos] : ~0ull;
-        const bool hk = real && (sg.meta & META_VALID);
-        const uint64_t k0 = hk ? w.keys[buf][pos] : 0ull;
-        const uint64_t r = warp_window(w, h, mygrp, sg.depth, pos, hk, k0, scratch[threadIdx.x >> 5]);
-        if (real) w.perm[pos] = h_id(w, r);
-    });
-}
-
 // Deep groups handed over by the block sorters: one warp per group, which
 // starts with the common-prefix jump and then sorts the group to the end.
-__global__ void __launch_bounds__(32 * TINY_WARPS) k_deep(Work w, const Seg* list, uint32_t count)
+constexpr int DEEP_WARPS = 8;
+__global__ void __launch_bounds__(32 * DEEP_WARPS) k_deep(Work w, const Seg* list, uint32_t count)
 {
-    __shared__ uint32_t scratch[TINY_WARPS][32];
+    __shared__ uint32_t scratch[DEEP_WARPS][32];
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t g = blockIdx.x * TINY_WARPS + (threadIdx.x >> 5);
+    const uint32_t g = blockIdx.x * DEEP_WARPS + (threadIdx.x >> 5);
     if (g >= count) return;  // whole warp
     const Seg sg = list[g];
     const bool real = lane < sg.size;
@@ -311,9 +287,5 @@ __global__ void __launch_bounds__(32 * TINY_WARPS) k_deep(Work w, const Seg* lis
                                    scratch[threadIdx.x >> 5], nullptr, 0u, true);
     if (real) w.perm[pos] = h_id(w, r);
 }
-
-// the block-sorted size classes (kernels_block.cuh)
-constexpr int SMALL_A = 256;
-constexpr int SMALL_A_THREADS = 64;
 
 }  // namespace pssgpu

@@ -4,7 +4,7 @@
 // Enqueue (src/parallel/bingmann-parallel_sample_sort.hpp:1613-1634) with
 // level-synchronous passes: every pass runs one sample-sort step over all
 // segments larger than SMALL_MAX strings (kernels_big.cuh) and finishes all
-// smaller segments in shared memory (kernels_block.cuh, kernels_small.cuh).
+// smaller segments in registers (kernels_leaf.cuh).
 // One device-to-host read of the counters per pass sizes the next grids.
 #include <cuda_runtime.h>
 
@@ -20,6 +20,7 @@
 #include "../../include/pssgpu.h"
 #include "kernels_big.cuh"
 #include "kernels_block.cuh"
+#include "kernels_leaf.cuh"
 #include "kernels_wave.cuh"
 #include "kernels_suffix.cuh"
 #include "prepare.cuh"
@@ -131,7 +132,8 @@ static Sizes sizes_for(uint64_t n)
     Sizes s;
     s.n = std::max<uint64_t>(n, 1);
     // a segment of class c has more strings than the class below it holds
-    s.cap[L_BIG] = s.n / (SMALL_MAX + 1) + 2;
+    s.cap[L_BIG] = s.n / (SUFFIX_SMALL_MAX + 1) + 2;
+    s.cap[L_SMALLC] = s.n / 1025 + 2;
     s.cap[L_SMALLB] = s.n / 257 + 2;
     s.cap[L_SMALLA] = s.n / (WARP_GROUP_MAX + 1) + 2;
     s.cap[L_TINY] = s.n / 2 + 2;
@@ -169,10 +171,10 @@ static uint64_t workspace_bytes(const Sizes& s)
 
 // Kernel classes reported by pssgpu_ctx_kernel_stats.
 enum KClass { K_INIT = 0, K_SAMPLE, K_CLASSIFY, K_BSTART, K_SCATTER, K_CHILDREN, K_TINY,
-              K_SMALLA, K_SMALLB, K_DEEP, K_BOUNDARY, K_WAVE, K_DBL, K_NCLASS };
+              K_SMALLA, K_SMALLB, K_SMALLC, K_DEEP, K_BOUNDARY, K_WAVE, K_DBL, K_NCLASS };
 static const char* const kclass_name[K_NCLASS] = {
     "init", "sample", "classify", "bstart", "scatter", "children", "tiny",
-    "small256", "small1024", "deep", "boundary", "wave", "doubling"};
+    "small256", "small1024", "small4096", "deep", "boundary", "wave", "doubling"};
 
 struct KStat {
     uint32_t launches = 0;
@@ -244,9 +246,9 @@ struct Ctx {
     // the small-segment classes of a pass run on their own streams, beside
     // the big-segment chain on the caller's stream (disjoint ranges of the
     // permutation); fork / join through events
-    cudaStream_t side[3] = {};
+    cudaStream_t side[4] = {};
     cudaEvent_t fork_ev = nullptr;
-    cudaEvent_t join_ev[3] = {};
+    cudaEvent_t join_ev[4] = {};
 };
 
 // Record the start / end of a kernel class in profile mode.
@@ -353,10 +355,13 @@ static int setup_kernels()
                                                                sizeof(WaveSmem)));
         g_wave_blocks[dev] = coop ? (uint32_t)(per_sm * sms) : 0u;
     }
-    PSS_CUDA(cudaFuncSetAttribute(K_BLOCK_A, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(BlockSmem<SMALL_A>)));
-    PSS_CUDA(cudaFuncSetAttribute(K_BLOCK_B, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(BlockSmem<SMALL_MAX>)));
+    PSS_CUDA(cudaFuncSetAttribute(k_tiny, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TINY_SMEM));
+    PSS_CUDA(cudaFuncSetAttribute(K_SEGS_A, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)segs_smem<1>(SEGS_A_WARPS, true)));
+    PSS_CUDA(cudaFuncSetAttribute(K_SEGS_B, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)segs_smem<4>(1, true)));
+    PSS_CUDA(cudaFuncSetAttribute(K_SEGS_C, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)segs_smem<16>(1, true)));
     PSS_CUDA(cudaFuncSetAttribute(k_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sizeof(ScatterSmem)));
     done[dev] = true;
@@ -590,7 +595,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         w.dbl_cap = (uint32_t)cap;
     }
     auto pending = [&]() {
-        return cnt[L_BIG] || cnt[L_TINY] || cnt[L_SMALLA] || cnt[L_SMALLB] || ndeep;
+        return cnt[L_BIG] || cnt[L_TINY] || cnt[L_SMALLA] || cnt[L_SMALLB] || cnt[L_SMALLC] || ndeep;
     };
     // Every pass takes each open segment at least 8 chars deeper or splits
     // it; the limit turns a pass structure that stops making progress into
@@ -610,21 +615,30 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         // small classes: on the side streams (after everything queued on st
         // so far), or serially on st in profile mode so that the per-class
         // events time one class at a time
-        const bool fork = !c->profile && (cnt[L_TINY] || cnt[L_SMALLA] || cnt[L_SMALLB] || ndeep);
+        const bool fork = !c->profile &&
+                          (cnt[L_TINY] || cnt[L_SMALLA] || cnt[L_SMALLB] || cnt[L_SMALLC] || ndeep);
         if (fork) PSS_CUDA(cudaEventRecord(c->fork_ev, st));
-        bool joined[3] = {};
+        bool joined[4] = {};
         auto small_stream = [&](int q) -> cudaStream_t {
             if (!fork) return st;
             cudaStreamWaitEvent(c->side[q], c->fork_ev, 0);
             joined[q] = true;
             return c->side[q];
         };
+        if (cnt[L_SMALLC]) {
+            cudaStream_t s = small_stream(3);
+            kt.begin(K_SMALLC);
+            K_SEGS_C<<<cnt[L_SMALLC], 512, segs_smem<16>(1, true), s>>>(w, w.list[L_SMALLC][cur], cnt[L_SMALLC]);
+            kt.end(K_SMALLC);
+            c->kstat[K_SMALLC].launches += 1;
+            stats.kernel_launches += 1;
+        }
         if (cnt[L_TINY]) {
             cudaStream_t s = small_stream(0);
             kt.begin(K_TINY);
-            constexpr uint32_t per_block = TINY_WARPS * TINY_PER_WARP;
-            k_tiny<<<(cnt[L_TINY] + per_block - 1) / per_block, 32 * TINY_WARPS, 0, s>>>(
-                w, w.list[L_TINY][cur], cnt[L_TINY]);
+            const uint32_t per = tiny_per(cnt[L_TINY]), per_block = per * (TINY_THREADS / 32);
+            k_tiny<<<(cnt[L_TINY] + per_block - 1) / per_block, TINY_THREADS, TINY_SMEM, s>>>(
+                w, w.list[L_TINY][cur], cnt[L_TINY], per);
             kt.end(K_TINY);
             c->kstat[K_TINY].launches += 1;
             stats.kernel_launches += 1;
@@ -632,8 +646,8 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         if (cnt[L_SMALLA]) {
             cudaStream_t s = small_stream(1);
             kt.begin(K_SMALLA);
-            K_BLOCK_A<<<cnt[L_SMALLA], SMALL_A_THREADS, sizeof(BlockSmem<SMALL_A>), s>>>(
-                w, w.list[L_SMALLA][cur]);
+            K_SEGS_A<<<(cnt[L_SMALLA] + SEGS_A_WARPS - 1) / SEGS_A_WARPS, 32 * SEGS_A_WARPS,
+                       segs_smem<1>(SEGS_A_WARPS, w.lcp != nullptr), s>>>(w, w.list[L_SMALLA][cur], cnt[L_SMALLA]);
             kt.end(K_SMALLA);
             c->kstat[K_SMALLA].launches += 1;
             stats.kernel_launches += 1;
@@ -643,8 +657,8 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
             // stream as the block sorters, which add to the other list
             cudaStream_t s = small_stream(2);
             kt.begin(K_DEEP);
-            constexpr uint32_t per_block = TINY_WARPS;
-            k_deep<<<(std::min(ndeep, w.deep_cap) + per_block - 1) / per_block, 32 * TINY_WARPS, 0, s>>>(
+            constexpr uint32_t per_block = DEEP_WARPS;
+            k_deep<<<(std::min(ndeep, w.deep_cap) + per_block - 1) / per_block, 32 * DEEP_WARPS, 0, s>>>(
                 w, w.deep[cur], std::min(ndeep, w.deep_cap));
             kt.end(K_DEEP);
             c->kstat[K_DEEP].launches += 1;
@@ -653,13 +667,12 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         if (cnt[L_SMALLB]) {
             cudaStream_t s = small_stream(2);
             kt.begin(K_SMALLB);
-            K_BLOCK_B<<<cnt[L_SMALLB], SMALL_THREADS, sizeof(BlockSmem<SMALL_MAX>), s>>>(
-                w, w.list[L_SMALLB][cur]);
+            K_SEGS_B<<<cnt[L_SMALLB], 128, segs_smem<4>(1, true), s>>>(w, w.list[L_SMALLB][cur], cnt[L_SMALLB]);
             kt.end(K_SMALLB);
             c->kstat[K_SMALLB].launches += 1;
             stats.kernel_launches += 1;
         }
-        for (int q = 0; q < 3; ++q)
+        for (int q = 0; q < 4; ++q)
             if (joined[q]) PSS_CUDA(cudaEventRecord(c->join_ev[q], c->side[q]));
         if (nbig) {
             kt.begin(K_SAMPLE);
@@ -700,7 +713,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
             stats.kernel_launches += 6;
             stats.passes += 1;
         }
-        for (int q = 0; q < 3; ++q)
+        for (int q = 0; q < 4; ++q)
             if (joined[q]) PSS_CUDA(cudaStreamWaitEvent(st, c->join_ev[q], 0));
         PSS_CUDA(cudaGetLastError());
         PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
@@ -722,9 +735,9 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
                 20 * stale + 8 * (big - stale) + (4 + out_bytes) * fin + 8 * jch;
             c->kstat[K_SCATTER].strings += sc;
             c->kstat[K_SCATTER].alg_bytes += 24 * sc;
-            const int sk[3] = {K_TINY, K_SMALLA, K_SMALLB};
-            const int lk[3] = {L_TINY, L_SMALLA, L_SMALLB};
-            for (int q = 0; q < 3; ++q) {
+            const int sk[4] = {K_TINY, K_SMALLA, K_SMALLB, K_SMALLC};
+            const int lk[4] = {L_TINY, L_SMALLA, L_SMALLB, L_SMALLC};
+            for (int q = 0; q < 4; ++q) {
                 c->kstat[sk[q]].strings += nstr[lk[q]];
                 c->kstat[sk[q]].alg_bytes += (12 + out_bytes) * nstr[lk[q]];
                 small_segments += cnt[lk[q]];
@@ -733,11 +746,11 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
             if (c->trace) {
                 std::fprintf(stderr,
                              "pssgpu pass %u: big %u segs %u tiles %llu strings (%llu stale, %llu tied, "
-                             "%llu jump chunks, %llu final) | tiny %u/%u small256 %u/%u small1024 %u/%u deep %u",
+                             "%llu jump chunks, %llu final) | tiny %u/%u small256 %u/%u small1024 %u/%u small4096 %u/%u deep %u",
                              npass, nbig, ntiles, (unsigned long long)big, (unsigned long long)stale,
                              (unsigned long long)hc[C_P_TIE], (unsigned long long)jch, (unsigned long long)fin,
                              cnt[L_TINY], nstr[L_TINY], cnt[L_SMALLA], nstr[L_SMALLA], cnt[L_SMALLB],
-                             nstr[L_SMALLB], ndeep);
+                             nstr[L_SMALLB], cnt[L_SMALLC], nstr[L_SMALLC], ndeep);
                 if (c->profile)
                     for (int k = 0; k < K_NCLASS; ++k)
                         if (kt.pass_ms[k] > 0) std::fprintf(stderr, " %s %.3f", kclass_name[k], kt.pass_ms[k]);
@@ -810,7 +823,7 @@ static int ctx_create(int device, Ctx** out)
                   cudaSuccess;
     for (int k = 0; ok && k < 2 * K_NCLASS; ++k) ok = cudaEventCreate(&c->kev[k]) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming) == cudaSuccess;
-    for (int q = 0; ok && q < 3; ++q)
+    for (int q = 0; ok && q < 4; ++q)
         ok = cudaStreamCreateWithFlags(&c->side[q], cudaStreamNonBlocking) == cudaSuccess &&
              cudaEventCreateWithFlags(&c->join_ev[q], cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
@@ -840,7 +853,7 @@ static void ctx_destroy(Ctx* c)
     for (int k = 0; k < 2 * K_NCLASS; ++k)
         if (c->kev[k]) cudaEventDestroy(c->kev[k]);
     if (c->fork_ev) cudaEventDestroy(c->fork_ev);
-    for (int q = 0; q < 3; ++q) {
+    for (int q = 0; q < 4; ++q) {
         if (c->join_ev[q]) cudaEventDestroy(c->join_ev[q]);
         if (c->side[q]) cudaStreamDestroy(c->side[q]);
     }
@@ -1966,7 +1979,7 @@ void pssgpu_sort_strings_out(unsigned char** strings, unsigned char** output, si
 // pssgpu_sort_device_noalloc sorts at most PSSGPU_NOALLOC_MAX_STRINGS strings
 // with the small-segment kernel and allocates nothing. Its scratch -- the
 // string-handle buffer, the one segment descriptor and the counters that
-// kernel uses -- is the file-scope array below (16,528 bytes), which every
+// kernel uses -- is the file-scope array below (16,576 bytes), which every
 // device that loads this library holds until the process exits. In host code
 // the array's name is only a host-side stand-in: kernels get the device
 // address that cudaGetSymbolAddress returns, looked up once per device with

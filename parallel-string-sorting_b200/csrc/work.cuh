@@ -10,7 +10,9 @@ constexpr int TILE_THREADS = 512;   // 16 strings per thread
 constexpr int MAX_TREE_BITS = 10;   // 1023 splitters, 2047 buckets (pS5's DefaultTreebits)
 constexpr int MAX_BKT = 2056;       // bucket slots per big segment: 2047 + the two prefix buckets
 constexpr int JMAX_CHUNKS = 32;     // common-prefix jump of one pass: at most 32 8-byte chunks
-constexpr int SMALL_MAX = 1024;     // largest segment the block sorters take
+constexpr int SMALL_MAX = 4096;     // largest segment the leaf sorters take
+constexpr int SUFFIX_SMALL_MAX = 1024;  // ... of a suffix set, whose larger groups are worth
+                                        // splitting for rank doubling
 constexpr int SMALL_THREADS = 256;
 constexpr int WARP_GROUP_MAX = 32;  // groups this small are finished by one warp
 constexpr int FINAL_INLINE = 64;    // equal-string buckets this small are copied inline
@@ -18,33 +20,34 @@ constexpr int CHUNK = 32;           // tiles per chunk of the destination scan
 constexpr uint32_t DBL_MAX = 4096;  // largest group a suffix sort hands to rank doubling
 
 // segment list classes
-enum : int { L_BIG = 0, L_TINY = 1, L_SMALLA = 2, L_SMALLB = 3, L_NCLASS = 4 };
+// (at most 32, 256, 1024 and SMALL_MAX strings; L_BIG above)
+enum : int { L_BIG = 0, L_TINY = 1, L_SMALLA = 2, L_SMALLB = 3, L_SMALLC = 4, L_NCLASS = 5 };
 
 // counters[] layout
 enum : int {
-    C_PAR = 8,        // counters per parity block: [class] lengths, then tiles
-    C_NTILES = 4,     // + C_PAR * parity: tiles of the big list
-    C_NSTR = 4,       // + C_PAR * parity + class (1..3): strings in the small lists
-    C_NBND = 16,      // boundary list length
-    C_SPARE = 17,
-    C_ERR = 18,       // error bits
-    C_SMALLSEGS = 19, // statistics: segments finished by the block sorter
+    C_PAR = 10,       // counters per parity block: [class] lengths, then tiles
+    C_NTILES = 5,     // + C_PAR * parity: tiles of the big list
+    C_NSTR = 5,       // + C_PAR * parity + class (1..4): strings in the small lists
+    C_NBND = 20,      // boundary list length
+    C_SPARE = 21,
+    C_ERR = 22,       // error bits
+    C_SMALLSEGS = 23, // statistics: segments finished by the leaf sorters
     // per-pass statistics, reset every pass
-    C_P_BIG = 20,     // strings in big sample-sort segments
-    C_P_STALE = 21,   // of those, strings whose key was gathered this pass
-    C_P_FINAL = 22,   // strings copied out of big all-equal segments
-    C_P_SCATTER = 23, // strings moved by the scatter
-    C_P_TIE = 24,     // of the big strings, those classified behind a common-prefix jump
-    C_P_JCHUNKS = 25, // their prefix chunks: sum over jump segments of size * jump / 8
+    C_P_BIG = 24,     // strings in big sample-sort segments
+    C_P_STALE = 25,   // of those, strings whose key was gathered this pass
+    C_P_FINAL = 26,   // strings copied out of big all-equal segments
+    C_P_SCATTER = 27, // strings moved by the scatter
+    C_P_TIE = 28,     // of the big strings, those classified behind a common-prefix jump
+    C_P_JCHUNKS = 29, // their prefix chunks: sum over jump segments of size * jump / 8
     C_P_FIRST = C_P_BIG,
     C_P_LAST = C_P_JCHUNKS,
-    C_MULTI = 26,     // + parity: big segments of more than CHUNK tiles in the list
-    C_DEEP = 28,      // + parity: length of the deep-group list
-    C_SFX = 30,       // suffix-set check: nonzero when the input is not all suffixes of a text
-    C_DBL = 31,       // groups handed to rank doubling by the passes
-    C_DBL_CNT = 32,   // + 3 * parity + class: rank-doubling round lists
-    C_DBL_MEMB = 38,  // 64-bit (38, 39): members of the rank-doubling groups, summed over rounds
-    C_COUNT = 40
+    C_MULTI = 30,     // + parity: big segments of more than CHUNK tiles in the list
+    C_DEEP = 32,      // + parity: length of the deep-group list
+    C_SFX = 34,       // suffix-set check: nonzero when the input is not all suffixes of a text
+    C_DBL = 35,       // groups handed to rank doubling by the passes
+    C_DBL_CNT = 36,   // + 3 * parity + class: rank-doubling round lists
+    C_DBL_MEMB = 42,  // 64-bit (42, 43): members of the rank-doubling groups, summed over rounds
+    C_COUNT = 44
 };
 
 struct Work {
@@ -121,6 +124,13 @@ __device__ __forceinline__ uint32_t seg_buckets(const Work& w, int s)
     return (2u << w.tree_bits[s]) - 1 + (w.jump[s] ? 2u : 0u);
 }
 
+// list class of a segment
+__device__ __forceinline__ int seg_class(const Work& w, uint32_t size)
+{
+    if (size > (uint32_t)(w.suffix ? SUFFIX_SMALL_MAX : SMALL_MAX)) return L_BIG;
+    return size > 1024 ? L_SMALLC : size > 256 ? L_SMALLB : size > (uint32_t)WARP_GROUP_MAX ? L_SMALLA : L_TINY;
+}
+
 __device__ __forceinline__ uint64_t h_make(const Work& w, uint32_t id, uint64_t off)
 {
     return w.packed ? (((uint64_t)id << w.hbits) | off) : (uint64_t)id;
@@ -140,6 +150,60 @@ __device__ __forceinline__ uint64_t h_off(const Work& w, uint64_t h)
 __device__ __forceinline__ uint64_t h_key(const Work& w, uint64_t h, uint32_t d)
 {
     return load_key(w.chars, w.nchars, h_off(w, h) + d);
+}
+
+// Append segment c to its class's list of parity nxt.
+__device__ __forceinline__ void push_seg(const Work& w, int nxt, Seg c)
+{
+    const int cls = seg_class(w, c.size);
+    const uint32_t at = atomicAdd(w.counters + C_PAR * nxt + cls, 1u);
+    if (at >= w.cap[cls]) {
+        set_error(w.counters + C_ERR, ERR_OVERFLOW);
+        return;
+    }
+    w.list[cls][nxt][at] = c;
+    if (cls == L_BIG) {
+        const uint32_t tiles = (c.size + TILE - 1) / TILE;
+        atomicAdd(w.counters + C_PAR * nxt + C_NTILES, tiles);
+        if (tiles > (uint32_t)CHUNK) atomicAdd(w.counters + C_MULTI + nxt, 1u);
+    } else {
+        atomicAdd(w.counters + C_PAR * nxt + C_NSTR + cls, c.size);
+    }
+}
+
+// push_seg for a whole warp: lanes with push set append c. One reservation
+// per class and warp, and the class's tile or string count added once (a
+// launch that pushes many segments would otherwise serialise on these few
+// counters).
+__device__ __forceinline__ void push_seg_warp(const Work& w, int nxt, bool push, const Seg& c)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    const int cls = push ? seg_class(w, c.size) : -1;
+#pragma unroll
+    for (int k = 0; k < L_NCLASS; ++k) {
+        const uint32_t m = __ballot_sync(0xffffffffu, cls == k);
+        if (!m) continue;
+        const int leader = __ffs(m) - 1;
+        const uint32_t tiles = cls == k && k == L_BIG ? (c.size + TILE - 1) / TILE : 0u;
+        const uint32_t amount = __reduce_add_sync(0xffffffffu, cls != k ? 0u : k == L_BIG ? tiles : c.size);
+        const uint32_t multi = __reduce_add_sync(0xffffffffu, tiles > (uint32_t)CHUNK ? 1u : 0u);
+        uint32_t base = 0;
+        if (lane == (uint32_t)leader) {
+            base = atomicAdd(w.counters + C_PAR * nxt + k, (uint32_t)__popc(m));
+            if (k == L_BIG) {
+                atomicAdd(w.counters + C_PAR * nxt + C_NTILES, amount);
+                if (multi) atomicAdd(w.counters + C_MULTI + nxt, multi);
+            } else {
+                atomicAdd(w.counters + C_PAR * nxt + C_NSTR + k, amount);
+            }
+        }
+        base = __shfl_sync(0xffffffffu, base, leader);
+        if (cls == k) {
+            const uint32_t at = base + __popc(m & ((1u << lane) - 1u));
+            if (at >= w.cap[k]) set_error(w.counters + C_ERR, ERR_OVERFLOW);
+            else w.list[k][nxt][at] = c;
+        }
+    }
 }
 
 }  // namespace pssgpu

@@ -42,3 +42,46 @@ def test_suffix_lcp_chains(pkg, orc, length, at_end):
     finally:
         c.close()
     check(orc, chars, np.arange(chars.shape[0], dtype=np.uint64), perm, lcp)
+
+
+LEAF_SIZES = [2, 3, 7, 8, 9, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1023,
+              1024, 1025, 2047, 2048, 2049, 4095, 4096, 4097]
+
+
+def leaf_strings(kind, n, rng):
+    if kind == "letters":
+        return [bytes(rng.integers(97, 123, rng.integers(0, 20)).astype(np.uint8)) for _ in range(n)]
+    if kind == "acgt":  # whole keys tie many times over, in runs around 32
+        return [bytes(rng.choice(np.frombuffer(b"ACGT", np.uint8), rng.integers(1, 30))) for _ in range(n)]
+    if kind == "ff":  # words of ones beside the padding's
+        return [bytes(rng.integers(254, 256, rng.integers(6, 12)).astype(np.uint8)) for _ in range(n)]
+    if kind == "eighth":  # no shared bits (an outlier at each end), keys equal in 7 chars
+        s = [b"aaaaaaa" + bytes(rng.integers(97, 105, 1).astype(np.uint8)) + bytes([97 + int(rng.integers(3))])
+             for _ in range(n - 2)]
+        return s + [b"\x01", b"\xf0" * 9]
+    if kind == "prefix":  # one group behind a long prefix
+        return [b"p" * 101 + bytes(rng.integers(97, 100, rng.integers(0, 7)).astype(np.uint8)) for _ in range(n)]
+    heads = [bytes(rng.integers(97, 99, 25).astype(np.uint8)) for _ in range(max(1, n // 40))]  # "runs"
+    return [heads[int(rng.integers(len(heads)))] + bytes(rng.integers(97, 100, 4).astype(np.uint8)) for _ in range(n)]
+
+
+@pytest.mark.parametrize("with_lcp", [True, False])
+@pytest.mark.parametrize("kind", ["letters", "acgt", "ff", "eighth", "prefix", "runs"])
+def test_leaf_sizes(pkg, orc, kind, with_lcp):
+    """The leaf sorters at the edges of their size classes and networks, one
+    instance of a batch per size: random strings, keys that tie in runs of
+    about 32, chars 254 and 255, keys without a shared bit that tie in 7
+    chars, one long shared prefix, and runs behind 25 shared chars."""
+    rng = np.random.default_rng(len(kind))
+    strings = [leaf_strings(kind, n, rng) for n in LEAF_SIZES]
+    chars, offs = pkg.pack_strings([x for s in strings for x in s])
+    inst = np.zeros(len(LEAF_SIZES) + 1, dtype=np.uint64)
+    np.cumsum(LEAF_SIZES, out=inst[1:])
+    c = pkg.Context(0)
+    try:
+        perm, lcp = c.sort_batch_host(chars, offs, inst, lcp=with_lcp)
+    finally:
+        c.close()
+    for k in range(len(LEAF_SIZES)):
+        b, e = int(inst[k]), int(inst[k + 1])
+        check(orc, chars, offs[b:e], perm[b:e], lcp[b:e] if with_lcp else None)
