@@ -95,7 +95,8 @@ int pssgpu_ctx_kernel_stats(pssgpu_ctx* ctx, pssgpu_kernel_stats* out, int max);
  * inputs.
  * PSSGPU_OPT_SINGLE_LAUNCH (default 1): a single-instance sort whose strings
  * fit one wave of resident blocks (about 1.2 M strings on a B200) runs as one
- * cooperative kernel launch, with no host round trip between its steps;
+ * kernel launch (a block for up to 4096 strings, else a cooperative launch),
+ * with no host round trip between its steps;
  * 0 sends every sort through the multi-launch pass loop.
  * PSSGPU_OPT_WAIT_LIMIT (default 4,194,304): polls of a grid-barrier wait in
  * that kernel before it gives up and the sort returns PSSGPU_ETIMEOUT.

@@ -37,9 +37,22 @@
 
 namespace pssgpu {
 
+// Order of two 64-bit words. WORD62: both are below 2^62, so that their bits
+// are non-negative finite doubles in the same order, and the compare is one
+// DSETP on the FP64 pipe instead of two ISETP on the ALU, which bounds the
+// warp sorts (75% busy in k_segs<16>): 1.16 -> 1.07 ms for the 27.7 M strings that
+// kernel sorts of the 100k-instance batch.
+template <bool WORD62>
+__device__ __forceinline__ bool word_less(uint64_t a, uint64_t b)
+{
+    if constexpr (WORD62) return __longlong_as_double((long long)a) < __longlong_as_double((long long)b);
+    else return a < b;
+}
+
+template <bool WORD62>
 __device__ __forceinline__ void cmp_exchange(uint64_t& a, uint64_t& b)
 {
-    const bool s = b < a;
+    const bool s = word_less<WORD62>(b, a);
     const uint64_t lo = s ? b : a;
     b = s ? a : b;
     a = lo;
@@ -108,7 +121,7 @@ __device__ __forceinline__ void group_sync()
 // block, so all compares are ascending. Partner distances below E stay
 // inside a thread, those inside a warp are shuffles, longer ones go through
 // xb (32 * E * G words of shared memory, G > 1 only).
-template <int E, int G>
+template <int E, int G, bool WORD62>
 __device__ __forceinline__ void group_sort(uint64_t (&x)[E], uint64_t* xb)
 {
     constexpr uint32_t T = 32 * G;
@@ -119,7 +132,7 @@ __device__ __forceinline__ void group_sort(uint64_t (&x)[E], uint64_t* xb)
             if (d > j) continue;
 #pragma unroll
             for (int e = 0; e < E; ++e)
-                if (!(e & d)) cmp_exchange(x[e], x[e + d]);
+                if (!(e & d)) cmp_exchange<WORD62>(x[e], x[e + d]);
         }
     };
     auto publish = [&]() {
@@ -132,7 +145,7 @@ __device__ __forceinline__ void group_sort(uint64_t (&x)[E], uint64_t* xb)
     for (int k = 2; k <= E; k <<= 1) {
 #pragma unroll
         for (int e = 0; e < E; ++e)
-            if (!(e & (k >> 1))) cmp_exchange(x[e], x[e ^ (k - 1)]);
+            if (!(e & (k >> 1))) cmp_exchange<WORD62>(x[e], x[e ^ (k - 1)]);
         inner(k / 4);
     }
     // merges of 2, 4, .. 32 * G threads
@@ -144,15 +157,15 @@ __device__ __forceinline__ void group_sort(uint64_t (&x)[E], uint64_t* xb)
             for (int e = 0; e < E / 2; ++e) {
                 const uint64_t y0 = __shfl_xor_sync(0xFFFFFFFFu, x[E - 1 - e], k - 1);
                 const uint64_t y1 = __shfl_xor_sync(0xFFFFFFFFu, x[e], k - 1);
-                if ((y0 < x[e]) == lower) x[e] = y0;
-                if ((y1 < x[E - 1 - e]) == lower) x[E - 1 - e] = y1;
+                if (word_less<WORD62>(y0, x[e]) == lower) x[e] = y0;
+                if (word_less<WORD62>(y1, x[E - 1 - e]) == lower) x[E - 1 - e] = y1;
             }
         } else {
             publish();
 #pragma unroll
             for (int e = 0; e < E; ++e) {
                 const uint64_t y = xb[(E - 1 - e) * T + (t ^ (k - 1))];
-                if ((y < x[e]) == lower) x[e] = y;
+                if (word_less<WORD62>(y, x[e]) == lower) x[e] = y;
             }
         }
         uint32_t j = k >> 2;
@@ -164,7 +177,7 @@ __device__ __forceinline__ void group_sort(uint64_t (&x)[E], uint64_t* xb)
 #pragma unroll
                 for (int e = 0; e < E; ++e) {
                     const uint64_t y = xb[e * T + (t ^ j)];
-                    if ((y < x[e]) == low) x[e] = y;
+                    if (word_less<WORD62>(y, x[e]) == low) x[e] = y;
                 }
             }
         }
@@ -174,40 +187,43 @@ __device__ __forceinline__ void group_sort(uint64_t (&x)[E], uint64_t* xb)
 #pragma unroll
             for (int e = 0; e < E; ++e) {
                 const uint64_t y = __shfl_xor_sync(0xFFFFFFFFu, x[e], j);
-                if ((y < x[e]) == low) x[e] = y;
+                if (word_less<WORD62>(y, x[e]) == low) x[e] = y;
             }
         }
         inner(E / 2);
     }
 }
 
-// The words of a segment (or tied group): IB index bits below the key's
-// chars. x is the OR of its keys' differences from key0, not 0.
+// The words of a segment (or tied group): 62 bits (word_less), IB index bits
+// below the key's chars. x is the OR of its keys' differences from key0, not
+// 0.
+constexpr uint64_t WORD_PAD = ~0ull >> 2;  // after every word (no padding where index bits are all ones)
 template <int IB>
 struct WordForm {
     uint64_t key0;
     int cp;      // bits all keys share
-    int chars;   // chars of the key in the word: 8, or 7 / 6 when the index takes their place
+    int chars;   // chars of the key in the word: 8, or fewer when the index takes their place
     __device__ __forceinline__ WordForm(uint64_t k0, uint64_t x) : key0(k0)
     {
         cp = __clzll((long long)x);
-        chars = cp >= IB ? 8 : IB <= 8 ? 7 : 6;
-        static_assert(IB <= 16, "6 chars leave 16 bits");
+        chars = cp >= IB + 2 ? 8 : IB <= 6 ? 7 : 6;
+        static_assert(IB <= 14, "6 chars leave 16 bits, 2 of them on top");
     }
     __device__ __forceinline__ uint64_t make(uint64_t key, uint32_t i) const
     {
-        return ((key & (~0ull << (64 - 8 * chars))) << cp) | i;
+        return (((key & (~0ull << (64 - 8 * chars))) << cp) >> 2) | i;
     }
     // do two words hold the same chars?
     __device__ __forceinline__ static bool same(uint64_t a, uint64_t b) { return ((a ^ b) >> IB) == 0; }
     // chars shared by two words that differ
     __device__ __forceinline__ uint32_t lcp(uint64_t a, uint64_t b) const
     {
-        return (uint32_t)(cp + __clzll((long long)(a ^ b))) >> 3;
+        return (uint32_t)(cp + __clzll((long long)(a ^ b)) - 2) >> 3;
     }
     __device__ __forceinline__ uint64_t key(uint64_t word) const
     {
-        return ((word & (~0ull << IB)) >> cp) | (cp ? key0 & (~0ull << (64 - cp)) & (~0ull << (64 - 8 * chars)) : 0ull);
+        return (((word & (~0ull << IB)) << 2) >> cp) |
+               (cp ? key0 & (~0ull << (64 - cp)) & (~0ull << (64 - 8 * chars)) : 0ull);
     }
     // do strings with this key (key()'s value) end inside the word's chars?
     __device__ __forceinline__ bool ended(uint64_t k) const { return ((k >> (64 - 8 * chars)) & 0xFF) == 0; }
@@ -486,7 +502,9 @@ struct alignas(16) SegState {
     uint64_t hnd[N];
     uint64_t last[G], key0, diff;
     uint16_t idx[IDX];
+    uint16_t tpos[N], trun[N];  // tied strings of a group: position and run number
     uint32_t tied[N / 32];    // bit i: the string at i ties with the one before
+    uint32_t wsum[G];
     uint32_t scratch[G][32];
     uint16_t g_start[N / 32], g_len[N / 32];
     uint32_t g_dep[N / 32];
@@ -505,6 +523,12 @@ constexpr size_t segs_smem(int segs, bool lcp)
 __device__ __forceinline__ uint32_t idx_at(uint32_t i) { return i + ((i >> 5) << 1); }
 __device__ __forceinline__ uint32_t lcp_at(uint32_t i) { return i + (i >> 5); }
 
+// Ties per warp beyond which all tied runs of a group are sorted together
+// (sort_runs), up to LEAF_RESORTS times in a row: 200 k ACGT strings (3 per
+// 8-char key) 186 -> 95 us, 2 M of them with LCPs 0.56 -> 0.52 ms, against warp
+// windows and another pass alone.
+constexpr uint32_t LEAF_RESORT_TIES = 24;
+constexpr int LEAF_RESORTS = 2;
 // Ties per warp beyond which a group hands its tied runs to the next pass
 // instead of sorting them in warp windows, or (runs over 32 strings) by all
 // its warps, one after another. Runs over LEAF_WINDOW_TIES * G stay: the
@@ -512,18 +536,42 @@ __device__ __forceinline__ uint32_t lcp_at(uint32_t i) { return i + (i >> 5); }
 constexpr uint32_t LEAF_WINDOW_TIES = 48;
 constexpr uint32_t LEAF_TIED = 0xFFFFFFFFu;  // LCP staging: not known yet
 
+// Bits that hold an index below n (a power of two).
+__host__ __device__ constexpr int word_index_bits(int n)
+{
+    int b = 0;
+    while ((1 << b) < n) ++b;
+    return b;
+}
+
+// Sum over the group of the ties each thread found (G > 1: sm.ntied is 0
+// before). Synchronises.
+template <int G>
+__device__ __forceinline__ uint32_t count_ties(SegState<G>& sm, uint32_t tied)
+{
+    uint32_t nt = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)__popc(tied));
+    if constexpr (G > 1) {
+        if ((threadIdx.x & 31) == 0 && nt) atomicAdd(&sm.ntied, nt);
+        __syncthreads();
+        nt = sm.ntied;
+    } else {
+        __syncwarp();
+    }
+    return nt;
+}
+
 // Sort the group of c strings (c <= 32 E G) at offset s of the segment, depth
-// d; with the segment's cached keys when `cached` (then s is 0). Tied groups
-// of more than 32 strings go to the stack, smaller ones to warp windows.
+// d; with the segment's cached keys when `cached` (then s is 0). Writes perm
+// and the LCPs it finds. Returns how many strings tie with their predecessor
+// (marked in sm.tied; *chars deeper than d); a group whose keys are all equal
+// goes back to the stack behind its common prefix.
 template <int E, int G>
-__device__ __forceinline__ void sort_group(const Work& w, SegState<G>& sm, unsigned char* tail, uint32_t begin,
-                                           int buf, uint32_t s, uint32_t c, uint32_t d, bool cached)
+__device__ __forceinline__ uint32_t sort_group(const Work& w, SegState<G>& sm, unsigned char* tail, uint32_t begin,
+                                               int buf, uint32_t s, uint32_t c, uint32_t d, bool cached,
+                                               uint32_t* chars)
 {
     constexpr uint32_t T = 32 * G;
-    constexpr int NMAX = 32 * E * G;
-    constexpr int IB = NMAX == 64 ? 6 : NMAX == 128 ? 7 : NMAX == 256 ? 8 : NMAX == 512 ? 9 : NMAX == 1024 ? 10
-                     : NMAX == 2048 ? 11 : NMAX == 4096 ? 12 : 13;
-    static_assert(NMAX <= 1 << IB && IB <= 13, "index bits");
+    constexpr int IB = word_index_bits(32 * E * G);
     const uint32_t lane = threadIdx.x & 31, warp = G == 1 ? 0u : threadIdx.x >> 5;
     const uint32_t t = 32 * warp + lane;
     uint32_t* slcp = reinterpret_cast<uint32_t*>(tail);
@@ -533,7 +581,7 @@ __device__ __forceinline__ void sort_group(const Work& w, SegState<G>& sm, unsig
         const uint32_t j = t + T * e;
         x[e] = 0;
         if (j < c)
-            x[e] = cached ? __ldg(w.keys[buf] + begin + j) : h_key(w, sm.hnd[sm.idx[idx_at(s + j)]], d);
+            x[e] = cached ? __ldcg(w.keys[buf] + begin + j) : h_key(w, sm.hnd[sm.idx[idx_at(s + j)]], d);
     }
     uint64_t key0 = __shfl_sync(0xFFFFFFFFu, x[0], 0);
     if constexpr (G > 1) {
@@ -562,7 +610,7 @@ __device__ __forceinline__ void sort_group(const Work& w, SegState<G>& sm, unsig
                 w.perm[begin + s + j] = h_id(w, sm.hnd[sm.idx[idx_at(s + j)]]);
                 if (w.lcp && j) w.lcp[begin + s + j] = d + lcp_key_depth(key0);
             }
-            return;
+            return 0;
         }
         // one tied group: its common prefix in chunks of 8 chars (at least 1)
         if (t == 0) sm.jump = 0xFFFFFFFFu;
@@ -577,15 +625,15 @@ __device__ __forceinline__ void sort_group(const Work& w, SegState<G>& sm, unsig
             sm.g_len[at] = (uint16_t)c;
             sm.g_dep[at] = d + 8u * sm.jump;
         }
-        return;
+        return 0;
     }
     const WordForm<IB> form(key0, diff);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const uint32_t j = t + T * e;
-        x[e] = j < c ? form.make(x[e], j) : ~0ull;
+        x[e] = j < c ? form.make(x[e], j) : WORD_PAD;
     }
-    group_sort<E, G>(x, reinterpret_cast<uint64_t*>(tail));
+    group_sort<E, G, true>(x, reinterpret_cast<uint64_t*>(tail));
     // LCPs and ties, from each word and the one before
     uint64_t up = __shfl_up_sync(0xFFFFFFFFu, x[E - 1], 1);
     if constexpr (G > 1) {
@@ -616,19 +664,11 @@ __device__ __forceinline__ void sort_group(const Work& w, SegState<G>& sm, unsig
         const uint32_t j = (uint32_t)x[e] & ((1u << IB) - 1);
         o[e] = t * E + e < c ? sm.idx[idx_at(s + j)] : (uint16_t)0;
     }
-    uint32_t nt = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)__popc(tied));  // strings that tie with their predecessor
-    if constexpr (G > 1) {
-        if (lane == 0 && nt) atomicAdd(&sm.ntied, nt);
-        __syncthreads();
-        nt = sm.ntied;
-    } else {
-        __syncwarp();
-    }
-    const bool any = nt != 0;
+    const uint32_t nt = count_ties<G>(sm, tied);
 #pragma unroll
     for (int e = 0; e < E; ++e)
         if (t * E + e < c) sm.idx[idx_at(s + t * E + e)] = o[e];
-    if (any && t < E * G) sm.tied[t] = 0;
+    if (nt && t < E * G) sm.tied[t] = 0;
     group_sync<G>();
     if (tied) atomicOr(&sm.tied[(t * E) >> 5], tied << ((t * E) & 31));
 #pragma unroll 4
@@ -639,44 +679,193 @@ __device__ __forceinline__ void sort_group(const Work& w, SegState<G>& sm, unsig
             if (l != LEAF_TIED) w.lcp[begin + s + j] = l;
         }
     }
-    if (!any) return;
+    *chars = form.chars;
     group_sync<G>();
-    // lane l < E of a warp takes the runs that start in positions
+    return nt;
+}
+
+// The tied strings of a group of c strings (their runs marked in sm.tied) into
+// sm.tpos / sm.trun in order of their positions; returns how many, *runs the
+// number of runs. A thread takes 8 positions.
+template <int G>
+__device__ __forceinline__ uint32_t collect_ties(SegState<G>& sm, uint32_t c, uint32_t* runs)
+{
+    const uint32_t lane = threadIdx.x & 31, warp = G == 1 ? 0u : threadIdx.x >> 5;
+    const uint32_t p0 = 8 * (32 * warp + lane);
+    const uint32_t words = (c + 31) / 32;
+    uint32_t at = 0;  // ties of positions p0 .. p0 + 8
+    if (p0 < c) {
+        const uint32_t lo = sm.tied[p0 >> 5], hi = (p0 >> 5) + 1 < words ? sm.tied[(p0 >> 5) + 1] : 0u;
+        at = __funnelshift_r(lo, hi, p0 & 31) & 0x1FFu;
+    }
+    const uint32_t member = (at | (at >> 1)) & 0xFFu, starts = (at >> 1) & ~at & 0xFFu;
+    const uint32_t mine = __popc(member) | (__popc(starts) << 16);
+    const uint32_t incl = warp_incl_sum(mine);
+    uint32_t before = incl - mine, total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    if constexpr (G > 1) {
+        if (lane == 31) sm.wsum[warp] = incl;
+        __syncthreads();
+        total = 0;
+        for (int v = 0; v < G; ++v) {
+            if (v < (int)warp) before += sm.wsum[v];
+            total += sm.wsum[v];
+        }
+    }
+    uint32_t j = before & 0xFFFFu, r = before >> 16;  // runs started before p0
+    for (uint32_t m = member; m; m &= m - 1) {
+        const uint32_t q = __ffs(m) - 1;
+        r += (starts >> q) & 1u;
+        sm.tpos[j] = (uint16_t)(p0 + q);
+        sm.trun[j++] = (uint16_t)(r - 1);
+    }
+    *runs = total >> 16;
+    group_sync<G>();
+    return total & 0xFFFFu;
+}
+
+// Sort the runs of n tied strings (collect_ties; n <= 32 E G) of the group at
+// offset s, all at once, by the chars at depth d: a word is (run, chars,
+// index), as many chars as fit (4 to 6). Writes perm, the LCPs it finds and
+// the new sm.tied; returns how many strings still tie (*chars deeper). Where
+// most neighbours in the runs share these chars too (a long common prefix),
+// nothing is done: *chars is 0.
+template <int E, int G>
+__device__ __forceinline__ uint32_t sort_runs(const Work& w, SegState<G>& sm, unsigned char* tail, uint32_t begin,
+                                              uint32_t s, uint32_t c, uint32_t n, uint32_t runs, uint32_t ties,
+                                              uint32_t d, uint32_t* chars)
+{
+    constexpr uint32_t T = 32 * G;
+    constexpr int IB = word_index_bits(32 * E * G);
+    const uint32_t lane = threadIdx.x & 31, warp = G == 1 ? 0u : threadIdx.x >> 5;
+    const uint32_t t = 32 * warp + lane;
+    const int rb = 32 - __clz((int)runs);  // run numbers are below 2^rb
+    const int kc = (62 - IB - rb) / 8;
+    const int ksh = 62 - rb - 8 * kc;      // the chars' lowest bit
+    uint64_t x[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint32_t j = t + T * e;
+        x[e] = WORD_PAD;
+        if (j < n) {
+            const uint64_t k = h_key(w, sm.hnd[sm.idx[idx_at(s + sm.tpos[j])]], d);
+            x[e] = ((uint64_t)sm.trun[j] << (62 - rb)) | ((k >> (64 - 8 * kc)) << ksh) | j;
+        }
+    }
+    uint32_t pairs = 0;  // neighbours of one run, and (<< 16) those equal
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint64_t df = x[e] ^ __shfl_up_sync(0xFFFFFFFFu, x[e], 1);
+        if (lane && t + T * e < n && !(df >> (62 - rb))) pairs += df >> ksh ? 1u : 0x10001u;
+    }
+    pairs = __reduce_add_sync(0xFFFFFFFFu, pairs);
+    if constexpr (G > 1) {
+        if (lane == 0) sm.wsum[warp] = pairs;
+        if (t == 0) sm.ntied = 0;
+        __syncthreads();
+        pairs = 0;
+        for (int v = 0; v < G; ++v) pairs += sm.wsum[v];
+    }
+    *chars = 0;
+    if ((pairs >> 16) * 2 > (pairs & 0xFFFFu)) return ties;
+    group_sort<E, G, true>(x, reinterpret_cast<uint64_t*>(tail));
+    uint64_t up = __shfl_up_sync(0xFFFFFFFFu, x[E - 1], 1);
+    if constexpr (G > 1) {
+        if (lane == 31) sm.last[warp] = x[E - 1];
+        __syncthreads();
+        if (lane == 0 && warp) up = sm.last[warp - 1];
+    }
+    uint32_t tied = 0;
+    uint16_t o[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint32_t i = t * E + e;
+        const uint64_t prev = e ? x[e > 0 ? e - 1 : 0] : up;
+        o[e] = 0;
+        if (i >= n) continue;
+        o[e] = sm.idx[idx_at(s + sm.tpos[(uint32_t)x[e] & ((1u << IB) - 1)])];
+        if (i == 0) continue;
+        const uint64_t df = x[e] ^ prev;
+        if (df >> (62 - rb)) continue;  // another run
+        uint32_t l;
+        if (df >> ksh) {
+            l = (uint32_t)(__clzll((long long)df) - 2 - rb) >> 3;
+        } else {
+            const uint64_t k = (x[e] >> ksh) << (64 - 8 * kc);  // the chars, left-aligned (run bits shifted out)
+            if ((k >> (64 - 8 * kc)) & 0xFF) {
+                tied |= 1u << e;
+                continue;
+            }
+            l = lcp_key_depth(k);
+        }
+        if (w.lcp) w.lcp[begin + s + sm.tpos[i]] = d + l;
+    }
+    const uint32_t nt = count_ties<G>(sm, tied);
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+        if (t * E + e < n) {
+            const uint32_t p = s + sm.tpos[t * E + e];
+            sm.idx[idx_at(p)] = o[e];
+            w.perm[begin + p] = h_id(w, sm.hnd[o[e]]);
+        }
+    for (uint32_t v = t; v < (c + 31) / 32; v += T) sm.tied[v] = 0;
+    group_sync<G>();
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+        if ((tied >> e) & 1u) {
+            const uint32_t p = sm.tpos[t * E + e];
+            atomicOr(&sm.tied[p >> 5], 1u << (p & 31));
+        }
+    *chars = kc;
+    group_sync<G>();
+    return nt;
+}
+
+// The nt ties left in the group of c strings at offset s, whose runs share
+// `dep` chars: to the next pass when there are many, else runs of up to 32
+// strings to warp windows and longer ones to the stack.
+template <int G>
+__device__ __forceinline__ void finish_ties(const Work& w, SegState<G>& sm, uint32_t begin, int buf, uint32_t s,
+                                            uint32_t c, uint32_t dep, uint32_t nt)
+{
+    constexpr uint32_t T = 32 * G;
+    const uint32_t lane = threadIdx.x & 31, warp = G == 1 ? 0u : threadIdx.x >> 5;
+    const uint32_t t = 32 * warp + lane;
+    // lane l of a warp takes the runs that start in positions
     // [32 v, 32 v + 32), v = l G + warp
-    const uint32_t dep = d + form.chars;
+    const uint32_t words = (c + 31) / 32;
     const uint32_t v = lane * G + warp;
     uint32_t starts = 0;
-    if (lane < E) {
-        const uint32_t m = sm.tied[v], nx = v + 1 < E * G ? sm.tied[v + 1] : 0u;
+    if (v < words) {
+        const uint32_t m = sm.tied[v], nx = v + 1 < words ? sm.tied[v + 1] : 0u;
         starts = ((m >> 1) | (nx << 31)) & ~m;
     }
     // runs over `most` strings stay with this group's warps
     const bool pass_on = nt > LEAF_WINDOW_TIES * G;
     const uint32_t most = pass_on ? LEAF_WINDOW_TIES * G : (uint32_t)WARP_GROUP_MAX;
     auto next_run = [&](uint32_t& start, uint32_t& len) {
-            while (starts) {
-                start = 32 * v + __ffs(starts) - 1;
-                starts &= starts - 1;
-                len = 1;
-                for (uint32_t q = start + 1; q < c;) {  // ones from q on
-                    const uint32_t rest = ~(sm.tied[q >> 5] >> (q & 31));
-                    const uint32_t room = 32 - (q & 31);
-                    const uint32_t ones = rest ? min((uint32_t)(__ffs(rest) - 1), room) : 32u;
-                    len += ones;
-                    if (ones < room) break;
-                    q += ones;
-                }
-                if (len <= most) return true;
-                const uint32_t at = atomicAdd(&sm.ng, 1u);
-                sm.g_start[at] = (uint16_t)(s + start);
-                sm.g_len[at] = (uint16_t)len;
-                sm.g_dep[at] = dep;
+        while (starts) {
+            start = 32 * v + __ffs(starts) - 1;
+            starts &= starts - 1;
+            len = 1;
+            for (uint32_t q = start + 1; q < c;) {  // ones from q on
+                const uint32_t rest = ~(sm.tied[q >> 5] >> (q & 31));
+                const uint32_t room = 32 - (q & 31);
+                const uint32_t ones = rest ? min((uint32_t)(__ffs(rest) - 1), room) : 32u;
+                len += ones;
+                if (ones < room) break;
+                q += ones;
             }
-            return false;
-        };
+            if (len <= most) return true;
+            const uint32_t at = atomicAdd(&sm.ng, 1u);
+            sm.g_start[at] = (uint16_t)(s + start);
+            sm.g_len[at] = (uint16_t)len;
+            sm.g_dep[at] = dep;
+        }
+        return false;
+    };
     if (pass_on) {
-        // many ties: the next pass sorts the runs as segments of their own
-        // size, from the segment's handles in the order reached here
+        // the next pass sorts the runs as segments of their own size, from the
+        // segment's handles in the order reached here
         for (uint32_t j = t; j < c; j += T) w.hnd[buf][begin + s + j] = sm.hnd[sm.idx[idx_at(s + j)]];
         uint32_t start = 0, len = 0;
         bool has = next_run(start, len);
@@ -687,16 +876,55 @@ __device__ __forceinline__ void sort_group(const Work& w, SegState<G>& sm, unsig
         return;
     }
     uint64_t* const defer = w.deep[w.cur ^ 1] ? w.hnd[buf] : nullptr;
-    tie_windows(
-        sm.scratch[warp], next_run,
-        [&](uint32_t, uint32_t start, uint32_t gs) {
-            const bool real = gs < 32;
-            const uint32_t q = s + start + (lane - gs);
-            const uint64_t h = real ? sm.hnd[sm.idx[idx_at(q)]] : ~0ull;
-            const uint64_t r =
-                warp_window(w, h, gs, dep, begin + q, false, 0ull, sm.scratch[warp], defer, (uint32_t)buf);
-            if (real) w.perm[begin + q] = h_id(w, r);
-        });
+    tie_windows(sm.scratch[warp], next_run, [&](uint32_t, uint32_t start, uint32_t gs) {
+        const bool real = gs < 32;
+        const uint32_t q = s + start + (lane - gs);
+        const uint64_t h = real ? sm.hnd[sm.idx[idx_at(q)]] : ~0ull;
+        const uint64_t r = warp_window(w, h, gs, dep, begin + q, false, 0ull, sm.scratch[warp], defer, (uint32_t)buf);
+        if (real) w.perm[begin + q] = h_id(w, r);
+    });
+}
+
+// Sort the segment of m strings at position begin by its group of G warps:
+// handles in sm.hnd (idx: 0..m-1), buf the buffer they came from, depth the
+// chars they share, cached whether keys[buf] holds their keys.
+template <int G>
+__device__ __forceinline__ void sort_segment(const Work& w, SegState<G>& sm, unsigned char* tail, uint32_t begin,
+                                             uint32_t m, int buf, uint32_t depth, bool cached)
+{
+    const uint32_t t = threadIdx.x % (32 * G);
+    if (t == 0) {
+        sm.ng = 1;
+        sm.g_start[0] = 0;
+        sm.g_len[0] = (uint16_t)m;
+        sm.g_dep[0] = depth;
+    }
+    group_sync<G>();
+    while (true) {
+        const uint32_t n = sm.ng;
+        if (n == 0) break;
+        const uint32_t s = sm.g_start[n - 1], c = sm.g_len[n - 1], d = sm.g_dep[n - 1];
+        group_sync<G>();
+        if (t == 0) sm.ng = n - 1;
+        group_sync<G>();
+        uint32_t chars = 0;
+        uint32_t nt = c <= 64 * G    ? sort_group<2, G>(w, sm, tail, begin, buf, s, c, d, cached, &chars)
+                      : c <= 128 * G ? sort_group<4, G>(w, sm, tail, begin, buf, s, c, d, cached, &chars)
+                                     : sort_group<8, G>(w, sm, tail, begin, buf, s, c, d, cached, &chars);
+        uint32_t dep = d + chars;
+        for (int r = 0; r < LEAF_RESORTS && nt > LEAF_RESORT_TIES * G; ++r) {
+            uint32_t runs = 0;
+            const uint32_t k = collect_ties<G>(sm, c, &runs);
+            nt = k <= 64 * G    ? sort_runs<2, G>(w, sm, tail, begin, s, c, k, runs, nt, dep, &chars)
+                 : k <= 128 * G ? sort_runs<4, G>(w, sm, tail, begin, s, c, k, runs, nt, dep, &chars)
+                                : sort_runs<8, G>(w, sm, tail, begin, s, c, k, runs, nt, dep, &chars);
+            if (!chars) break;
+            dep += chars;
+        }
+        if (nt) finish_ties<G>(w, sm, begin, buf, s, c, dep, nt);
+        cached = false;
+        group_sync<G>();
+    }
 }
 
 // SEGS segments per block for G == 1, one for G > 1.
@@ -724,30 +952,43 @@ __global__ void __launch_bounds__(32 * G * SEGS, BLOCKS) k_segs(Work w, const Se
     }
 #pragma unroll 8
     for (uint32_t i = t; i < m; i += T) {
-        sm.hnd[i] = __ldg(w.hnd[buf] + begin + i);
+        sm.hnd[i] = __ldcg(w.hnd[buf] + begin + i);
         sm.idx[idx_at(i)] = (uint16_t)i;
     }
-    if (t == 0) {
-        sm.ng = 1;
-        sm.g_start[0] = 0;
-        sm.g_len[0] = (uint16_t)m;
-        sm.g_dep[0] = sg.depth;
+    sort_segment<G>(w, sm, tail, begin, m, buf, sg.depth, sg.meta & META_VALID);
+}
+
+// The whole sort of an input of at most 256 G strings, by one block: handles
+// from the offsets, the input checks, and the counters, which go to the
+// host's copy at the end (mapped memory: no memset before and no copy after
+// the kernel). w.cur is 0: what is left over goes to the lists of parity 1,
+// in buffer 0.
+template <int G>
+__global__ void __launch_bounds__(32 * G) k_one(Work w, uint32_t* host_counters)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SegState<G>& sm = *reinterpret_cast<SegState<G>*>(smem_raw);
+    constexpr uint32_t T = 32 * G;
+    const uint32_t t = threadIdx.x;
+    for (uint32_t k = t; k < (uint32_t)C_COUNT; k += T) w.counters[k] = 0;
+    uint32_t err = t == 0 && w.chars[w.nchars - 1] != 0 ? ERR_UNTERMINATED : 0u;
+#pragma unroll 8
+    for (uint32_t i = t; i < w.n; i += T) {
+        const uint64_t off = __ldg(w.offs + i);
+        if (off >= w.nchars) err |= ERR_OFFSET;
+        sm.hnd[i] = h_make(w, i, off);
+        sm.idx[idx_at(i)] = (uint16_t)i;
     }
-    bool cached = sg.meta & META_VALID;
-    group_sync<G>();
-    while (true) {
-        const uint32_t n = sm.ng;
-        if (n == 0) break;
-        const uint32_t s = sm.g_start[n - 1], c = sm.g_len[n - 1], d = sm.g_dep[n - 1];
-        group_sync<G>();
-        if (t == 0) sm.ng = n - 1;
-        group_sync<G>();
-        if (c <= 64 * G) sort_group<2, G>(w, sm, tail, begin, buf, s, c, d, cached);
-        else if (c <= 128 * G) sort_group<4, G>(w, sm, tail, begin, buf, s, c, d, cached);
-        else sort_group<8, G>(w, sm, tail, begin, buf, s, c, d, cached);
-        cached = false;
-        group_sync<G>();
+    if (t == 0) sm.ntied = 0;
+    __syncthreads();
+    if (err) {
+        set_error(w.counters + C_ERR, err);
+        sm.ntied = 1;
     }
+    __syncthreads();
+    if (!sm.ntied) sort_segment<G>(w, sm, smem_raw + sizeof(SegState<G>), 0, w.n, 0, 0, false);
+    __syncthreads();
+    for (uint32_t k = t; k < (uint32_t)C_COUNT; k += T) host_counters[k] = __ldcg(w.counters + k);
 }
 
 constexpr int SEGS_A_WARPS = 8;

@@ -8,72 +8,81 @@
 // 405-676). Here the same steps are phases of one kernel, separated by grid
 // barriers (all blocks are co-resident by the cooperative launch):
 //   A  every block gathers the first 8 chars (get_char_uint64_simple) of its
-//      tile of strings into registers; the first blocks also draw 2^(L+1)
-//      samples in chunks of 512 and sort their chunk
-//   B  every block merges the sorted chunks and builds the splitters and the
-//      level-order tree itself (SampleSortStep::sample,
-//      TreeBuilderLevelOrder), classifies its tile (find_bkt), counts per bucket in
-//      shared memory, reserve the tile's share of every bucket with one
-//      global atomic per non-empty bucket (count, hpp:1414-1435)
+//      tile of strings into registers, draws the same `over` * 2^L samples, sorts
+//      them and builds the level-order tree (SampleSortStep::sample,
+//      TreeBuilderLevelOrder)
+//   B  classifies its tile (find_bkt), counts per bucket in shared memory,
+//      reserves the tile's share of every bucket with one global atomic per
+//      non-empty bucket (count, hpp:1414-1435)
 //   C  bucket starts (count_finished), scatter keys and handles in bucket
 //      order (distribute, hpp:1464-1490)
-//   D  a dynamic queue of windows of WAVE_WINDOW positions: the runs of
-//      buckets of at most WAVE_WINDOW strings that start in a window are
-//      finished by the block sorter as one group (block_sort_groups, the
-//      SmallsortJob counterpart); larger buckets are finished alone (up to
-//      WAVE_SORT_MAX strings), copied out when their strings are all equal,
-//      or handed to the level-synchronous passes as a segment
-//      (distribute_finished, hpp:1492-1584). With LCP output a fourth
-//      barrier precedes the LCPs at the bucket boundaries, which come from
-//      the neighbouring buckets' key ranges (sample_sort_lcp, hpp:311-396).
+//   D  a dynamic queue of windows of `window` positions: the runs of buckets
+//      of at most `window` strings that start in a window are finished by the
+//      leaf sorter as one segment (sort_segment, the SmallsortJob
+//      counterpart); larger buckets are finished alone (up to SMALL_MAX
+//      strings), copied out when their strings are all equal, or handed to
+//      the level-synchronous passes as a segment (distribute_finished,
+//      hpp:1492-1584). With LCP output a third barrier precedes the LCPs at
+//      the first positions of the runs, which come from the neighbouring
+//      buckets' key ranges (sample_sort_lcp, hpp:311-396).
+// Latency-bound: dependent gathers, the sorts' chains and the barriers.
+// Sorting the samples in every block costs less than a barrier after one
+// shared sort did, and the register sorts of phase D less than sample-sort
+// steps in shared memory: 487 k digit strings 150 -> 96 us, 7.8 k strings
+// 65 -> 33 us of device time.
 // Every barrier wait is bounded: after `limit` polls a block sets
 // ERR_TIMEOUT and returns, and the blocks still waiting see the flag and
 // return as well.
 #pragma once
 
-#include "kernels_big.cuh"
-#include "kernels_block.cuh"
+#include "kernels_leaf.cuh"
 
 namespace pssgpu {
 
-constexpr int WAVE_THREADS = 512;
+constexpr int WAVE_G = 16;
+constexpr int WAVE_THREADS = 32 * WAVE_G;
 constexpr int WAVE_PER = 8;           // strings per thread through phases A-C
 constexpr int WAVE_MAX_BITS = 11;     // at most 2047 splitters, 4095 buckets
 constexpr int WAVE_BKT = 2 << WAVE_MAX_BITS;   // 4096 bucket slots
-constexpr int WAVE_WINDOW = 1024;     // positions per window task
-constexpr int WAVE_SORT_MAX = 2048;   // the block sorter of phase D
+constexpr uint32_t WAVE_WINDOW_MAX = 1024;     // largest window (positions)
 constexpr uint32_t WAVE_TILE_MAX = (uint32_t)WAVE_THREADS * WAVE_PER;
-constexpr uint32_t WAVE_SAMPLE_CHUNK = WAVE_THREADS;  // samples one block draws and sorts
 
-// Global state of one wave sort (in the workspace). The header is zeroed by
-// the host before the launch; everything else is written inside.
+// Global state of one wave sort (in the workspace). Everything up to the
+// splitters is zeroed by the host before the launch.
 struct WaveState {
     uint32_t bar;        // grid barrier arrivals
     uint32_t next_task;  // phase-D windows taken
-    uint32_t pad[4];
+    uint32_t nruns;      // runs recorded (LCP output only)
+    uint32_t pad[3];
     // with tracing on: the largest SM-clock cycles any block spent in phase
-    // A (incl. block 0's samples), the first barrier wait, B (+ the second
-    // wait), C (+ the third) and D (+ the LCPs)
+    // A, B, the wait behind it, C (+ its wait) and D (+ the LCPs)
     unsigned long long cycles[5];
     uint32_t gcount[WAVE_BKT];   // bucket counts
     uint64_t spl[WAVE_BKT / 2];  // sorted splitters
-    uint64_t samp[WAVE_BKT];     // the samples, sorted in chunks of WAVE_SAMPLE_CHUNK
-    uint64_t bmin[WAVE_BKT];     // key range of '<' buckets (LCP output only)
+    // LCP output only: the first bucket of every run that phase D finished
+    // or handed over, its smallest key and the largest key of its last bucket
+    uint16_t run[WAVE_BKT];
+    uint64_t bmin[WAVE_BKT];
     uint64_t bmax[WAVE_BKT];
 };
 
 // Dynamic shared memory of k_wave: bucket starts, then either the phase A-C
-// view (samples / tree, per-bucket counts) or the block sorter's.
+// view (samples, tree, per-bucket counts) or the leaf sorter's.
 struct WaveSmemABC {
-    uint64_t m[2][WAVE_BKT];     // sample chunks merged back and forth; then the tree
+    uint64_t samp[WAVE_BKT];     // exchange buffer of the sort, then the sorted samples
+    uint64_t tree[WAVE_BKT / 2]; // level order, index 1..k
     uint32_t cnt[WAVE_BKT];      // per bucket: count in the tile, then the tile's base
+};
+struct WaveSmemSort {
+    SegState<WAVE_G> seg;
+    unsigned char tail[SegState<WAVE_G>::TAIL];
 };
 struct WaveSmem {
     uint32_t start[WAVE_BKT + 1];  // bucket starts (exclusive scan), start[B] = n
     uint32_t pad[3];
     union {
         WaveSmemABC abc;
-        BlockSmem<WAVE_SORT_MAX> sort;
+        WaveSmemSort sort;
     } u;
 };
 
@@ -115,13 +124,13 @@ __device__ __forceinline__ uint32_t wave_lower(const uint32_t* start, uint32_t B
     return lo;
 }
 
-// Key range of '<' bucket b (c >= 1 strings at position P of keys[1]) into
-// ws->bmin / bmax, by the whole block; red is two words of shared memory.
-__device__ __forceinline__ void wave_range_block(const Work& w, WaveState* ws, uint32_t b,
-                                                 uint32_t P, uint32_t c, uint64_t* red)
+// LCP output: record the run of positions [P, P + m), m >= 1, which starts
+// and ends with a bucket, and its key range. red: two words of shared memory.
+__device__ __forceinline__ void wave_note_run(const Work& w, WaveState* ws, const uint32_t* start, uint32_t B,
+                                              uint32_t P, uint32_t m, uint64_t* red)
 {
     uint64_t mn = ~0ull, mx = 0;
-    for (uint32_t q = threadIdx.x; q < c; q += WAVE_THREADS) {
+    for (uint32_t q = threadIdx.x; q < m; q += WAVE_THREADS) {
         const uint64_t k = __ldcg(w.keys[1] + P + q);
         mn = min(mn, k);
         mx = max(mx, k);
@@ -142,60 +151,65 @@ __device__ __forceinline__ void wave_range_block(const Work& w, WaveState* ws, u
     }
     __syncthreads();
     if (threadIdx.x == 0) {
+        const uint32_t b = wave_lower(start, B, P + 1) - 1;   // the bucket that starts at P
+        const uint32_t e = wave_lower(start, B, P + m) - 1;   // the bucket that ends the run
         ws->bmin[b] = red[0];
-        ws->bmax[b] = red[1];
+        ws->bmax[e] = red[1];
+        if (P) ws->run[atomicAdd(&ws->nruns, 1u)] = (uint16_t)b;
     }
     __syncthreads();
 }
 
-// Phase D: sort the strings at positions [P, P + m) of buffer 1, the buckets
-// [b0, b1) (all of at most WAVE_SORT_MAX strings together), with the block
-// sorter. The run is one group at depth 0: its buckets are consecutive key
-// ranges and the keys at depth 0 are cached, so one sample-sort step over
-// the whole run (about 8 strings per bucket) replaces a step per bucket.
-// Bucket key ranges are recorded when the LCP array is wanted (the LCPs at
-// the run's bucket boundaries follow from them).
-__device__ __forceinline__ void wave_sort_run(const Work& w, WaveState* ws, WaveSmem& sm,
-                                              uint32_t b0, uint32_t b1, uint32_t (*wscratch)[32],
-                                              uint32_t* err)
+// Phase D: sort the strings at positions [P, P + m) of buffer 1 (m <=
+// SMALL_MAX), whole buckets, by the leaf sorter. The run is one segment at
+// depth 0: its buckets are consecutive key ranges and the keys at depth 0 are
+// cached.
+__device__ __forceinline__ void wave_sort_run(const Work& w, WaveState* ws, WaveSmem& sm, uint32_t B,
+                                              uint32_t P, uint32_t m, uint64_t* red)
 {
-    BlockSmem<WAVE_SORT_MAX>& bs = sm.u.sort;
-    const uint32_t P = sm.start[b0], m = sm.start[b1] - P;
     if (m == 0) return;
+    if (w.lcp) wave_note_run(w, ws, sm.start, B, P, m, red);
+    if (m == 1) {
+        if (threadIdx.x == 0) w.perm[P] = h_id(w, __ldcg(w.hnd[1] + P));
+        return;
+    }
+    SegState<WAVE_G>& seg = sm.u.sort.seg;
+#pragma unroll 4
     for (uint32_t i = threadIdx.x; i < m; i += WAVE_THREADS) {
-        bs.hnd[i] = __ldcg(w.hnd[1] + P + i);
-        bs.key[i] = __ldcg(w.keys[1] + P + i);
+        seg.hnd[i] = __ldcg(w.hnd[1] + P + i);
+        seg.idx[idx_at(i)] = (uint16_t)i;
     }
-    if (threadIdx.x == 0) {
-        bs.ng = 0;
-        bs.nw = 0;
-        if (m > 1) blk_push<WAVE_SORT_MAX, WAVE_THREADS>(bs, 0, m, 0u, true, err);
-    }
-    __syncthreads();
-    if (w.lcp) {
-        for (uint32_t b = b0 + threadIdx.x; b < b1; b += WAVE_THREADS) {
-            const uint32_t st = sm.start[b], c = sm.start[b + 1] - st;
-            if (c == 0 || (b & 1)) continue;  // '=' buckets: the splitter is their key
-            uint64_t mn = ~0ull, mx = 0;
-            for (uint32_t q = 0; q < c; ++q) {
-                mn = min(mn, bs.key[st - P + q]);
-                mx = max(mx, bs.key[st - P + q]);
-            }
-            ws->bmin[b] = mn;
-            ws->bmax[b] = mx;
-        }
-    }
-    block_sort_groups<WAVE_SORT_MAX, WAVE_THREADS>(w, bs, P, m, 1, wscratch, err);
+    sort_segment<WAVE_G>(w, seg, sm.u.sort.tail, P, m, 1, 0, true);
     __syncthreads();
 }
 
-// w.cur must be 0: the wave's leftovers (big segments, deep groups) go to
-// the lists of parity 1, with their strings in buffer 1.
-__global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws, uint32_t L,
+// Draw and sort S samples (at most E * WAVE_THREADS) into samp, the same ones
+// in every block.
+template <int E>
+__device__ __forceinline__ void wave_samples(const Work& w, uint32_t S, uint64_t* samp)
+{
+    uint64_t x[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint32_t i = threadIdx.x + e * WAVE_THREADS;
+        const uint64_t h = mix64(0x7761766573616d70ull ^ i);
+        const uint32_t r = (uint32_t)(((h >> 32) * w.n) >> 32);
+        x[e] = i < S ? load_key(w.chars, w.nchars, __ldg(w.offs + r)) : ~0ull;
+    }
+    group_sort<E, WAVE_G, false>(x, samp);
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < E; ++e) samp[threadIdx.x * E + e] = x[e];
+    __syncthreads();
+}
+
+// L: levels of the splitter tree, over: samples per splitter (1 or 2).
+// w.cur must be 0: the wave's leftovers (big segments, tied runs, deep
+// groups) go to the lists of parity 1, with their strings in buffer 1.
+__global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws, uint32_t L, uint32_t over, uint32_t window,
                                                           uint32_t limit, int trace)
 {
-    const long long c0 = clock64();
-    long long cl = c0;
+    long long cl = clock64();
     auto lap = [&](int k) {  // phase k ended here (tracing only)
         if (!trace || threadIdx.x) return;
         const long long t = clock64();
@@ -204,7 +218,6 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
     };
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WaveSmem& sm = *reinterpret_cast<WaveSmem*>(smem_raw);
-    __shared__ uint32_t wscratch[WAVE_THREADS / 32][32];
     __shared__ uint32_t tmp[32];
     __shared__ uint64_t red[2];
     __shared__ uint32_t task, big_at;
@@ -214,93 +227,40 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
     const uint32_t per_blk = (n + G - 1) / G;  // <= WAVE_TILE_MAX (host)
     const uint32_t t0 = min(blockIdx.x * per_blk, n), t1 = min(t0 + per_blk, n);
 
-    // ---- A: keys of the tile; samples and tree (block 0) ----------------
-    for (uint32_t b = blockIdx.x * WAVE_THREADS + threadIdx.x; b < (uint32_t)WAVE_BKT;
-         b += G * WAVE_THREADS)
-        ws->gcount[b] = 0;
+    // ---- A: keys of the tile; samples and tree -------------------------------
     if (blockIdx.x == 0 && threadIdx.x == 0 && w.chars[w.nchars - 1] != 0)
         set_error(err, ERR_UNTERMINATED);
-    uint64_t key[WAVE_PER], hnd[WAVE_PER];
+    uint64_t key[WAVE_PER];
 #pragma unroll
     for (int j = 0; j < WAVE_PER; ++j) {
         const uint32_t i = t0 + threadIdx.x + j * WAVE_THREADS;
         key[j] = 0;
-        hnd[j] = 0;
         if (i < t1) {
             const uint64_t off = __ldg(w.offs + i);
             if (off >= w.nchars) set_error(err, ERR_OFFSET);
-            hnd[j] = h_make(w, i, off);
             key[j] = load_key(w.chars, w.nchars, off);
         }
     }
-    // 2^(L+1) samples (oversampling factor 2, hpp:1388), drawn and sorted in
-    // chunks of WAVE_SAMPLE_CHUNK by the first blocks
-    const uint32_t S = 2u << L;
-    const uint32_t chunk = min(S, WAVE_SAMPLE_CHUNK);
-    for (uint32_t c = blockIdx.x; c < S / chunk; c += G) {
-        uint64_t* samp = sm.u.abc.m[0];
-        if (threadIdx.x < chunk) {
-            const uint64_t h = mix64(0x7761766573616d70ull ^ (c * chunk + threadIdx.x));
-            const uint32_t r = (uint32_t)(((h >> 32) * n) >> 32);
-            samp[threadIdx.x] = load_key(w.chars, w.nchars, __ldg(w.offs + r));
-        }
-        __syncthreads();
-        bitonic_sort_block(samp, chunk);
-        if (threadIdx.x < chunk) ws->samp[c * chunk + threadIdx.x] = samp[threadIdx.x];
-        __syncthreads();
-    }
-    lap(0);
-    if (!wave_barrier(ws, 1, err, limit)) return;
-    lap(1);
-    // input errors are all flagged in phase A: every block sees the same
-    // bits here and leaves together
-    if (*(volatile uint32_t*)err & (ERR_OFFSET | ERR_UNTERMINATED)) return;
-
-    // ---- B: the splitter tree (every block), classify, count, reserve -----
-    // Merge the sorted sample chunks (merge path: each thread makes 8
-    // consecutive outputs of a pair of runs), then the splitters are every
-    // second sample and the tree is their level order.
-    uint64_t* src = sm.u.abc.m[0];
-    uint64_t* dst = sm.u.abc.m[1];
-    for (uint32_t i = threadIdx.x; i < S; i += WAVE_THREADS) src[i] = __ldcg(ws->samp + i);
-    __syncthreads();
-    for (uint32_t R = chunk; R < S; R <<= 1) {
-        for (uint32_t o0 = 8 * threadIdx.x; o0 < S; o0 += 8 * WAVE_THREADS) {
-            const uint64_t* A = src + (o0 / (2 * R)) * (2 * R);
-            const uint64_t* Bv = A + R;
-            const uint32_t d = o0 % (2 * R);
-            // A-run members among the first d outputs (ties: A first)
-            uint32_t lo = d > R ? d - R : 0u, hi = min(d, R);
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (A[mid] <= Bv[d - mid - 1]) lo = mid + 1; else hi = mid;
-            }
-            uint32_t i = lo, j = d - lo;
-            uint64_t* out = dst + (o0 - d) + d;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const bool ta = j >= R || (i < R && A[i] <= Bv[j]);
-                out[q] = ta ? A[i] : Bv[j];
-                if (ta) ++i; else ++j;
-            }
-        }
-        __syncthreads();
-        uint64_t* t = src;
-        src = dst;
-        dst = t;
-    }
-    uint64_t* tree = dst;  // src holds the sorted samples
+    uint64_t* samp = sm.u.abc.samp;
+    const uint32_t S = over << L;
+    if (S <= 2u * WAVE_THREADS) wave_samples<2>(w, S, samp);
+    else if (S <= 4u * WAVE_THREADS) wave_samples<4>(w, S, samp);
+    else wave_samples<8>(w, S, samp);
+    uint64_t* tree = sm.u.abc.tree;
     uint32_t* cnt = sm.u.abc.cnt;
     if (blockIdx.x == 0)
-        for (uint32_t j = threadIdx.x; j < k; j += WAVE_THREADS) ws->spl[j] = src[2 * j + 1];
+        for (uint32_t j = threadIdx.x; j < k; j += WAVE_THREADS) ws->spl[j] = samp[over * (j + 1) - (over - 1)];
     for (uint32_t v = 1 + threadIdx.x; v <= k; v += WAVE_THREADS) {
         const uint32_t h = 31 - __clz((int)v);
         const uint32_t p = v - (1u << h);
         const uint32_t r = ((2 * p + 1) << (L - 1 - h)) - 1;  // in-order rank
-        tree[v] = src[2 * r + 1];
+        tree[v] = samp[over * (r + 1) - (over - 1)];
     }
     for (uint32_t b = threadIdx.x; b < B; b += WAVE_THREADS) cnt[b] = 0;
     __syncthreads();
+    lap(0);
+
+    // ---- B: classify, count, reserve ---------------------------------------------
     uint32_t pk[WAVE_PER];  // (bucket << 16) | rank inside the tile's share
 #pragma unroll
     for (int j = 0; j < WAVE_PER; ++j) {
@@ -325,8 +285,12 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
         const uint32_t c = cnt[b];
         cnt[b] = c ? atomicAdd(&ws->gcount[b], c) : 0u;
     }
-    if (!wave_barrier(ws, 2, err, limit)) return;
+    lap(1);
+    if (!wave_barrier(ws, 1, err, limit)) return;
     lap(2);
+    // input errors are all flagged in phase A: every block sees the same
+    // bits here and leaves together
+    if (*(volatile uint32_t*)err & (ERR_OFFSET | ERR_UNTERMINATED)) return;
 
     // ---- C: bucket starts, scatter ----------------------------------------
     for (uint32_t b = threadIdx.x; b < B; b += WAVE_THREADS) sm.start[b] = __ldcg(ws->gcount + b);
@@ -337,6 +301,7 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
 #pragma unroll
     for (int j = 0; j < WAVE_PER; ++j) {
         if (pk[j] == 0xFFFFFFFFu) continue;
+        const uint32_t i = t0 + threadIdx.x + j * WAVE_THREADS;
         const uint32_t b = pk[j] >> 16;
         const uint32_t dest = sm.start[b] + cnt[b] + (pk[j] & 0xFFFFu);
         if (dest >= n) {  // counts and starts disagree
@@ -344,33 +309,33 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
             continue;
         }
         w.keys[1][dest] = key[j];
-        w.hnd[1][dest] = hnd[j];
+        w.hnd[1][dest] = h_make(w, i, __ldg(w.offs + i));
     }
-    if (!wave_barrier(ws, 3, err, limit)) return;
+    if (!wave_barrier(ws, 2, err, limit)) return;
     lap(3);
-    (void)c0;
 
-    // ---- D: buckets over WAVE_WINDOW strings, one block each --------------
+    // ---- D: buckets over `window` strings, one block each ----------------------
     for (uint32_t b = blockIdx.x; b < B; b += G) {
         const uint32_t P = sm.start[b], c = sm.start[b + 1] - P;
-        if (c <= (uint32_t)WAVE_WINDOW) continue;
+        if (c <= window) continue;
         const uint64_t s = (b & 1) ? __ldcg(ws->spl + (b >> 1)) : 0ull;
         if ((b & 1) && key_terminated(s)) {
+            if (w.lcp) wave_note_run(w, ws, sm.start, B, P, c, red);
             for (uint32_t q = threadIdx.x; q < c; q += WAVE_THREADS) {
                 w.perm[P + q] = h_id(w, __ldcg(w.hnd[1] + P + q));
                 if (w.lcp && q) w.lcp[P + q] = lcp_key_depth(s);
             }
-        } else if (c <= (uint32_t)WAVE_SORT_MAX) {
-            wave_sort_run(w, ws, sm, b, b + 1, wscratch, err);
+        } else if (c <= (uint32_t)SMALL_MAX) {
+            wave_sort_run(w, ws, sm, B, P, c, red);
         } else {
-            if (w.lcp && !(b & 1)) wave_range_block(w, ws, b, P, c, red);
+            if (w.lcp) wave_note_run(w, ws, sm.start, B, P, c, red);
             if (threadIdx.x == 0)
                 push_seg(w, 1, (b & 1) ? Seg{P, c, 8u, 1u} : Seg{P, c, 0u, 1u | META_VALID});
         }
         __syncthreads();
     }
     // ---- D: windows of small buckets ---------------------------------------
-    const uint32_t ntask = (n + WAVE_WINDOW - 1) / WAVE_WINDOW;
+    const uint32_t ntask = (n + window - 1) / window;
     while (true) {
         if (threadIdx.x == 0) {
             task = atomicAdd(&ws->next_task, 1u);
@@ -379,20 +344,16 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
         __syncthreads();
         const uint32_t t = task;
         if (t >= ntask) break;
-        const uint32_t lo = t * WAVE_WINDOW, hi = min(lo + WAVE_WINDOW, n);
+        const uint32_t lo = t * window, hi = min(lo + window, n);
         const uint32_t b_lo = wave_lower(sm.start, B, lo);
         const uint32_t b_hi = wave_lower(sm.start, B, hi);
-        // at most one bucket over WAVE_WINDOW strings starts in a window
+        // at most one bucket over `window` strings starts in a window
         for (uint32_t b = b_lo + threadIdx.x; b < b_hi; b += WAVE_THREADS)
-            if (sm.start[b + 1] - sm.start[b] > (uint32_t)WAVE_WINDOW) atomicMin(&big_at, b);
+            if (sm.start[b + 1] - sm.start[b] > window) atomicMin(&big_at, b);
         __syncthreads();
-        const uint32_t bb = big_at;
-        if (bb < b_hi) {
-            wave_sort_run(w, ws, sm, b_lo, bb, wscratch, err);
-            wave_sort_run(w, ws, sm, bb + 1, b_hi, wscratch, err);
-        } else {
-            wave_sort_run(w, ws, sm, b_lo, b_hi, wscratch, err);
-        }
+        const uint32_t bb = min(big_at, b_hi);
+        wave_sort_run(w, ws, sm, B, sm.start[b_lo], sm.start[bb] - sm.start[b_lo], red);
+        if (bb < b_hi) wave_sort_run(w, ws, sm, B, sm.start[bb + 1], sm.start[b_hi] - sm.start[bb + 1], red);
         __syncthreads();  // task and big_at are rewritten next round
     }
     if (!w.lcp) {
@@ -400,16 +361,14 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
         return;
     }
 
-    // ---- LCPs at the bucket boundaries ---------------------------------------
-    if (!wave_barrier(ws, 4, err, limit)) return;
-    for (uint32_t b = blockIdx.x * WAVE_THREADS + threadIdx.x; b < B; b += G * WAVE_THREADS) {
+    // ---- LCPs at the first positions of the runs --------------------------------
+    if (!wave_barrier(ws, 3, err, limit)) return;
+    const uint32_t nruns = __ldcg(&ws->nruns);
+    for (uint32_t q = blockIdx.x * WAVE_THREADS + threadIdx.x; q < nruns; q += G * WAVE_THREADS) {
+        const uint32_t b = __ldcg(ws->run + q);
         const uint32_t P = sm.start[b];
-        if (P == 0 || sm.start[b + 1] == P) continue;
-        uint32_t p = b - 1;  // previous non-empty bucket
-        while (sm.start[p] == P) --p;
-        const uint64_t hi_prev = (p & 1) ? __ldcg(ws->spl + (p >> 1)) : __ldcg(ws->bmax + p);
-        const uint64_t lo_this = (b & 1) ? __ldcg(ws->spl + (b >> 1)) : __ldcg(ws->bmin + b);
-        w.lcp[P] = lcp_key_type(hi_prev, lo_this);
+        const uint32_t p = wave_lower(sm.start, B, P) - 1;  // previous non-empty bucket
+        w.lcp[P] = lcp_key_type(__ldcg(ws->bmax + p), __ldcg(ws->bmin + b));
     }
     lap(4);
 }

@@ -355,6 +355,8 @@ static int setup_kernels()
                                                                sizeof(WaveSmem)));
         g_wave_blocks[dev] = coop ? (uint32_t)(per_sm * sms) : 0u;
     }
+    PSS_CUDA(cudaFuncSetAttribute(k_one<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)segs_smem<16>(1, true)));
     PSS_CUDA(cudaFuncSetAttribute(k_tiny, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TINY_SMEM));
     PSS_CUDA(cudaFuncSetAttribute(K_SEGS_A, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)segs_smem<1>(SEGS_A_WARPS, true)));
@@ -514,40 +516,56 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
     for (int k = 0; k < K_NCLASS; ++k) c->kstat[k] = KStat{};
     KTimer kt{c, st};
     const uint64_t out_bytes = lcp ? 8 : 4;  // perm (+ lcp) per string
-    // An input that fits one wave of resident k_wave blocks sorts in one
-    // cooperative launch; what it leaves (buckets over WAVE_SORT_MAX strings,
-    // deep groups) continues in the passes below from the lists of parity 1.
+    // An input of one leaf segment sorts in one block (k_one), one that fits
+    // one wave of resident k_wave blocks in one cooperative launch; what they
+    // leave (buckets over SMALL_MAX strings, tied runs, deep groups)
+    // continues in the passes below from the lists of parity 1.
     const uint32_t wave_cap = g_wave_blocks[c->device];
-    const bool wave = !d_inst && c->single_launch && n >= 2 && wave_cap > 0 &&
+    const bool one = !d_inst && c->single_launch && n >= 2 && n <= (uint32_t)SMALL_MAX;
+    const bool wave = !one && !d_inst && c->single_launch && n >= 2 && wave_cap > 0 &&
                       (uint64_t)n <= (uint64_t)wave_cap * WAVE_TILE_MAX;
     int cur = 0;
-    const bool suffix_try = !wave && !d_inst && c->suffix_doubling && n >= 2 && (uint64_t)n == nchars;
+    const bool suffix_try = !one && !wave && !d_inst && c->suffix_doubling && n >= 2 && (uint64_t)n == nchars;
     PSS_CUDA(cudaEventRecord(c->ev0, st));
-    if (wave) {
-        // the counters and the wave state's header are adjacent: one memset
+    uint32_t* hc = c->host_counters;
+    if (one) {
+        w.cur = 0;
+        kt.begin(K_WAVE);
+        if (n <= 256) k_one<1><<<1, 32, segs_smem<1>(1, true), st>>>(w, hc);
+        else if (n <= 1024) k_one<4><<<1, 128, segs_smem<4>(1, true), st>>>(w, hc);
+        else k_one<16><<<1, 512, segs_smem<16>(1, true), st>>>(w, hc);
+        kt.end(K_WAVE);
+        PSS_CUDA(cudaGetLastError());
+        cur = 1;
+    } else if (wave) {
+        // the counters and the wave state up to its splitters are adjacent: one memset
         const size_t head = (size_t)((unsigned char*)c->wave - (unsigned char*)w.counters) +
-                            offsetof(WaveState, gcount);
+                            offsetof(WaveState, spl);
         PSS_CUDA(cudaMemsetAsync(w.counters, 0, head, st));
-        uint32_t G = std::min<uint32_t>(wave_cap, std::max<uint32_t>(1u, (n + WAVE_WINDOW - 1) / WAVE_WINDOW));
+        // Windows small enough to give a short input's work to many blocks
+        // (7.8 k strings: 33 us with 256, 36 with 1024), large ones for the
+        // rest (a run is padded to 1024 words; 487 k digit strings: 96 us with
+        // 1024, 111 with 512). Buckets of 128 to 256 strings up to 2^18, then
+        // as WAVE_MAX_BITS allows. With one sample per splitter a bucket's
+        // size is exponential: two samples where its largest would take a
+        // block longer than sorting them twice over takes every block (487 k:
+        // 102 us with one, 96 with two; 300 k: 72 and 82), or would exceed
+        // SMALL_MAX (1.2 M: 311 us with the pass that takes, 188 without).
+        uint32_t window = n < (1u << 14) ? 256 : n < (1u << 16) ? 512 : WAVE_WINDOW_MAX;
+        uint32_t G = std::min<uint32_t>(wave_cap, (n + window - 1) / window);
         G = std::max<uint32_t>(G, (n + WAVE_TILE_MAX - 1) / WAVE_TILE_MAX);
-        // about 128 strings per bucket slot, at most WAVE_MAX_BITS levels
         const uint32_t lg = bit_length(n) - 1;
-        uint32_t L = std::min<uint32_t>(WAVE_MAX_BITS, lg > 8 ? lg - 7 : 1u);
+        uint32_t L = lg < 18 ? std::max<uint32_t>(1u, lg - 7) : std::min<uint32_t>(WAVE_MAX_BITS, lg - 8);
+        uint32_t over = (n >> L) > 340 ? 2 : 1;
         w.cur = 0;
         WaveState* ws = c->wave;
         uint32_t limit = c->wait_limit;
         int trace = c->trace ? 1 : 0;
-        void* args[] = {&w, &ws, &L, &limit, &trace};
+        void* args[] = {&w, &ws, &L, &over, &window, &limit, &trace};
         kt.begin(K_WAVE);
         PSS_CUDA(cudaLaunchCooperativeKernel((const void*)k_wave, dim3(G), dim3(WAVE_THREADS), args,
                                              sizeof(WaveSmem), st));
         kt.end(K_WAVE);
-        c->kstat[K_WAVE].launches += 1;
-        c->kstat[K_WAVE].strings += n;
-        // offset 8 + chars 8 read, key + handle 16 written and read back, output
-        c->kstat[K_WAVE].alg_bytes += (48 + out_bytes) * n;
-        stats.kernel_launches += 1;
-        stats.passes += 1;
         cur = 1;
     } else {
         PSS_CUDA(cudaMemsetAsync(w.counters, 0, 4 * C_COUNT, st));
@@ -563,8 +581,18 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         c->kstat[K_INIT].alg_bytes += 12ull * n;  // offset read + id write
         stats.kernel_launches += 2;
     }
-    uint32_t* hc = c->host_counters;
-    PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
+    if (one || wave) {
+        c->kstat[K_WAVE].launches += 1;
+        c->kstat[K_WAVE].strings += n;
+        // offset 8 + chars 8 read, output; the wave also writes key + handle
+        // 16 and reads them back
+        c->kstat[K_WAVE].alg_bytes += ((wave ? 48 : 16) + out_bytes) * n;
+        stats.kernel_launches += 1;
+        stats.passes += 1;
+        PSS_CUDA(cudaEventRecord(c->ev1, st));  // the end, when nothing is left over
+    }
+    // k_one has written the host's counters itself
+    if (!one) PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
     PSS_CUDA(cudaStreamSynchronize(st));
     kt.collect();
     uint32_t cnt[L_NCLASS], nstr[L_NCLASS];
@@ -582,7 +610,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         if (cudaMemcpy(cyc, c->wave->cycles, sizeof(cyc), cudaMemcpyDeviceToHost) == cudaSuccess)
             std::fprintf(stderr,
                          "pssgpu single launch: %u strings, SM cycles (max over blocks): keys + samples "
-                         "%llu, first barrier wait %llu, classify %llu, scatter %llu, bucket sorts %llu\n",
+                         "%llu, classify %llu, barrier wait %llu, scatter %llu, bucket sorts %llu\n",
                          n, cyc[0], cyc[1], cyc[2], cyc[3], cyc[4]);
     }
     const bool suffix = suffix_try && !err && hc[C_SFX] == 0;
@@ -773,7 +801,9 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         kt.end(K_DBL);
         if (rc) return rc;
     }
-    if (!err && lcp) {
+    // one launch was all there was to do
+    const bool whole = (one || wave) && npass == 0;
+    if (!err && lcp && hc[C_NBND]) {
         kt.begin(K_BOUNDARY);
         k_boundary_lcp<<<1184, 256, 0, st>>>(w);
         kt.end(K_BOUNDARY);
@@ -784,10 +814,12 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         k_localize<<<std::max(1u, (n + LOC_CHUNK - 1) / LOC_CHUNK), 256, 0, st>>>(perm, lcp, d_inst, ninst, n);
         stats.kernel_launches += 1;
     }
-    PSS_CUDA(cudaEventRecord(c->ev1, st));
-    PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
-    PSS_CUDA(cudaStreamSynchronize(st));
-    kt.collect();
+    if (!whole) {
+        PSS_CUDA(cudaEventRecord(c->ev1, st));
+        PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
+        PSS_CUDA(cudaStreamSynchronize(st));
+        kt.collect();
+    }
     if (lcp) {
         // boundary (position, depth) 8 + two perm reads 8 + two keys 16 + lcp 4
         c->kstat[K_BOUNDARY].strings += hc[C_NBND];

@@ -85,3 +85,23 @@ def test_leaf_sizes(pkg, orc, kind, with_lcp):
     for k in range(len(LEAF_SIZES)):
         b, e = int(inst[k]), int(inst[k + 1])
         check(orc, chars, offs[b:e], perm[b:e], lcp[b:e] if with_lcp else None)
+
+
+@pytest.mark.parametrize("n", [2, 31, 255, 256, 257, 1023, 1024, 1025, 2047, 4095, 4096, 4097, 4608, 16383, 16384,
+                               65536, 262144])
+@pytest.mark.parametrize("kind", ["letters", "acgt", "eighth", "prefix"])
+def test_single_launch_sizes(pkg, orc, kind, n):
+    """The one-block and single-launch sorts at the edges of their size
+    rules, with and without LCPs."""
+    if kind == "prefix" and n > 20000:
+        pytest.skip("one segment behind a prefix: the pass loop's tests")
+    rng = np.random.default_rng(n)
+    chars, offs = pkg.pack_strings(leaf_strings(kind, n, rng))
+    c = pkg.Context(0)
+    try:
+        perm, lcp = c.sort_host(chars, offs, lcp=True)
+        only, _ = c.sort_host(chars, offs, lcp=False)
+    finally:
+        c.close()
+    check(orc, chars, offs, perm, lcp)
+    check(orc, chars, offs, only, None)
