@@ -32,6 +32,7 @@ enum : uint32_t {
     META_BUF = 1u,    // which ping-pong buffer holds the segment
     META_VALID = 2u,  // keys at `depth` are cached in keys[buf]
     META_FINAL = 4u,  // all strings equal: copy out, LCP inside = depth
+    META_PERM = 8u,   // the strings' ids are in perm (groups of a suffix set)
 };
 
 __device__ __forceinline__ uint64_t bswap64(uint64_t x)

@@ -43,13 +43,12 @@ __device__ __forceinline__ uint32_t tree_bits_for(const Work& w, uint32_t m)
     // a tuned value for this size class, else about 128 strings per '<'
     // bucket, which the leaf sorters finish for less than finer splitting
     // costs (64 Mi prefix sort: 7.63 ms at 8 strings, 7.51 at 64, 7.41 at
-    // 128, 7.48 at 256; 613-instance batch: 535, 496, 478, 478 us); a suffix
-    // set's buckets go on to rank doubling, at about 8. At most pS5's 10 tree
-    // levels.
+    // 128, 7.48 at 256; 613-instance batch: 535, 496, 478, 478 us). At most
+    // pS5's 10 tree levels.
     const int lg = 31 - __clz((int)m);
     const uint32_t tuned = w.tree_bits_by_size[lg];
     if (tuned) return min((uint32_t)MAX_TREE_BITS, tuned);
-    return (uint32_t)min(MAX_TREE_BITS, max(1, lg - (w.suffix ? 3 : 7)));
+    return (uint32_t)min(MAX_TREE_BITS, max(1, lg - 7));
 }
 
 __global__ void k_tile_scan(Work w, uint32_t nbig)
@@ -148,7 +147,8 @@ __global__ void __launch_bounds__(1024) k_sample(Work w)
     }
     __syncthreads();
     uint32_t J = 0;  // chunks of the common-prefix jump
-    if (smin == smax && !key_terminated(smin)) {
+    const uint32_t K = w.kchars;  // chars of a chunk
+    if (smin == smax && !key_ends(w, smin)) {
         // Every sample shares the chunk at the segment depth: count the
         // further chunks that the first (up to blockDim) samples share with
         // sample 0, four per round, up to JMAX_CHUNKS. pS5 would advance such
@@ -163,15 +163,15 @@ __global__ void __launch_bounds__(1024) k_sample(Work w)
             __syncthreads();
             uint64_t rk[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) rk[q] = load_key(w.chars, w.nchars, ref + 8ull * (J + q));
+            for (int q = 0; q < 4; ++q) rk[q] = key_at(w, ref + (uint64_t)K * (J + q));
             uint32_t mine = 4;
             if (threadIdx.x < JS) {
                 const uint64_t o = h_off(w, shnd[threadIdx.x]) + sg.depth;
                 uint32_t e = 0;
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const uint64_t kq = load_key(w.chars, w.nchars, o + 8ull * (J + q));
-                    if (e == (uint32_t)q && kq == rk[q] && !key_terminated(kq)) e = q + 1;
+                    const uint64_t kq = key_at(w, o + (uint64_t)K * (J + q));
+                    if (e == (uint32_t)q && kq == rk[q] && !key_ends(w, kq)) e = q + 1;
                 }
                 mine = min(mine, e);
             }
@@ -186,15 +186,15 @@ __global__ void __launch_bounds__(1024) k_sample(Work w)
         // the shared chunks as keys, and the samples' keys behind them
         uint64_t* jp = w.jpre + (size_t)s * JMAX_CHUNKS;
         for (uint32_t c = threadIdx.x; c < J; c += blockDim.x)
-            jp[c] = load_key(w.chars, w.nchars, ref + 8ull * c);
+            jp[c] = key_at(w, ref + (uint64_t)K * c);
 #pragma unroll 8
         for (uint32_t i = threadIdx.x; i < S; i += blockDim.x)
-            samp[i] = h_key(w, shnd[i], sg.depth + 8 * J);
+            samp[i] = h_key(w, shnd[i], sg.depth + K * J);
         __syncthreads();
     }
     bitonic_sort_block(samp, S);
     if (threadIdx.x == 0) {
-        w.jump[s] = 8 * J;
+        w.jump[s] = K * J;
         atomicAdd(w.counters + C_P_BIG, sg.size);
         if (!valid || J) atomicAdd(w.counters + C_P_STALE, sg.size);
         if (J) {
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1536 / TILE_THREADS) k_classify(
     }
     const uint32_t L = w.tree_bits[s];
     const uint32_t J = w.jump[s];
-    const uint32_t nc = J / 8;
+    const uint32_t nc = J / w.kchars;
     const uint32_t k = (1u << L) - 1;
     const uint32_t B = seg_buckets(w, s);
     const uint64_t* gtree = w.tree + (size_t)s * 1024;
@@ -265,6 +265,14 @@ __global__ void __launch_bounds__(TILE_THREADS, 1536 / TILE_THREADS) k_classify(
             key = keys[p];
         } else if (!J) {
             key = h_key(w, hs[p], sg.depth);
+            keys[p] = key;
+        } else if (w.suffix) {
+            const uint64_t o = h_off(w, hs[p]) + sg.depth;
+            for (uint32_t c = 0; c < nc && !side; ++c) {
+                const uint64_t kc = packed_key(w, o + (uint64_t)c * w.kchars);
+                if (kc != jp[c]) side = kc < jp[c] ? -1 : 1;
+            }
+            if (!side) key = packed_key(w, o + J);
             keys[p] = key;
         } else {
             const uint64_t o = h_off(w, hs[p]) + sg.depth;
@@ -631,7 +639,7 @@ __global__ void __launch_bounds__(1024) k_children(Work w)
                     child = Seg{P, c, sg.depth, (uint32_t)nbuf};
                 } else if (tb & 1) {
                     const uint64_t key = spl[tb >> 1];
-                    if (key_terminated(key)) {
+                    if (key_ends(w, key)) {
                         const uint32_t v = dj + lcp_key_depth(key);
                         if (c <= FINAL_INLINE) {
                             for (uint32_t q = 0; q < c; ++q) {
@@ -643,20 +651,16 @@ __global__ void __launch_bounds__(1024) k_children(Work w)
                             child = Seg{P, c, v, (uint32_t)nbuf | META_FINAL};
                         }
                     } else if (w.suffix && c <= DBL_MAX) {
-                        // a suffix set: the group is sorted by rank doubling
-                        // after the passes
-                        const uint32_t at = atomicAdd(w.counters + C_DBL, 1u);
-                        if (at < w.dbl_cap) w.dbl[at] = Seg{P, c, dj + 8, (uint32_t)nbuf};
-                        else set_error(w.counters + C_ERR, ERR_OVERFLOW);
+                        push_dbl(w, Seg{P, c, dj + w.kchars, (uint32_t)nbuf});
                         inline_done = true;
                     } else {
-                        child = Seg{P, c, dj + 8, (uint32_t)nbuf};
+                        child = Seg{P, c, dj + w.kchars, (uint32_t)nbuf};
                     }
                 } else {
                     child = Seg{P, c, dj, (uint32_t)nbuf | META_VALID};
                 }
                 if (!inline_done) {
-                    cls = seg_class(w, c);
+                    cls = seg_class(c);
                     slot = atomicAdd(&lcnt[cls], 1u);
                     if (cls == L_BIG) {
                         const uint32_t tiles = (c + TILE - 1) / TILE;

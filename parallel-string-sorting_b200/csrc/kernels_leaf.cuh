@@ -201,17 +201,19 @@ constexpr uint64_t WORD_PAD = ~0ull >> 2;  // after every word (no padding where
 template <int IB>
 struct WordForm {
     uint64_t key0;
-    int cp;      // bits all keys share
-    int chars;   // chars of the key in the word: 8, or fewer when the index takes their place
-    __device__ __forceinline__ WordForm(uint64_t k0, uint64_t x) : key0(k0)
+    int cp;          // bits all keys share
+    uint32_t chars;  // chars of the key in the word: all, or those the index leaves room for
+    int low;         // bits below them
+    __device__ __forceinline__ WordForm(const Work& w, uint64_t k0, uint64_t x) : key0(k0)
     {
         cp = __clzll((long long)x);
-        chars = cp >= IB + 2 ? 8 : IB <= 6 ? 7 : 6;
-        static_assert(IB <= 14, "6 chars leave 16 bits, 2 of them on top");
+        chars = cp >= IB + 2 ? w.kchars : w.suffix ? (62u - IB) / w.kbits : IB <= 6 ? 7u : 6u;
+        low = cp >= IB + 2 ? 0 : 64 - (int)(chars * w.kbits);
+        static_assert(IB <= 14, "6 chars of 8 bits leave 16 bits, 2 of them on top");
     }
     __device__ __forceinline__ uint64_t make(uint64_t key, uint32_t i) const
     {
-        return (((key & (~0ull << (64 - 8 * chars))) << cp) >> 2) | i;
+        return (((key & (~0ull << low)) << cp) >> 2) | i;
     }
     // do two words hold the same chars?
     __device__ __forceinline__ static bool same(uint64_t a, uint64_t b) { return ((a ^ b) >> IB) == 0; }
@@ -223,10 +225,13 @@ struct WordForm {
     __device__ __forceinline__ uint64_t key(uint64_t word) const
     {
         return (((word & (~0ull << IB)) << 2) >> cp) |
-               (cp ? key0 & (~0ull << (64 - cp)) & (~0ull << (64 - 8 * chars)) : 0ull);
+               (cp ? key0 & (~0ull << (64 - cp)) & (~0ull << low) : 0ull);
     }
     // do strings with this key (key()'s value) end inside the word's chars?
-    __device__ __forceinline__ bool ended(uint64_t k) const { return ((k >> (64 - 8 * chars)) & 0xFF) == 0; }
+    __device__ __forceinline__ bool ended(const Work& w, uint64_t k) const
+    {
+        return !w.suffix && ((k >> low) & 0xFF) == 0;
+    }
 };
 
 // Runs of tied strings (at most 32 each) into warp windows of up to 32
@@ -377,7 +382,7 @@ __device__ __forceinline__ void tiny_warp_sort(const Work& w, TinyWarp& sm, cons
         for (uint32_t m = near; m; m &= m - 1) {
             const uint32_t i = __ffs(m) - 1;
             const uint64_t a = key[idx[i - 1]], b = key[idx[i]];
-            if (a == b && !key_terminated(b)) ties |= 1u << i;
+            if (a == b && !key_ends(w, b)) ties |= 1u << i;
             else if (w.lcp) sm.lcp[off + i] = sg.depth + (a != b ? lcp_key_type(a, b) : lcp_key_depth(b));
         }
     }
@@ -403,18 +408,27 @@ __device__ __forceinline__ void tiny_warp_sort(const Work& w, TinyWarp& sm, cons
     }
     if (!__any_sync(0xFFFFFFFFu, ties)) return;
     __syncwarp();
+    auto next_run = [&](uint32_t& start, uint32_t& len) {
+        if (!ties) return false;
+        const uint32_t i = __ffs(ties) - 1;  // >= 1
+        const uint32_t rest = ~(ties >> i);
+        const uint32_t ones = __ffs(rest) - 1;  // at most 31: bit 0 is never set
+        start = i - 1;
+        len = ones + 1;
+        ties &= i + ones >= 32 ? 0u : ~0u << (i + ones);
+        return true;
+    };
+    if (w.suffix) {
+        uint32_t start = 0, len = 0;
+        bool has = next_run(start, len);
+        while (__any_sync(0xFFFFFFFFu, has)) {
+            push_dbl_warp(w, has, Seg{sg.begin + start, len, sg.depth + w.kchars, META_PERM});
+            has = has && next_run(start, len);
+        }
+        return;
+    }
     tie_windows(
-        sm.scratch,
-        [&](uint32_t& start, uint32_t& len) {
-            if (!ties) return false;
-            const uint32_t i = __ffs(ties) - 1;  // >= 1
-            const uint32_t rest = ~(ties >> i);
-            const uint32_t ones = __ffs(rest) - 1;  // at most 31: bit 0 is never set
-            start = i - 1;
-            len = ones + 1;
-            ties &= i + ones >= 32 ? 0u : ~0u << (i + ones);
-            return true;
-        },
+        sm.scratch, next_run,
         [&](uint32_t owner, uint32_t start, uint32_t gs) {
             const bool real = gs < 32;
             const uint32_t o = __shfl_sync(0xFFFFFFFFu, off, owner);
@@ -605,6 +619,11 @@ __device__ __forceinline__ uint32_t sort_group(const Work& w, SegState<G>& sm, u
         diff = sm.diff;
     }
     if (diff == 0) {
+        if (w.suffix) {
+            for (uint32_t j = t; j < c; j += T) w.perm[begin + s + j] = h_id(w, sm.hnd[sm.idx[idx_at(s + j)]]);
+            if (t == 0) push_dbl(w, Seg{begin + s, c, d + w.kchars, META_PERM});
+            return 0;
+        }
         if (key_terminated(key0)) {  // all equal: any order
             for (uint32_t j = t; j < c; j += T) {
                 w.perm[begin + s + j] = h_id(w, sm.hnd[sm.idx[idx_at(s + j)]]);
@@ -627,7 +646,7 @@ __device__ __forceinline__ uint32_t sort_group(const Work& w, SegState<G>& sm, u
         }
         return 0;
     }
-    const WordForm<IB> form(key0, diff);
+    const WordForm<IB> form(w, key0, diff);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const uint32_t j = t + T * e;
@@ -652,7 +671,7 @@ __device__ __forceinline__ uint32_t sort_group(const Work& w, SegState<G>& sm, u
             l = d + form.lcp(prev, x[e]);
         } else {
             const uint64_t k = form.key(x[e]);
-            if (form.ended(k)) l = d + lcp_key_depth(k);
+            if (form.ended(w, k)) l = d + lcp_key_depth(k);
             else tied |= 1u << e;
         }
         if (w.lcp) slcp[lcp_at(i)] = l;
@@ -821,7 +840,7 @@ __device__ __forceinline__ uint32_t sort_runs(const Work& w, SegState<G>& sm, un
 }
 
 // The nt ties left in the group of c strings at offset s, whose runs share
-// `dep` chars: to the next pass when there are many, else runs of up to 32
+// `dep` chars: to the list dbl (a suffix set), to the next pass when there are many, else runs of up to 32
 // strings to warp windows and longer ones to the stack.
 template <int G>
 __device__ __forceinline__ void finish_ties(const Work& w, SegState<G>& sm, uint32_t begin, int buf, uint32_t s,
@@ -841,7 +860,7 @@ __device__ __forceinline__ void finish_ties(const Work& w, SegState<G>& sm, uint
     }
     // runs over `most` strings stay with this group's warps
     const bool pass_on = nt > LEAF_WINDOW_TIES * G;
-    const uint32_t most = pass_on ? LEAF_WINDOW_TIES * G : (uint32_t)WARP_GROUP_MAX;
+    const uint32_t most = w.suffix ? c : pass_on ? LEAF_WINDOW_TIES * G : (uint32_t)WARP_GROUP_MAX;
     auto next_run = [&](uint32_t& start, uint32_t& len) {
         while (starts) {
             start = 32 * v + __ffs(starts) - 1;
@@ -863,6 +882,15 @@ __device__ __forceinline__ void finish_ties(const Work& w, SegState<G>& sm, uint
         }
         return false;
     };
+    if (w.suffix) {
+        uint32_t start = 0, len = 0;
+        bool has = next_run(start, len);
+        while (__any_sync(0xFFFFFFFFu, has)) {
+            push_dbl_warp(w, has, Seg{begin + s + start, len, dep, META_PERM});
+            has = has && next_run(start, len);
+        }
+        return;
+    }
     if (pass_on) {
         // the next pass sorts the runs as segments of their own size, from the
         // segment's handles in the order reached here
@@ -912,7 +940,7 @@ __device__ __forceinline__ void sort_segment(const Work& w, SegState<G>& sm, uns
                       : c <= 128 * G ? sort_group<4, G>(w, sm, tail, begin, buf, s, c, d, cached, &chars)
                                      : sort_group<8, G>(w, sm, tail, begin, buf, s, c, d, cached, &chars);
         uint32_t dep = d + chars;
-        for (int r = 0; r < LEAF_RESORTS && nt > LEAF_RESORT_TIES * G; ++r) {
+        for (int r = 0; r < LEAF_RESORTS && nt > LEAF_RESORT_TIES * G && !w.suffix; ++r) {
             uint32_t runs = 0;
             const uint32_t k = collect_ties<G>(sm, c, &runs);
             nt = k <= 64 * G    ? sort_runs<2, G>(w, sm, tail, begin, s, c, k, runs, nt, dep, &chars)

@@ -132,7 +132,7 @@ static Sizes sizes_for(uint64_t n)
     Sizes s;
     s.n = std::max<uint64_t>(n, 1);
     // a segment of class c has more strings than the class below it holds
-    s.cap[L_BIG] = s.n / (SUFFIX_SMALL_MAX + 1) + 2;
+    s.cap[L_BIG] = s.n / (SMALL_MAX + 1) + 2;
     s.cap[L_SMALLC] = s.n / 1025 + 2;
     s.cap[L_SMALLB] = s.n / 257 + 2;
     s.cap[L_SMALLA] = s.n / (WARP_GROUP_MAX + 1) + 2;
@@ -393,103 +393,128 @@ static int ensure_buf(unsigned char** buf, uint64_t* have, uint64_t bytes)
     return PSSGPU_OK;
 }
 
-// Rank doubling over the ndbl groups the passes handed over (a suffix set):
-// ranks of every suffix, then rounds that sort each group by the rank of its
-// members' suffixes `depth` chars further, until every group is split into
-// single suffixes; with LCP output, the LCPs at the separated positions.
-// Works in the workspace's key and handle arrays, which the passes no longer
-// need. Caller holds c->mu; *err receives the device error bits.
-static int run_doubling(Ctx* c, Work& w, uint32_t ndbl, cudaStream_t st, pssgpu_stats& stats,
+// Finish the ndbl groups the passes handed over (a suffix set): chain rounds
+// while they leave less than three quarters of the groups, then rank
+// doubling; with LCP output, the LCP array.
+// Works in the workspace's key, handle and bucket arrays, which the passes no
+// longer need. Caller holds c->mu; *err receives the device error bits.
+static int run_doubling(Ctx* c, Work& w, uint32_t ndbl, uint32_t* lcp, cudaStream_t st, pssgpu_stats& stats,
                         uint32_t* err)
 {
     const uint32_t n = w.n;
     const uint64_t capn = c->cap.n;
     DblArrays a{};
-    a.text = w.chars;
-    a.ntext = w.nchars;
     a.isa = reinterpret_cast<uint32_t*>(w.keys[0]);
     a.gd[0] = a.isa + capn;
     a.gd[1] = reinterpret_cast<uint32_t*>(w.keys[1]);
     a.key = a.gd[1] + capn;
-    a.lb = w.lcp ? reinterpret_cast<uint32_t*>(w.hnd[0]) : nullptr;
     const int lcls[3] = {L_TINY, L_SMALLA, L_SMALLB};
     for (int k = 0; k < 3; ++k) {
         a.list[k][0] = w.list[lcls[k]][0];
         a.list[k][1] = w.list[lcls[k]][1];
         a.cap[k] = w.cap[lcls[k]];
     }
+    // chain bits and their levels: n / 31 * 4 bytes and a little, in the
+    // bucket ids' 2 n bytes
+    uint32_t* cb = reinterpret_cast<uint32_t*>(w.bkt);
+    uint32_t bits = n;
+    for (int lv = 0; lv < CHAIN_LEVELS; ++lv) {
+        a.chain[lv] = cb;
+        a.clen[lv] = (bits + 31) / 32;
+        cb += a.clen[lv];
+        bits = a.clen[lv];
+    }
     uint32_t* hc = c->host_counters;
-    const unsigned gblocks = std::min<uint32_t>(ndbl, 148u * 16u);
-    // marks of the handed-over positions, in the round-key array (free
-    // until the first round)
-    uint8_t* taken = reinterpret_cast<uint8_t*>(a.key);
     auto* members = reinterpret_cast<unsigned long long*>(w.counters + C_DBL_MEMB);
-    PSS_CUDA(cudaMemsetAsync(w.counters + C_DBL_CNT, 0, 4 * (C_COUNT - C_DBL_CNT), st));
-    PSS_CUDA(cudaMemsetAsync(taken, 0, n, st));
-    k_dbl_init<<<gblocks, 256, 0, st>>>(w, w.dbl, ndbl, a, taken, w.counters, members);
-    if (a.lb) PSS_CUDA(cudaMemsetAsync(a.lb, 0xFF, 4ull * n, st));
-    k_dbl_isa<<<1184, 256, 0, st>>>(w.perm, n, taken, a.isa);
-    stats.kernel_launches += 2;
-    c->kstat[K_DBL].launches += 2;
+    auto launched = [&](uint32_t k) {
+        stats.kernel_launches += k;
+        c->kstat[K_DBL].launches += k;
+    };
+    auto fetch = [&]() -> int {
+        PSS_CUDA(cudaGetLastError());
+        PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
+        PSS_CUDA(cudaStreamSynchronize(st));
+        return PSSGPU_OK;
+    };
+    int rc, par = 0;
     c->kstat[K_DBL].strings += n;
-    PSS_CUDA(cudaGetLastError());
-    PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
-    PSS_CUDA(cudaStreamSynchronize(st));
-    int par = 0;
-    // the depth of every group at least doubles per round after the first
-    // (n <= 2^32 chars): a loop beyond this many rounds is an internal error
+    PSS_CUDA(cudaMemsetAsync(w.counters + C_DBL_CNT, 0, 4 * (C_DBL_MEMB + 2 - C_DBL_CNT), st));
+    if (ndbl) {
+        PSS_CUDA(cudaMemsetAsync(a.isa, 0xFF, 4ull * n, st));
+        k_dbl_init<<<(ndbl + 255) / 256, 256, 0, st>>>(w, w.dbl, ndbl, a, members);
+        launched(1);
+    }
+    if ((rc = fetch())) return rc;
+    // the depth of every group at least doubles per rank round (n <= 2^32
+    // chars): a loop beyond this many rounds is an internal error
     constexpr int MAX_ROUNDS = 64;
+    bool chain = true;
+    uint64_t groups = 0;
     for (int round = 0; !hc[C_ERR]; ++round) {
         uint32_t cnt[3];
         for (int k = 0; k < 3; ++k) cnt[k] = std::min(hc[C_DBL_CNT + 3 * par + k], a.cap[k]);
         if (!cnt[0] && !cnt[1] && !cnt[2]) break;
         if (round >= MAX_ROUNDS) return fail(PSSGPU_ETIMEOUT, "rank doubling round limit exceeded");
         PSS_CUDA(cudaMemsetAsync(w.counters + C_DBL_CNT + 3 * (par ^ 1), 0, 12, st));
-        // round 0 sorts by text chars (dbl_round0_key); later rounds by the
-        // ranks of one snapshot, read first
-        const int round0 = round == 0;
-        if (!round0) {
+        const uint64_t total = (uint64_t)cnt[0] + cnt[1] + cnt[2];
+        const bool fill = chain && round > 0 && (round >= DBL_CHAIN_ROUNDS || 4 * total > 3 * groups);
+        if (fill) chain = false;
+        groups = total;
+        const uint32_t classes = (cnt[0] != 0) + (cnt[1] != 0) + (cnt[2] != 0);
+        if (chain) {
+            PSS_CUDA(cudaMemsetAsync(a.chain[0], 0, 4ull * a.clen[0], st));
+            for (int k = 0; k < 3; ++k)
+                if (cnt[k])
+                    k_dbl_link<<<(cnt[k] + 255) / 256, 256, 0, st>>>(a.list[k][par], cnt[k], w.perm, a);
+            for (int lv = 1; lv < CHAIN_LEVELS; ++lv)
+                k_chain_level<<<std::min<uint32_t>((a.clen[lv] + 7) / 8, 1184u), 256, 0, st>>>(
+                    a.chain[lv - 1], a.clen[lv - 1], a.chain[lv], a.clen[lv]);
+            for (int k = 0; k < 3; ++k)
+                if (cnt[k])
+                    k_dbl_chain_keys<<<(cnt[k] + 255) / 256, 256, 0, st>>>(a.list[k][par], cnt[k], w.perm, a, par);
+            launched(CHAIN_LEVELS - 1 + 2 * classes);
+        } else {
+            if (fill) {
+                k_dbl_fill<<<1184, 256, 0, st>>>(w.perm, n, a.isa, 0);
+                launched(1);
+            }
+            // the ranks of one snapshot
             if (cnt[0])
                 k_dbl_keys_small<<<(cnt[0] + 255) / 256, 256, 0, st>>>(a.list[0][par], cnt[0], w.perm, a,
                                                                        members);
             for (int k = 1; k < 3; ++k)
                 if (cnt[k])
                     k_dbl_keys<<<(cnt[k] + 7) / 8, 256, 0, st>>>(a.list[k][par], cnt[k], w.perm, a, members);
+            launched(classes);
         }
         if (cnt[0]) {
             constexpr uint32_t per_block = 8 * DBL_PER_WARP;  // 8 warps
             k_dbl_sort_small<<<(cnt[0] + per_block - 1) / per_block, 256, 0, st>>>(
-                a.list[0][par], cnt[0], w.perm, a, w.counters, par, round0);
+                w, a.list[0][par], cnt[0], w.perm, a, w.counters, par, chain);
         }
         if (cnt[1])
-            k_dbl_sort_block<DBL_MID><<<cnt[1], 256, 12 * DBL_MID, st>>>(a.list[1][par], w.perm, a,
-                                                                         w.counters, par, round0);
+            k_dbl_sort_block<DBL_MID><<<cnt[1], 256, 12 * DBL_MID, st>>>(w, a.list[1][par], w.perm, a,
+                                                                         w.counters, par, chain);
         if (cnt[2])
-            k_dbl_sort_block<DBL_MAX><<<cnt[2], 512, 12 * DBL_MAX, st>>>(a.list[2][par], w.perm, a,
-                                                                         w.counters, par, round0);
-        const uint32_t per_class = round0 ? 1 : 2;  // (keys and) sort
-        const uint32_t launched = (cnt[0] ? per_class : 0) + (cnt[1] ? per_class : 0) + (cnt[2] ? per_class : 0);
-        stats.kernel_launches += launched;
-        c->kstat[K_DBL].launches += launched;
-        PSS_CUDA(cudaGetLastError());
-        PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
-        PSS_CUDA(cudaStreamSynchronize(st));
+            k_dbl_sort_block<DBL_MAX><<<cnt[2], 512, 12 * DBL_MAX, st>>>(w, a.list[2][par], w.perm, a,
+                                                                         w.counters, par, chain);
+        launched(classes);
+        if ((rc = fetch())) return rc;
         if (c->trace)
-            std::fprintf(stderr, "pssgpu doubling round %d: groups %u / %u / %u (<=32 / <=%u / <=%u)\n",
-                         round, cnt[0], cnt[1], cnt[2], DBL_MID, DBL_MAX);
+            std::fprintf(stderr, "pssgpu %s round %d: groups %u / %u / %u (<=32 / <=%u / <=%u)\n",
+                         chain ? "chain" : "rank", round, cnt[0], cnt[1], cnt[2], DBL_MID, DBL_MAX);
         par ^= 1;
     }
     *err = hc[C_ERR];
-    // algorithmic bytes: every suffix's first rank (its position read, its
-    // rank written), then per group member and round its id and the rank
-    // `depth` chars further read, its id and new rank written
+    // algorithmic bytes: per group member and round its id and the chars or
+    // the rank `depth` further read, its id and new rank written
     const uint64_t memb = (uint64_t)hc[C_DBL_MEMB] | ((uint64_t)hc[C_DBL_MEMB + 1] << 32);
-    c->kstat[K_DBL].alg_bytes += 8ull * n + 16ull * memb;
-    if (!*err && a.lb) {
+    c->kstat[K_DBL].alg_bytes += 16ull * memb + (lcp ? 16ull * n : 0);
+    if (!*err && lcp) {
+        k_dbl_fill<<<1184, 256, 0, st>>>(w.perm, n, a.isa, 1);
         k_dbl_lcp<<<(unsigned)std::min<uint64_t>(((uint64_t)n + 255) / 256, 148ull * 16), 256, 0, st>>>(
-            w.chars, w.nchars, w.perm, a.isa, a.lb, w.lcp, n);
-        stats.kernel_launches += 1;
-        c->kstat[K_DBL].launches += 1;
+            w.chars, w.nchars, w.perm, a.isa, lcp, n);
+        launched(2);
         PSS_CUDA(cudaGetLastError());
     }
     return PSSGPU_OK;
@@ -510,6 +535,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
     w.n = n;
     w.perm = perm;
     w.lcp = lcp;
+    w.kbits = w.kchars = 8;
     set_handle_format(w, c->indirect_handles);
     memcpy(w.tree_bits_by_size, c->tree_bits_by_size, sizeof(w.tree_bits_by_size));
     pssgpu_stats stats{};
@@ -525,7 +551,8 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
     const bool wave = !one && !d_inst && c->single_launch && n >= 2 && wave_cap > 0 &&
                       (uint64_t)n <= (uint64_t)wave_cap * WAVE_TILE_MAX;
     int cur = 0;
-    const bool suffix_try = !one && !wave && !d_inst && c->suffix_doubling && n >= 2 && (uint64_t)n == nchars;
+    const bool suffix_try = !one && !wave && !d_inst && c->suffix_doubling && n > (uint32_t)SMALL_MAX &&
+                            (uint64_t)n == nchars;
     PSS_CUDA(cudaEventRecord(c->ev0, st));
     uint32_t* hc = c->host_counters;
     if (one) {
@@ -574,7 +601,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         k_roots<<<d_inst ? std::max(1u, std::min((ninst + 255) / 256, 148u * 16u)) : 1u, 256, 0, st>>>(
             w, d_inst, ninst);
         // every string a suffix of one text (n == nchars is necessary)?
-        if (suffix_try) k_suffix_check<<<1184, 256, 0, st>>>(chars, offs, n, w.counters + C_SFX);
+        if (suffix_try) k_suffix_check<<<1184, 256, 0, st>>>(chars, offs, n, w.counters + C_SFX, w.counters + C_ALPHA);
         kt.end(K_INIT);
         c->kstat[K_INIT].launches += 2;
         c->kstat[K_INIT].strings += n;
@@ -615,12 +642,29 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
     }
     const bool suffix = suffix_try && !err && hc[C_SFX] == 0;
     if (suffix) {
-        // groups of at least 2 strings: at most n / 2 of them
-        const uint64_t cap = (uint64_t)n / 2 + 2;
-        if ((rc = ensure_buf(&c->sfx, &c->sfx_bytes, 16 * cap))) return rc;
+        // groups of at least 2 strings: at most n / 2 of them; behind them the
+        // packed text, the bits of a char from the number of chars that occur
+        PackMap map{};
+        uint32_t sigma = 0;
+        for (uint32_t ch = 1; ch < 256; ++ch)
+            if ((hc[C_ALPHA + (ch >> 5)] >> (ch & 31)) & 1u) map.code[ch] = (uint8_t)++sigma;
+        w.kbits = std::max<uint32_t>(1, bit_length(sigma));
+        w.kchars = 64 / w.kbits;
+        w.kmask = ~0ull << (64 - w.kchars * w.kbits);
+        const uint64_t cap = (uint64_t)n / 2 + 2, words = ((uint64_t)n * w.kbits + 63) / 64 + 2;
+        if ((rc = ensure_buf(&c->sfx, &c->sfx_bytes, 16 * cap + 8 * words))) return rc;
         w.suffix = 1;
         w.dbl = reinterpret_cast<Seg*>(c->sfx);
         w.dbl_cap = (uint32_t)cap;
+        uint64_t* pt = reinterpret_cast<uint64_t*>(c->sfx + 16 * cap);
+        w.ptext = pt;
+        w.lcp = nullptr;  // the LCPs come last, in text order
+        kt.begin(K_DBL);
+        k_pack_text<<<(unsigned)std::min<uint64_t>((words + 255) / 256, 148ull * 16), 256, 0, st>>>(
+            chars, nchars, w.kbits, map, pt, words);
+        kt.end(K_DBL);
+        c->kstat[K_DBL].launches += 1;
+        stats.kernel_launches += 1;
     }
     auto pending = [&]() {
         return cnt[L_BIG] || cnt[L_TINY] || cnt[L_SMALLA] || cnt[L_SMALLB] || cnt[L_SMALLC] || ndeep;
@@ -795,9 +839,9 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         err = hc[C_ERR];
         cur = nxt;
     }
-    if (!err && suffix && hc[C_DBL]) {
+    if (!err && suffix && (hc[C_DBL] || lcp)) {
         kt.begin(K_DBL);
-        rc = run_doubling(c, w, std::min(hc[C_DBL], w.dbl_cap), st, stats, &err);
+        rc = run_doubling(c, w, std::min(hc[C_DBL], w.dbl_cap), lcp, st, stats, &err);
         kt.end(K_DBL);
         if (rc) return rc;
     }
@@ -2011,7 +2055,7 @@ void pssgpu_sort_strings_out(unsigned char** strings, unsigned char** output, si
 // pssgpu_sort_device_noalloc sorts at most PSSGPU_NOALLOC_MAX_STRINGS strings
 // with the small-segment kernel and allocates nothing. Its scratch -- the
 // string-handle buffer, the one segment descriptor and the counters that
-// kernel uses -- is the file-scope array below (16,576 bytes), which every
+// kernel uses -- is the file-scope array below (16,608 bytes), which every
 // device that loads this library holds until the process exits. In host code
 // the array's name is only a host-side stand-in: kernels get the device
 // address that cudaGetSymbolAddress returns, looked up once per device with

@@ -11,8 +11,6 @@ constexpr int MAX_TREE_BITS = 10;   // 1023 splitters, 2047 buckets (pS5's Defau
 constexpr int MAX_BKT = 2056;       // bucket slots per big segment: 2047 + the two prefix buckets
 constexpr int JMAX_CHUNKS = 32;     // common-prefix jump of one pass: at most 32 8-byte chunks
 constexpr int SMALL_MAX = 4096;     // largest segment the leaf sorters take
-constexpr int SUFFIX_SMALL_MAX = 1024;  // ... of a suffix set, whose larger groups are worth
-                                        // splitting for rank doubling
 constexpr int SMALL_THREADS = 256;
 constexpr int WARP_GROUP_MAX = 32;  // groups this small are finished by one warp
 constexpr int FINAL_INLINE = 64;    // equal-string buckets this small are copied inline
@@ -47,7 +45,8 @@ enum : int {
     C_DBL = 35,       // groups handed to rank doubling by the passes
     C_DBL_CNT = 36,   // + 3 * parity + class: rank-doubling round lists
     C_DBL_MEMB = 42,  // 64-bit (42, 43): members of the rank-doubling groups, summed over rounds
-    C_COUNT = 44
+    C_ALPHA = 44,     // suffix-set check: which of the 256 chars occur (8 words)
+    C_COUNT = 52
 };
 
 struct Work {
@@ -110,8 +109,16 @@ struct Work {
     // (0: the default rule), set from a tuning table
     uint8_t tree_bits_by_size[33];
     // Suffix sets (every string is a suffix of one text: offs[i] = i, no NUL
-    // before the last char): '=' groups of at most DBL_MAX strings below
-    // depth 8 go to the rank-doubling list instead of deeper passes.
+    // before the last char): the text is packed at kbits bits per char (its
+    // chars numbered from 1 in their order, 0 past the end), so a key holds
+    // kchars chars, 21 of a 4-letter text where bytes hold 8, and most
+    // suffixes are told apart by their first key. Groups of at most DBL_MAX
+    // that share a key go to the list dbl, which is finished by text rounds
+    // and rank doubling (kernels_suffix.cuh). No LCPs are written before that.
+    // kchars is 8 and kbits 8 otherwise.
+    const uint64_t* ptext;
+    uint64_t kmask;  // the kchars * kbits top bits
+    uint32_t kbits, kchars;
     int suffix;
     Seg* dbl;
     uint32_t dbl_cap;
@@ -125,9 +132,9 @@ __device__ __forceinline__ uint32_t seg_buckets(const Work& w, int s)
 }
 
 // list class of a segment
-__device__ __forceinline__ int seg_class(const Work& w, uint32_t size)
+__device__ __forceinline__ int seg_class(uint32_t size)
 {
-    if (size > (uint32_t)(w.suffix ? SUFFIX_SMALL_MAX : SMALL_MAX)) return L_BIG;
+    if (size > (uint32_t)SMALL_MAX) return L_BIG;
     return size > 1024 ? L_SMALLC : size > 256 ? L_SMALLB : size > (uint32_t)WARP_GROUP_MAX ? L_SMALLA : L_TINY;
 }
 
@@ -146,16 +153,66 @@ __device__ __forceinline__ uint64_t h_off(const Work& w, uint64_t h)
     return w.packed ? (h & w.hmask) : __ldg(w.offs + h);
 }
 
+// Key of the kchars chars of a packed text at position p (0 past its end).
+__device__ __forceinline__ uint64_t packed_key(const Work& w, uint64_t p)
+{
+    if (p >= w.nchars) return 0;
+    const uint64_t bit = p * w.kbits;
+    const uint64_t* q = w.ptext + (bit >> 6);
+    const uint32_t s = (uint32_t)bit & 63u;
+    const uint64_t hi = __ldg(q), lo = __ldg(q + 1);
+    return (s ? (hi << s) | (lo >> (64 - s)) : hi) & w.kmask;
+}
+
+// key at arena position p
+__device__ __forceinline__ uint64_t key_at(const Work& w, uint64_t p)
+{
+    return w.suffix ? packed_key(w, p) : load_key(w.chars, w.nchars, p);
+}
+
 // key of the string behind handle h at depth d
 __device__ __forceinline__ uint64_t h_key(const Work& w, uint64_t h, uint32_t d)
 {
-    return load_key(w.chars, w.nchars, h_off(w, h) + d);
+    return key_at(w, h_off(w, h) + d);
+}
+
+// Do strings that share this key end inside it (and so are equal)? Suffixes
+// of one text never are.
+__device__ __forceinline__ bool key_ends(const Work& w, uint64_t k)
+{
+    return !w.suffix && key_terminated(k);
+}
+
+// A tied group of a suffix set: the strings at [pos, pos + size), which share
+// depth chars, to the list dbl. META_PERM: their ids are in perm, else their
+// handles in buffer meta & META_BUF.
+__device__ __forceinline__ void push_dbl(const Work& w, const Seg& g)
+{
+    const uint32_t at = atomicAdd(w.counters + C_DBL, 1u);
+    if (at < w.dbl_cap) w.dbl[at] = g;
+    else set_error(w.counters + C_ERR, ERR_OVERFLOW);
+}
+
+// push_dbl for a whole warp: lanes with push set append g.
+__device__ __forceinline__ void push_dbl_warp(const Work& w, bool push, const Seg& g)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t m = __ballot_sync(0xffffffffu, push);
+    if (!m) return;
+    const int leader = __ffs(m) - 1;
+    uint32_t base = 0;
+    if (lane == (uint32_t)leader) base = atomicAdd(w.counters + C_DBL, (uint32_t)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (!push) return;
+    const uint32_t at = base + __popc(m & ((1u << lane) - 1u));
+    if (at < w.dbl_cap) w.dbl[at] = g;
+    else set_error(w.counters + C_ERR, ERR_OVERFLOW);
 }
 
 // Append segment c to its class's list of parity nxt.
 __device__ __forceinline__ void push_seg(const Work& w, int nxt, Seg c)
 {
-    const int cls = seg_class(w, c.size);
+    const int cls = seg_class(c.size);
     const uint32_t at = atomicAdd(w.counters + C_PAR * nxt + cls, 1u);
     if (at >= w.cap[cls]) {
         set_error(w.counters + C_ERR, ERR_OVERFLOW);
@@ -178,7 +235,7 @@ __device__ __forceinline__ void push_seg(const Work& w, int nxt, Seg c)
 __device__ __forceinline__ void push_seg_warp(const Work& w, int nxt, bool push, const Seg& c)
 {
     const uint32_t lane = threadIdx.x & 31;
-    const int cls = push ? seg_class(w, c.size) : -1;
+    const int cls = push ? seg_class(c.size) : -1;
 #pragma unroll
     for (int k = 0; k < L_NCLASS; ++k) {
         const uint32_t m = __ballot_sync(0xffffffffu, cls == k);

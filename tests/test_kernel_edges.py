@@ -105,3 +105,26 @@ def test_single_launch_sizes(pkg, orc, kind, n):
         c.close()
     check(orc, chars, offs, perm, lcp)
     check(orc, chars, offs, only, None)
+
+
+@pytest.mark.parametrize("with_lcp", [True, False])
+@pytest.mark.parametrize("sigma", [1, 2, 3, 4, 7, 8, 15, 16, 31, 32, 63, 64, 127, 128, 255])
+def test_suffix_alphabets(pkg, orc, sigma, with_lcp):
+    """Suffix sets over alphabets around the powers of two (the packed keys'
+    bits per char), with copies, copies of copies and a copy of all of it (the
+    chains' ends part into groups of several sizes)."""
+    rng = np.random.default_rng(sigma)
+    symbols = np.sort(rng.choice(np.arange(1, 256, dtype=np.uint8), sigma, replace=False))
+    t = rng.choice(symbols, 6000 + sigma)
+    t[3000:4500] = t[100:1600]
+    t[5000:5700] = t[3300:4000]
+    t = np.concatenate([t, t[2500:5900], t[:40]])
+    chars = np.concatenate([t, np.zeros(1, np.uint8)])
+    offs = np.arange(chars.shape[0], dtype=np.uint64)
+    c = pass_loop(pkg)
+    try:
+        perm, lcp = c.sort_host(chars, offs, lcp=with_lcp)
+        assert {k["name"]: k["launches"] for k in c.kernel_stats()}["doubling"] > 0
+    finally:
+        c.close()
+    check(orc, chars, offs, perm, lcp)
