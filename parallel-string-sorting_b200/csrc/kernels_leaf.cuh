@@ -58,6 +58,17 @@ __device__ __forceinline__ void cmp_exchange(uint64_t& a, uint64_t& b)
     a = lo;
 }
 
+// Key of the string behind handle h at depth d; SFX: a suffix set (whose keys
+// are packed and whose ties go to the list dbl; the leaf kernels are built for
+// each, as the one's code costs the other instruction cache: suffixes of a
+// 32 MiB text 3.46 ms with both in one kernel, 3.27 with either).
+template <bool SFX>
+__device__ __forceinline__ uint64_t leaf_key(const Work& w, uint64_t h, uint32_t d)
+{
+    if constexpr (SFX) return packed_key(w, h_off(w, h) + d);
+    else return load_key(w.chars, w.nchars, h_off(w, h) + d);
+}
+
 __device__ __forceinline__ void cmp_exchange(uint32_t& a, uint32_t& b)
 {
     const uint32_t lo = min(a, b);
@@ -198,7 +209,7 @@ __device__ __forceinline__ void group_sort(uint64_t (&x)[E], uint64_t* xb)
 // below the key's chars. x is the OR of its keys' differences from key0, not
 // 0.
 constexpr uint64_t WORD_PAD = ~0ull >> 2;  // after every word (no padding where index bits are all ones)
-template <int IB>
+template <int IB, bool SFX>
 struct WordForm {
     uint64_t key0;
     int cp;          // bits all keys share
@@ -207,8 +218,13 @@ struct WordForm {
     __device__ __forceinline__ WordForm(const Work& w, uint64_t k0, uint64_t x) : key0(k0)
     {
         cp = __clzll((long long)x);
-        chars = cp >= IB + 2 ? w.kchars : w.suffix ? (62u - IB) / w.kbits : IB <= 6 ? 7u : 6u;
-        low = cp >= IB + 2 ? 0 : 64 - (int)(chars * w.kbits);
+        if constexpr (SFX) {
+            chars = cp >= IB + 2 ? w.kchars : (62u - IB) / w.kbits;
+            low = cp >= IB + 2 ? 0 : 64 - (int)(chars * w.kbits);
+        } else {
+            chars = cp >= IB + 2 ? 8u : IB <= 6 ? 7u : 6u;
+            low = 64 - 8 * (int)chars;
+        }
         static_assert(IB <= 14, "6 chars of 8 bits leave 16 bits, 2 of them on top");
     }
     __device__ __forceinline__ uint64_t make(uint64_t key, uint32_t i) const
@@ -228,10 +244,7 @@ struct WordForm {
                (cp ? key0 & (~0ull << (64 - cp)) & (~0ull << low) : 0ull);
     }
     // do strings with this key (key()'s value) end inside the word's chars?
-    __device__ __forceinline__ bool ended(const Work& w, uint64_t k) const
-    {
-        return !w.suffix && ((k >> low) & 0xFF) == 0;
-    }
+    __device__ __forceinline__ bool ended(uint64_t k) const { return !SFX && ((k >> low) & 0xFF) == 0; }
 };
 
 // Runs of tied strings (at most 32 each) into warp windows of up to 32
@@ -292,7 +305,7 @@ struct TinyWarp {
 // The warp's segments, one per lane (sg.size 0: none; packed from lane
 // `first` on), `total` strings from row entries `off`; N the network. Sorts
 // and writes them.
-template <int N>
+template <int N, bool SFX>
 __device__ __forceinline__ void tiny_warp_sort(const Work& w, TinyWarp& sm, const Seg& sg, uint32_t first,
                                                uint32_t off, uint32_t total)
 {
@@ -330,7 +343,7 @@ __device__ __forceinline__ void tiny_warp_sort(const Work& w, TinyWarp& sm, cons
         if (stale) {
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u)
-                if (32 * (r0 + u) + lane < total && !(q[u].z & META_VALID)) v[u] = h_key(w, v[u], q[u].w);
+                if (32 * (r0 + u) + lane < total && !(q[u].z & META_VALID)) v[u] = leaf_key<SFX>(w, v[u], q[u].w);
         }
 #pragma unroll
         for (uint32_t u = 0; u < U; ++u) {
@@ -382,7 +395,7 @@ __device__ __forceinline__ void tiny_warp_sort(const Work& w, TinyWarp& sm, cons
         for (uint32_t m = near; m; m &= m - 1) {
             const uint32_t i = __ffs(m) - 1;
             const uint64_t a = key[idx[i - 1]], b = key[idx[i]];
-            if (a == b && !key_ends(w, b)) ties |= 1u << i;
+            if (a == b && (SFX || !key_terminated(b))) ties |= 1u << i;
             else if (w.lcp) sm.lcp[off + i] = sg.depth + (a != b ? lcp_key_type(a, b) : lcp_key_depth(b));
         }
     }
@@ -418,15 +431,14 @@ __device__ __forceinline__ void tiny_warp_sort(const Work& w, TinyWarp& sm, cons
         ties &= i + ones >= 32 ? 0u : ~0u << (i + ones);
         return true;
     };
-    if (w.suffix) {
+    if constexpr (SFX) {
         uint32_t start = 0, len = 0;
         bool has = next_run(start, len);
         while (__any_sync(0xFFFFFFFFu, has)) {
             push_dbl_warp(w, has, Seg{sg.begin + start, len, sg.depth + w.kchars, META_PERM});
             has = has && next_run(start, len);
         }
-        return;
-    }
+    } else
     tie_windows(
         sm.scratch, next_run,
         [&](uint32_t owner, uint32_t start, uint32_t gs) {
@@ -443,6 +455,7 @@ __device__ __forceinline__ void tiny_warp_sort(const Work& w, TinyWarp& sm, cons
         });
 }
 
+template <bool SFX>
 __global__ void __launch_bounds__(TINY_THREADS, 3) k_tiny(Work w, const Seg* list, uint32_t count, uint32_t per)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -484,9 +497,9 @@ __global__ void __launch_bounds__(TINY_THREADS, 3) k_tiny(Work w, const Seg* lis
         const uint32_t total = __shfl_sync(0xFFFFFFFFu, end, 31);
         if (!total) continue;
         const uint32_t off = part.size ? end - part.size : 0u;
-        if (most <= 8) tiny_warp_sort<8>(w, warps[warp], part, 16 * t, off, total);
-        else if (most <= 16) tiny_warp_sort<16>(w, warps[warp], part, 16 * t, off, total);
-        else tiny_warp_sort<32>(w, warps[warp], part, 16 * t, off, total);
+        if (most <= 8) tiny_warp_sort<8, SFX>(w, warps[warp], part, 16 * t, off, total);
+        else if (most <= 16) tiny_warp_sort<16, SFX>(w, warps[warp], part, 16 * t, off, total);
+        else tiny_warp_sort<32, SFX>(w, warps[warp], part, 16 * t, off, total);
         __syncwarp();
     }
 }
@@ -579,7 +592,7 @@ __device__ __forceinline__ uint32_t count_ties(SegState<G>& sm, uint32_t tied)
 // and the LCPs it finds. Returns how many strings tie with their predecessor
 // (marked in sm.tied; *chars deeper than d); a group whose keys are all equal
 // goes back to the stack behind its common prefix.
-template <int E, int G>
+template <int E, int G, bool SFX>
 __device__ __forceinline__ uint32_t sort_group(const Work& w, SegState<G>& sm, unsigned char* tail, uint32_t begin,
                                                int buf, uint32_t s, uint32_t c, uint32_t d, bool cached,
                                                uint32_t* chars)
@@ -595,7 +608,7 @@ __device__ __forceinline__ uint32_t sort_group(const Work& w, SegState<G>& sm, u
         const uint32_t j = t + T * e;
         x[e] = 0;
         if (j < c)
-            x[e] = cached ? __ldcg(w.keys[buf] + begin + j) : h_key(w, sm.hnd[sm.idx[idx_at(s + j)]], d);
+            x[e] = cached ? __ldcg(w.keys[buf] + begin + j) : leaf_key<SFX>(w, sm.hnd[sm.idx[idx_at(s + j)]], d);
     }
     uint64_t key0 = __shfl_sync(0xFFFFFFFFu, x[0], 0);
     if constexpr (G > 1) {
@@ -619,11 +632,11 @@ __device__ __forceinline__ uint32_t sort_group(const Work& w, SegState<G>& sm, u
         diff = sm.diff;
     }
     if (diff == 0) {
-        if (w.suffix) {
+        if constexpr (SFX) {
             for (uint32_t j = t; j < c; j += T) w.perm[begin + s + j] = h_id(w, sm.hnd[sm.idx[idx_at(s + j)]]);
             if (t == 0) push_dbl(w, Seg{begin + s, c, d + w.kchars, META_PERM});
             return 0;
-        }
+        } else {
         if (key_terminated(key0)) {  // all equal: any order
             for (uint32_t j = t; j < c; j += T) {
                 w.perm[begin + s + j] = h_id(w, sm.hnd[sm.idx[idx_at(s + j)]]);
@@ -645,8 +658,9 @@ __device__ __forceinline__ uint32_t sort_group(const Work& w, SegState<G>& sm, u
             sm.g_dep[at] = d + 8u * sm.jump;
         }
         return 0;
+        }
     }
-    const WordForm<IB> form(w, key0, diff);
+    const WordForm<IB, SFX> form(w, key0, diff);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const uint32_t j = t + T * e;
@@ -667,11 +681,11 @@ __device__ __forceinline__ uint32_t sort_group(const Work& w, SegState<G>& sm, u
         const uint64_t prev = e ? x[e > 0 ? e - 1 : 0] : up;
         if (i == 0 || i >= c) continue;
         uint32_t l = LEAF_TIED;
-        if (!WordForm<IB>::same(prev, x[e])) {
+        if (!WordForm<IB, SFX>::same(prev, x[e])) {
             l = d + form.lcp(prev, x[e]);
         } else {
             const uint64_t k = form.key(x[e]);
-            if (form.ended(w, k)) l = d + lcp_key_depth(k);
+            if (form.ended(k)) l = d + lcp_key_depth(k);
             else tied |= 1u << e;
         }
         if (w.lcp) slcp[lcp_at(i)] = l;
@@ -766,7 +780,7 @@ __device__ __forceinline__ uint32_t sort_runs(const Work& w, SegState<G>& sm, un
         const uint32_t j = t + T * e;
         x[e] = WORD_PAD;
         if (j < n) {
-            const uint64_t k = h_key(w, sm.hnd[sm.idx[idx_at(s + sm.tpos[j])]], d);
+            const uint64_t k = leaf_key<false>(w, sm.hnd[sm.idx[idx_at(s + sm.tpos[j])]], d);
             x[e] = ((uint64_t)sm.trun[j] << (62 - rb)) | ((k >> (64 - 8 * kc)) << ksh) | j;
         }
     }
@@ -842,7 +856,7 @@ __device__ __forceinline__ uint32_t sort_runs(const Work& w, SegState<G>& sm, un
 // The nt ties left in the group of c strings at offset s, whose runs share
 // `dep` chars: to the list dbl (a suffix set), to the next pass when there are many, else runs of up to 32
 // strings to warp windows and longer ones to the stack.
-template <int G>
+template <int G, bool SFX>
 __device__ __forceinline__ void finish_ties(const Work& w, SegState<G>& sm, uint32_t begin, int buf, uint32_t s,
                                             uint32_t c, uint32_t dep, uint32_t nt)
 {
@@ -860,7 +874,7 @@ __device__ __forceinline__ void finish_ties(const Work& w, SegState<G>& sm, uint
     }
     // runs over `most` strings stay with this group's warps
     const bool pass_on = nt > LEAF_WINDOW_TIES * G;
-    const uint32_t most = w.suffix ? c : pass_on ? LEAF_WINDOW_TIES * G : (uint32_t)WARP_GROUP_MAX;
+    const uint32_t most = SFX ? c : pass_on ? LEAF_WINDOW_TIES * G : (uint32_t)WARP_GROUP_MAX;
     auto next_run = [&](uint32_t& start, uint32_t& len) {
         while (starts) {
             start = 32 * v + __ffs(starts) - 1;
@@ -882,15 +896,14 @@ __device__ __forceinline__ void finish_ties(const Work& w, SegState<G>& sm, uint
         }
         return false;
     };
-    if (w.suffix) {
+    if constexpr (SFX) {
         uint32_t start = 0, len = 0;
         bool has = next_run(start, len);
         while (__any_sync(0xFFFFFFFFu, has)) {
             push_dbl_warp(w, has, Seg{begin + s + start, len, dep, META_PERM});
             has = has && next_run(start, len);
         }
-        return;
-    }
+    } else {
     if (pass_on) {
         // the next pass sorts the runs as segments of their own size, from the
         // segment's handles in the order reached here
@@ -911,12 +924,13 @@ __device__ __forceinline__ void finish_ties(const Work& w, SegState<G>& sm, uint
         const uint64_t r = warp_window(w, h, gs, dep, begin + q, false, 0ull, sm.scratch[warp], defer, (uint32_t)buf);
         if (real) w.perm[begin + q] = h_id(w, r);
     });
+    }
 }
 
 // Sort the segment of m strings at position begin by its group of G warps:
 // handles in sm.hnd (idx: 0..m-1), buf the buffer they came from, depth the
 // chars they share, cached whether keys[buf] holds their keys.
-template <int G>
+template <int G, bool SFX>
 __device__ __forceinline__ void sort_segment(const Work& w, SegState<G>& sm, unsigned char* tail, uint32_t begin,
                                              uint32_t m, int buf, uint32_t depth, bool cached)
 {
@@ -936,11 +950,11 @@ __device__ __forceinline__ void sort_segment(const Work& w, SegState<G>& sm, uns
         if (t == 0) sm.ng = n - 1;
         group_sync<G>();
         uint32_t chars = 0;
-        uint32_t nt = c <= 64 * G    ? sort_group<2, G>(w, sm, tail, begin, buf, s, c, d, cached, &chars)
-                      : c <= 128 * G ? sort_group<4, G>(w, sm, tail, begin, buf, s, c, d, cached, &chars)
-                                     : sort_group<8, G>(w, sm, tail, begin, buf, s, c, d, cached, &chars);
+        uint32_t nt = c <= 64 * G    ? sort_group<2, G, SFX>(w, sm, tail, begin, buf, s, c, d, cached, &chars)
+                      : c <= 128 * G ? sort_group<4, G, SFX>(w, sm, tail, begin, buf, s, c, d, cached, &chars)
+                                     : sort_group<8, G, SFX>(w, sm, tail, begin, buf, s, c, d, cached, &chars);
         uint32_t dep = d + chars;
-        for (int r = 0; r < LEAF_RESORTS && nt > LEAF_RESORT_TIES * G && !w.suffix; ++r) {
+        for (int r = 0; !SFX && r < LEAF_RESORTS && nt > LEAF_RESORT_TIES * G; ++r) {
             uint32_t runs = 0;
             const uint32_t k = collect_ties<G>(sm, c, &runs);
             nt = k <= 64 * G    ? sort_runs<2, G>(w, sm, tail, begin, s, c, k, runs, nt, dep, &chars)
@@ -949,14 +963,14 @@ __device__ __forceinline__ void sort_segment(const Work& w, SegState<G>& sm, uns
             if (!chars) break;
             dep += chars;
         }
-        if (nt) finish_ties<G>(w, sm, begin, buf, s, c, dep, nt);
+        if (nt) finish_ties<G, SFX>(w, sm, begin, buf, s, c, dep, nt);
         cached = false;
         group_sync<G>();
     }
 }
 
 // SEGS segments per block for G == 1, one for G > 1.
-template <int G, int SEGS, int BLOCKS>
+template <int G, int SEGS, int BLOCKS, bool SFX>
 __global__ void __launch_bounds__(32 * G * SEGS, BLOCKS) k_segs(Work w, const Seg* list, uint32_t count)
 {
     static_assert(G == 1 || SEGS == 1, "a block's barriers serve one segment");
@@ -983,7 +997,7 @@ __global__ void __launch_bounds__(32 * G * SEGS, BLOCKS) k_segs(Work w, const Se
         sm.hnd[i] = __ldcg(w.hnd[buf] + begin + i);
         sm.idx[idx_at(i)] = (uint16_t)i;
     }
-    sort_segment<G>(w, sm, tail, begin, m, buf, sg.depth, sg.meta & META_VALID);
+    sort_segment<G, SFX>(w, sm, tail, begin, m, buf, sg.depth, sg.meta & META_VALID);
 }
 
 // The whole sort of an input of at most 256 G strings, by one block: handles
@@ -1014,14 +1028,17 @@ __global__ void __launch_bounds__(32 * G) k_one(Work w, uint32_t* host_counters)
         sm.ntied = 1;
     }
     __syncthreads();
-    if (!sm.ntied) sort_segment<G>(w, sm, smem_raw + sizeof(SegState<G>), 0, w.n, 0, 0, false);
+    if (!sm.ntied) sort_segment<G, false>(w, sm, smem_raw + sizeof(SegState<G>), 0, w.n, 0, 0, false);
     __syncthreads();
     for (uint32_t k = t; k < (uint32_t)C_COUNT; k += T) host_counters[k] = __ldcg(w.counters + k);
 }
 
 constexpr int SEGS_A_WARPS = 8;
-#define K_SEGS_A k_segs<1, SEGS_A_WARPS, 3>
-#define K_SEGS_B k_segs<4, 1, 6>
-#define K_SEGS_C k_segs<16, 1, 2>
+template <bool SFX>
+constexpr auto k_segs_a = k_segs<1, SEGS_A_WARPS, 3, SFX>;
+template <bool SFX>
+constexpr auto k_segs_b = k_segs<4, 1, 6, SFX>;
+template <bool SFX>
+constexpr auto k_segs_c = k_segs<16, 1, 2, SFX>;
 
 }  // namespace pssgpu

@@ -179,7 +179,7 @@ __device__ __forceinline__ void wave_sort_run(const Work& w, WaveState* ws, Wave
         seg.hnd[i] = __ldcg(w.hnd[1] + P + i);
         seg.idx[idx_at(i)] = (uint16_t)i;
     }
-    sort_segment<WAVE_G>(w, seg, sm.u.sort.tail, P, m, 1, 0, true);
+    sort_segment<WAVE_G, false>(w, seg, sm.u.sort.tail, P, m, 1, 0, true);
     __syncthreads();
 }
 

@@ -357,13 +357,17 @@ static int setup_kernels()
     }
     PSS_CUDA(cudaFuncSetAttribute(k_one<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)segs_smem<16>(1, true)));
-    PSS_CUDA(cudaFuncSetAttribute(k_tiny, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TINY_SMEM));
-    PSS_CUDA(cudaFuncSetAttribute(K_SEGS_A, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)segs_smem<1>(SEGS_A_WARPS, true)));
-    PSS_CUDA(cudaFuncSetAttribute(K_SEGS_B, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)segs_smem<4>(1, true)));
-    PSS_CUDA(cudaFuncSetAttribute(K_SEGS_C, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)segs_smem<16>(1, true)));
+    for (int sfx = 0; sfx < 2; ++sfx) {
+        PSS_CUDA(cudaFuncSetAttribute(sfx ? k_tiny<true> : k_tiny<false>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TINY_SMEM));
+        PSS_CUDA(cudaFuncSetAttribute(sfx ? k_segs_a<true> : k_segs_a<false>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)segs_smem<1>(SEGS_A_WARPS, true)));
+        PSS_CUDA(cudaFuncSetAttribute(sfx ? k_segs_b<true> : k_segs_b<false>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)segs_smem<4>(1, true)));
+        PSS_CUDA(cudaFuncSetAttribute(sfx ? k_segs_c<true> : k_segs_c<false>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)segs_smem<16>(1, true)));
+    }
     PSS_CUDA(cudaFuncSetAttribute(k_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sizeof(ScatterSmem)));
     done[dev] = true;
@@ -700,7 +704,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         if (cnt[L_SMALLC]) {
             cudaStream_t s = small_stream(3);
             kt.begin(K_SMALLC);
-            K_SEGS_C<<<cnt[L_SMALLC], 512, segs_smem<16>(1, true), s>>>(w, w.list[L_SMALLC][cur], cnt[L_SMALLC]);
+            (suffix ? k_segs_c<true> : k_segs_c<false>)<<<cnt[L_SMALLC], 512, segs_smem<16>(1, true), s>>>(w, w.list[L_SMALLC][cur], cnt[L_SMALLC]);
             kt.end(K_SMALLC);
             c->kstat[K_SMALLC].launches += 1;
             stats.kernel_launches += 1;
@@ -709,7 +713,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
             cudaStream_t s = small_stream(0);
             kt.begin(K_TINY);
             const uint32_t per = tiny_per(cnt[L_TINY]), per_block = per * (TINY_THREADS / 32);
-            k_tiny<<<(cnt[L_TINY] + per_block - 1) / per_block, TINY_THREADS, TINY_SMEM, s>>>(
+            (suffix ? k_tiny<true> : k_tiny<false>)<<<(cnt[L_TINY] + per_block - 1) / per_block, TINY_THREADS, TINY_SMEM, s>>>(
                 w, w.list[L_TINY][cur], cnt[L_TINY], per);
             kt.end(K_TINY);
             c->kstat[K_TINY].launches += 1;
@@ -718,7 +722,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         if (cnt[L_SMALLA]) {
             cudaStream_t s = small_stream(1);
             kt.begin(K_SMALLA);
-            K_SEGS_A<<<(cnt[L_SMALLA] + SEGS_A_WARPS - 1) / SEGS_A_WARPS, 32 * SEGS_A_WARPS,
+            (suffix ? k_segs_a<true> : k_segs_a<false>)<<<(cnt[L_SMALLA] + SEGS_A_WARPS - 1) / SEGS_A_WARPS, 32 * SEGS_A_WARPS,
                        segs_smem<1>(SEGS_A_WARPS, w.lcp != nullptr), s>>>(w, w.list[L_SMALLA][cur], cnt[L_SMALLA]);
             kt.end(K_SMALLA);
             c->kstat[K_SMALLA].launches += 1;
@@ -739,7 +743,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         if (cnt[L_SMALLB]) {
             cudaStream_t s = small_stream(2);
             kt.begin(K_SMALLB);
-            K_SEGS_B<<<cnt[L_SMALLB], 128, segs_smem<4>(1, true), s>>>(w, w.list[L_SMALLB][cur], cnt[L_SMALLB]);
+            (suffix ? k_segs_b<true> : k_segs_b<false>)<<<cnt[L_SMALLB], 128, segs_smem<4>(1, true), s>>>(w, w.list[L_SMALLB][cur], cnt[L_SMALLB]);
             kt.end(K_SMALLB);
             c->kstat[K_SMALLB].launches += 1;
             stats.kernel_launches += 1;
