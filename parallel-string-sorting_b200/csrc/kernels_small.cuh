@@ -48,6 +48,8 @@ __device__ __forceinline__ uint32_t chunks_equal(const Work& w, uint64_t base, u
     }
 }
 
+constexpr int WINDOW_STEPS = 8;
+
 // Finish a warp window. Per lane on entry: the string handle of the slot,
 // mygrp = lane index where the slot's group starts (32 for an unused lane),
 // mydep = chars the group shares, mypos = output position of the slot, and
@@ -78,14 +80,40 @@ __device__ __forceinline__ uint64_t warp_window(const Work& w, uint64_t myh, uin
         if (A == 0) break;
         if (stalled >= 2) {
             // the last two rounds neither split a group nor finished a
-            // string: defer the groups, or move every active group to its
-            // common prefix, one group at a time, 64 chunks of 8 bytes per step
+            // string: move every active group to its common prefix. First
+            // every lane compares its string with its group's first one, 32
+            // chars a step, all groups at once (walking the members of one
+            // group after another took k_tiny 0.2 ms for 27 groups behind
+            // 48-char prefixes). Groups equal in WINDOW_STEPS steps are
+            // deferred, or walked one at a time, 64 chunks of 8 bytes a step.
             stalled = 0;
+            bool open = mystate == 0;  // this lane's group shared every chunk so far
+            {
+                const uint32_t same = __match_any_sync(0xffffffffu, mystate == 0 ? mygrp : 64u + lane);
+                const uint64_t first_h = __shfl_sync(0xffffffffu, myh, mygrp & 31u);
+                for (int step = 0; step < WINDOW_STEPS && __any_sync(0xffffffffu, open); ++step) {
+                    uint32_t e = 4;
+                    if (open && mygrp != lane) {
+                        uint64_t ra[4], rb[4];
+                        load_raw_chunks<4>(w.chars, w.nchars, h_off(w, first_h) + mydep, 4, ra);
+                        load_raw_chunks<4>(w.chars, w.nchars, h_off(w, myh) + mydep, 4, rb);
+#pragma unroll
+                        for (int q = 3; q >= 0; --q) {
+                            const uint64_t z = (ra[q] - 0x0101010101010101ull) & ~ra[q] & 0x8080808080808080ull;
+                            if (ra[q] != rb[q] || z) e = q;
+                        }
+                    }
+                    e = __reduce_min_sync(same, e);
+                    if (open) mydep += 8u * e;
+                    open = open && e == 4;
+                }
+            }
+            gstarts &= __ballot_sync(0xffffffffu, open);
             uint32_t todo = gstarts;
             if (defer_hnd) {
                 const int nxt = w.cur ^ 1;
-                const bool lead = mystate == 0 && mygrp == lane;
-                const uint32_t same = __match_any_sync(0xffffffffu, mystate == 0 ? mygrp : 64u + lane);
+                const bool lead = open && mygrp == lane;
+                const uint32_t same = __match_any_sync(0xffffffffu, open ? mygrp : 64u + lane);
                 uint32_t at = 0xFFFFFFFFu;
                 if (lead) {
                     at = atomicAdd(w.counters + C_DEEP + nxt, 1u);
@@ -93,7 +121,7 @@ __device__ __forceinline__ uint64_t warp_window(const Work& w, uint64_t myh, uin
                         w.deep[nxt][at] = Seg{mypos, (uint32_t)__popc(same), mydep, defer_meta};
                 }
                 const uint32_t D = __ballot_sync(0xffffffffu, lead && at < w.deep_cap);
-                if (mystate == 0 && ((D >> mygrp) & 1u)) {
+                if (open && ((D >> mygrp) & 1u)) {
                     defer_hnd[mypos] = myh;
                     mystate = 1;
                 }
