@@ -33,6 +33,7 @@ enum : uint32_t {
     META_VALID = 2u,  // keys at `depth` are cached in keys[buf]
     META_FINAL = 4u,  // all strings equal: copy out, LCP inside = depth
     META_PERM = 8u,   // the strings' ids are in perm (groups of a suffix set)
+    META_ROOT = 16u,  // as they came: position p holds string p, its handle is made from offs[p]
 };
 
 __device__ __forceinline__ uint64_t bswap64(uint64_t x)

@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(1024) k_sample(Work w)
     for (uint32_t i = threadIdx.x; i < S; i += blockDim.x) {
         const uint64_t h = mix64(((uint64_t)sg.begin << 32) ^ ((uint64_t)sg.depth << 12) ^ i);
         const uint32_t r = sg.begin + (uint32_t)(((h >> 32) * sg.size) >> 32);
-        shnd[i] = w.hnd[buf][r];
+        shnd[i] = handle_at(w, sg.meta, sg.begin, r);
         if (valid) samp[i] = w.keys[buf][r];
     }
     if (!valid) {
@@ -234,10 +234,9 @@ __global__ void __launch_bounds__(TILE_THREADS, 1536 / TILE_THREADS) k_classify(
     const uint32_t lo = sg.begin + (t - w.tile_start[s]) * TILE;
     const uint32_t hi = min(lo + TILE, sg.begin + sg.size);
     const int buf = sg.meta & META_BUF;
-    const uint64_t* hs = w.hnd[buf];
     if (sg.meta & META_FINAL) {
         for (uint32_t p = lo + threadIdx.x; p < hi; p += TILE_THREADS) {
-            w.perm[p] = h_id(w, hs[p]);
+            w.perm[p] = h_id(w, handle_at(w, sg.meta, sg.begin, p));
             if (w.lcp && p > sg.begin) w.lcp[p] = sg.depth;
         }
         return;
@@ -258,16 +257,25 @@ __global__ void __launch_bounds__(TILE_THREADS, 1536 / TILE_THREADS) k_classify(
     __syncthreads();
     const bool valid = (sg.meta & META_VALID) && !J;
     uint64_t* keys = w.keys[buf];
+    const bool root = sg.meta & META_ROOT;
+    const uint64_t* hs = handle_src(w, sg.meta);
+    bool bad = false;  // a root offset outside the arena
+    auto offset = [&](uint32_t p) {
+        const uint64_t x = __ldg(hs + p);
+        if (!root) return h_off(w, x);
+        bad |= x >= w.nchars;
+        return x;
+    };
     for (uint32_t p = lo + threadIdx.x; p < hi; p += TILE_THREADS) {
         uint64_t key = 0;
         int side = 0;  // -1: below the prefix, +1: above it
         if (valid) {
             key = keys[p];
         } else if (!J) {
-            key = h_key(w, hs[p], sg.depth);
+            key = key_at(w, offset(p) + sg.depth);
             keys[p] = key;
         } else if (w.suffix) {
-            const uint64_t o = h_off(w, hs[p]) + sg.depth;
+            const uint64_t o = offset(p) + sg.depth;
             for (uint32_t c = 0; c < nc && !side; ++c) {
                 const uint64_t kc = packed_key(w, o + (uint64_t)c * w.kchars);
                 if (kc != jp[c]) side = kc < jp[c] ? -1 : 1;
@@ -275,7 +283,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1536 / TILE_THREADS) k_classify(
             if (!side) key = packed_key(w, o + J);
             keys[p] = key;
         } else {
-            const uint64_t o = h_off(w, hs[p]) + sg.depth;
+            const uint64_t o = offset(p) + sg.depth;
             constexpr uint32_t NB = 7;  // chunks per batch: a 6-chunk prefix and its key
             for (uint32_t c0 = 0; c0 <= nc && !side; c0 += NB) {
                 uint64_t raw[NB];
@@ -314,6 +322,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1536 / TILE_THREADS) k_classify(
         w.bkt[p] = (uint16_t)b;
         atomicAdd(&hist[b], 1u);
     }
+    if (bad) set_error(w.counters + C_ERR, ERR_OFFSET);
     __syncthreads();
     uint32_t* bc = w.bcount + (size_t)s * MAX_BKT;
     uint32_t* row = w.tcount + (size_t)t * MAX_BKT;
@@ -499,7 +508,6 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) k_scatter(Work w, uint32_t nb
     const uint32_t B = seg_buckets(w, s);
     const int buf = sg.meta & META_BUF;
     const uint64_t* ikeys = w.keys[buf];
-    const uint64_t* ihs = w.hnd[buf];
     const uint32_t* dst = w.tcount + (size_t)t * MAX_BKT;
     uint32_t first[NBT];
 #pragma unroll
@@ -554,7 +562,10 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) k_scatter(Work w, uint32_t nb
         const uint32_t b = threadIdx.x + i * TILE_THREADS;
         if (b < B) sm.lcount[b] = first[i] - sm.lcount[b];
     }
-    // the handles, in flight while the keys go out
+    // the handles, in flight while the keys go out (a root segment's are made
+    // from the offsets when they are staged)
+    const bool root = sg.meta & META_ROOT;
+    const uint64_t* ihs = root ? w.offs : w.hnd[buf];
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
         const uint32_t p = lo + threadIdx.x + j * TILE_THREADS;
@@ -573,9 +584,11 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) k_scatter(Work w, uint32_t nb
         okeys[dest] = sm.stage[slot];
     }
     __syncthreads();
+    const uint32_t id0 = w.local ? sg.begin : 0u;
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
         const uint32_t slot = (ps[j / 2] >> (16 * (j & 1))) & 0xFFFFu;
+        if (root) v[j] = h_make(w, lo - id0 + threadIdx.x + j * TILE_THREADS, v[j]);
         if (slot != 0xFFFFu) sm.stage[slot] = v[j];
     }
     __syncthreads();
@@ -611,7 +624,8 @@ __global__ void __launch_bounds__(1024) k_children(Work w)
     const uint32_t* bc = w.bcount + (size_t)s * MAX_BKT;
     const uint32_t* bs = w.bstart + (size_t)s * MAX_BKT;
     const uint64_t* spl = w.spl + (size_t)s * 1024;
-    const uint64_t* hs = w.hnd[nbuf];
+    // no scatter: a root segment's strings are where they came
+    const uint32_t nmeta = w.bflags[s] ? (uint32_t)buf | (sg.meta & META_ROOT) : (uint32_t)nbuf;
     for (uint32_t base = 0; base < B; base += blockDim.x) {
         if (threadIdx.x < L_NCLASS) { lcnt[threadIdx.x] = 0; lstr[threadIdx.x] = 0; }
         if (threadIdx.x == 0) { ltiles = 0; lmulti = 0; lbnd = 0; }
@@ -631,33 +645,33 @@ __global__ void __launch_bounds__(1024) k_children(Work w)
                 bdep = (J && (b == B - 1 || bs[b] == bc[0])) ? sg.depth : dj;
             }
             if (c == 1) {
-                w.perm[P] = h_id(w, hs[P]);
+                w.perm[P] = h_id(w, handle_at(w, nmeta, sg.begin, P));
             } else {
                 const uint32_t tb = J ? b - 1 : b;  // tree bucket
                 bool inline_done = false;
                 if (edge) {
-                    child = Seg{P, c, sg.depth, (uint32_t)nbuf};
+                    child = Seg{P, c, sg.depth, nmeta};
                 } else if (tb & 1) {
                     const uint64_t key = spl[tb >> 1];
                     if (key_ends(w, key)) {
                         const uint32_t v = dj + lcp_key_depth(key);
                         if (c <= FINAL_INLINE) {
                             for (uint32_t q = 0; q < c; ++q) {
-                                w.perm[P + q] = h_id(w, hs[P + q]);
+                                w.perm[P + q] = h_id(w, handle_at(w, nmeta, sg.begin, P + q));
                                 if (w.lcp && q) w.lcp[P + q] = v;
                             }
                             inline_done = true;
                         } else {
-                            child = Seg{P, c, v, (uint32_t)nbuf | META_FINAL};
+                            child = Seg{P, c, v, nmeta | META_FINAL};
                         }
                     } else if (w.suffix && c <= DBL_MAX) {
-                        push_dbl(w, Seg{P, c, dj + w.kchars, (uint32_t)nbuf});
+                        push_dbl(w, Seg{P, c, dj + w.kchars, nmeta});
                         inline_done = true;
                     } else {
-                        child = Seg{P, c, dj + w.kchars, (uint32_t)nbuf};
+                        child = Seg{P, c, dj + w.kchars, nmeta};
                     }
                 } else {
-                    child = Seg{P, c, dj, (uint32_t)nbuf | META_VALID};
+                    child = Seg{P, c, dj, nmeta | META_VALID};
                 }
                 if (!inline_done) {
                     cls = seg_class(c);

@@ -335,9 +335,9 @@ __device__ __forceinline__ void tiny_warp_sort(const Work& w, TinyWarp& sm, cons
             const uint32_t f = 32 * (r0 + u) + lane;
             q[u] = sm.seg[row_seg(r0 + u)];
             if (f >= total) continue;
-            const int buf = q[u].z & META_BUF;
             const bool cached = q[u].z & META_VALID;
-            v[u] = (cached ? w.keys[buf] : w.hnd[buf])[q[u].x + f];
+            v[u] = cached ? w.keys[q[u].z & META_BUF][q[u].x + f]
+                          : handle_at_checked(w, q[u].z, q[u].x + q[u].y, q[u].x + f);
             stale = stale || !cached;
         }
         if (stale) {
@@ -408,7 +408,7 @@ __device__ __forceinline__ void tiny_warp_sort(const Work& w, TinyWarp& sm, cons
         for (uint32_t u = 0; u < U; ++u) {
             const uint32_t f = 32 * (r0 + u) + lane;
             q[u] = sm.seg[row_seg(r0 + u)];
-            if (f < total) h[u] = w.hnd[q[u].z & META_BUF][q[u].x + q[u].y + sm.idx[f]];
+            if (f < total) h[u] = handle_at(w, q[u].z, q[u].x + q[u].y, q[u].x + q[u].y + sm.idx[f]);
         }
 #pragma unroll
         for (uint32_t u = 0; u < U; ++u) {
@@ -449,7 +449,7 @@ __device__ __forceinline__ void tiny_warp_sort(const Work& w, TinyWarp& sm, cons
             const uint32_t dep = __shfl_sync(0xFFFFFFFFu, sg.depth + 8, owner);
             const uint32_t f = o + start + (lane - gs);
             const uint32_t pos = bo + f;
-            const uint64_t h = real ? w.hnd[meta & META_BUF][bo + o + sm.idx[f]] : ~0ull;
+            const uint64_t h = real ? handle_at(w, meta, bo + o, bo + o + sm.idx[f]) : ~0ull;
             const uint64_t r = warp_window(w, h, gs, dep, pos, false, 0ull, sm.scratch);
             if (real) w.perm[pos] = h_id(w, r);
         });
@@ -987,15 +987,26 @@ __global__ void __launch_bounds__(32 * G * SEGS, BLOCKS) k_segs(Work w, const Se
     const int buf = sg.meta & META_BUF;
     if (sg.meta & META_FINAL) {
         for (uint32_t i = t; i < m; i += T) {
-            w.perm[begin + i] = h_id(w, w.hnd[buf][begin + i]);
+            w.perm[begin + i] = h_id(w, handle_at(w, sg.meta, begin, begin + i));
             if (w.lcp && i) w.lcp[begin + i] = sg.depth;
         }
         return;
     }
+    const uint64_t* src = handle_src(w, sg.meta) + begin;
 #pragma unroll 8
     for (uint32_t i = t; i < m; i += T) {
-        sm.hnd[i] = __ldcg(w.hnd[buf] + begin + i);
+        sm.hnd[i] = __ldg(src + i);
         sm.idx[idx_at(i)] = (uint16_t)i;
+    }
+    if (sg.meta & META_ROOT) {  // the offsets become handles (short code beside the loads' loop)
+        bool bad = false;
+#pragma unroll 1
+        for (uint32_t i = t; i < m; i += T) {
+            const uint64_t x = sm.hnd[i];
+            bad |= x >= w.nchars;
+            sm.hnd[i] = h_make(w, w.local ? i : begin + i, x);
+        }
+        if (bad) set_error(w.counters + C_ERR, ERR_OFFSET);
     }
     sort_segment<G, SFX>(w, sm, tail, begin, m, buf, sg.depth, sg.meta & META_VALID);
 }

@@ -176,14 +176,13 @@ __global__ void __launch_bounds__(256) k_dbl_init(Work w, const Seg* __restrict_
     const uint32_t m = __reduce_add_sync(0xFFFFFFFFu, s.size);
     if ((threadIdx.x & 31) == 0 && m) atomicAdd(members, (unsigned long long)m);
     dbl_each_group(s, [&](const Seg& q, uint32_t, uint32_t first, uint32_t step) {
-        const uint64_t* hs = w.hnd[q.meta & META_BUF];
         for (uint32_t i = first; i < q.size; i += step) {
             const uint32_t p = q.begin + i;
             uint32_t x;
             if (q.meta & META_PERM) {
                 x = w.perm[p];
             } else {
-                x = h_id(w, hs[p]);
+                x = h_id(w, handle_at(w, q.meta, q.begin, p));
                 w.perm[p] = x;
             }
             a.isa[x] = q.begin;

@@ -44,23 +44,15 @@ static int fail(int code, const std::string& msg)
                         std::string(#call) + ": " + cudaGetErrorString(e_));       \
     } while (0)
 
-__global__ void k_init(Work w)
+// Root segments: the whole input, or one per instance of a batch (instance k
+// owns positions [inst[k], inst[k+1])). A one-string instance is final at
+// once; the batch's ids are global until k_localize unless w.local.
+__global__ void k_roots(Work w, const uint64_t* __restrict__ inst, uint32_t ninst)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0 && w.chars[w.nchars - 1] != 0)
         set_error(w.counters + C_ERR, ERR_UNTERMINATED);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < w.n; i += gridDim.x * blockDim.x) {
-        w.hnd[0][i] = h_make(w, i, w.offs[i]);
-        if (w.offs[i] >= w.nchars) set_error(w.counters + C_ERR, ERR_OFFSET);
-    }
-}
-
-// Root segments: the whole input, or one per instance of a batch (instance k
-// owns positions [inst[k], inst[k+1])). A one-string instance is final at
-// once; the batch's ids are global until k_localize.
-__global__ void k_roots(Work w, const uint64_t* __restrict__ inst, uint32_t ninst)
-{
     if (!inst) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) push_seg(w, 0, Seg{0u, w.n, 0u, 0u});
+        if (blockIdx.x == 0 && threadIdx.x == 0) push_seg(w, 0, Seg{0u, w.n, 0u, META_ROOT});
         return;
     }
     // warp-uniform trips, so that the list appends aggregate per warp
@@ -72,8 +64,11 @@ __global__ void k_roots(Work w, const uint64_t* __restrict__ inst, uint32_t nins
             b = (uint32_t)inst[k];
             e = (uint32_t)inst[k + 1];
         }
-        if (e - b == 1) w.perm[b] = b;
-        push_seg_warp(w, 0, e - b >= 2, Seg{b, e - b, 0u, 0u});
+        if (e - b == 1) {
+            if (__ldg(w.offs + b) >= w.nchars) set_error(w.counters + C_ERR, ERR_OFFSET);
+            w.perm[b] = w.local ? 0u : b;
+        }
+        push_seg_warp(w, 0, e - b >= 2, Seg{b, e - b, 0u, META_ROOT});
     }
 }
 
@@ -601,16 +596,14 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
     } else {
         PSS_CUDA(cudaMemsetAsync(w.counters, 0, 4 * C_COUNT, st));
         kt.begin(K_INIT);
-        k_init<<<1184, 256, 0, st>>>(w);
+        w.local = d_inst && !lcp && w.packed;
         k_roots<<<d_inst ? std::max(1u, std::min((ninst + 255) / 256, 148u * 16u)) : 1u, 256, 0, st>>>(
             w, d_inst, ninst);
         // every string a suffix of one text (n == nchars is necessary)?
         if (suffix_try) k_suffix_check<<<1184, 256, 0, st>>>(chars, offs, n, w.counters + C_SFX, w.counters + C_ALPHA);
         kt.end(K_INIT);
-        c->kstat[K_INIT].launches += 2;
-        c->kstat[K_INIT].strings += n;
-        c->kstat[K_INIT].alg_bytes += 12ull * n;  // offset read + id write
-        stats.kernel_launches += 2;
+        c->kstat[K_INIT].launches += 1;
+        stats.kernel_launches += 1;
     }
     if (one || wave) {
         c->kstat[K_WAVE].launches += 1;
@@ -622,10 +615,26 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         stats.passes += 1;
         PSS_CUDA(cudaEventRecord(c->ev1, st));  // the end, when nothing is left over
     }
-    // k_one has written the host's counters itself
-    if (!one) PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
-    PSS_CUDA(cudaStreamSynchronize(st));
-    kt.collect();
+    // what k_roots pushes for a single input is known here: no round trip
+    // (an arena without a NUL at its end shows after the first pass)
+    const bool known = !one && !wave && !d_inst && !suffix_try && n >= 2;
+    if (known) {
+        memset(hc, 0, 4 * C_COUNT);
+        const int cls = seg_class(n);
+        const uint32_t tiles = (n + TILE - 1) / TILE;
+        hc[cls] = 1;
+        if (cls == L_BIG) {
+            hc[C_NTILES] = tiles;
+            hc[C_MULTI] = tiles > (uint32_t)CHUNK;
+        } else {
+            hc[C_NSTR + cls] = n;
+        }
+    } else {
+        // k_one has written the host's counters itself
+        if (!one) PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
+        PSS_CUDA(cudaStreamSynchronize(st));
+        kt.collect();
+    }
     uint32_t cnt[L_NCLASS], nstr[L_NCLASS];
     for (int k = 0; k < L_NCLASS; ++k) {
         cnt[k] = hc[C_PAR * cur + k];
@@ -858,7 +867,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         c->kstat[K_BOUNDARY].launches += 1;
         stats.kernel_launches += 1;
     }
-    if (!err && d_inst) {
+    if (!err && d_inst && !w.local) {
         k_localize<<<std::max(1u, (n + LOC_CHUNK - 1) / LOC_CHUNK), 256, 0, st>>>(perm, lcp, d_inst, ninst, n);
         stats.kernel_launches += 1;
     }
