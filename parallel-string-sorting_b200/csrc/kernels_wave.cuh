@@ -53,7 +53,8 @@ struct WaveState {
     uint32_t bar;        // grid barrier arrivals
     uint32_t next_task;  // phase-D windows taken
     uint32_t nruns;      // runs recorded (LCP output only)
-    uint32_t pad[3];
+    uint32_t done;       // blocks that have ended
+    uint32_t pad[2];
     // with tracing on: the largest SM-clock cycles any block spent in phase
     // A, B, the wait behind it, C (+ its wait) and D (+ the LCPs)
     unsigned long long cycles[5];
@@ -207,7 +208,7 @@ __device__ __forceinline__ void wave_samples(const Work& w, uint32_t S, uint64_t
 // w.cur must be 0: the wave's leftovers (big segments, tied runs, deep
 // groups) go to the lists of parity 1, with their strings in buffer 1.
 __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws, uint32_t L, uint32_t over, uint32_t window,
-                                                          uint32_t limit, int trace)
+                                                          uint32_t limit, int trace, uint32_t* host_counters)
 {
     long long cl = clock64();
     auto lap = [&](int k) {  // phase k ended here (tracing only)
@@ -221,6 +222,21 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
     __shared__ uint32_t tmp[32];
     __shared__ uint64_t red[2];
     __shared__ uint32_t task, big_at;
+    __shared__ uint32_t ended;
+    // every block's way out: the last one hands the counters to the host (no
+    // copy after the kernel)
+    auto leave = [&]() {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            ended = atomicAdd(&ws->done, 1u);
+            __threadfence();
+        }
+        __syncthreads();
+        if (ended + 1 == gridDim.x)
+            for (uint32_t q = threadIdx.x; q < (uint32_t)C_COUNT; q += WAVE_THREADS)
+                host_counters[q] = __ldcg(w.counters + q);
+    };
     uint32_t* err = w.counters + C_ERR;
     const uint32_t G = gridDim.x, n = w.n;
     const uint32_t k = (1u << L) - 1, B = 2 * k + 1;
@@ -286,11 +302,11 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
         cnt[b] = c ? atomicAdd(&ws->gcount[b], c) : 0u;
     }
     lap(1);
-    if (!wave_barrier(ws, 1, err, limit)) return;
+    if (!wave_barrier(ws, 1, err, limit)) return leave();
     lap(2);
     // input errors are all flagged in phase A: every block sees the same
     // bits here and leaves together
-    if (*(volatile uint32_t*)err & (ERR_OFFSET | ERR_UNTERMINATED)) return;
+    if (*(volatile uint32_t*)err & (ERR_OFFSET | ERR_UNTERMINATED)) return leave();
 
     // ---- C: bucket starts, scatter ----------------------------------------
     for (uint32_t b = threadIdx.x; b < B; b += WAVE_THREADS) sm.start[b] = __ldcg(ws->gcount + b);
@@ -311,7 +327,7 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
         w.keys[1][dest] = key[j];
         w.hnd[1][dest] = h_make(w, i, __ldg(w.offs + i));
     }
-    if (!wave_barrier(ws, 2, err, limit)) return;
+    if (!wave_barrier(ws, 2, err, limit)) return leave();
     lap(3);
 
     // ---- D: buckets over `window` strings, one block each ----------------------
@@ -358,11 +374,11 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
     }
     if (!w.lcp) {
         lap(4);
-        return;
+        return leave();
     }
 
     // ---- LCPs at the first positions of the runs --------------------------------
-    if (!wave_barrier(ws, 3, err, limit)) return;
+    if (!wave_barrier(ws, 3, err, limit)) return leave();
     const uint32_t nruns = __ldcg(&ws->nruns);
     for (uint32_t q = blockIdx.x * WAVE_THREADS + threadIdx.x; q < nruns; q += G * WAVE_THREADS) {
         const uint32_t b = __ldcg(ws->run + q);
@@ -371,6 +387,7 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
         w.lcp[P] = lcp_key_type(__ldcg(ws->bmax + p), __ldcg(ws->bmin + b));
     }
     lap(4);
+    leave();
 }
 
 }  // namespace pssgpu

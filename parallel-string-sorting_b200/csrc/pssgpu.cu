@@ -587,7 +587,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         WaveState* ws = c->wave;
         uint32_t limit = c->wait_limit;
         int trace = c->trace ? 1 : 0;
-        void* args[] = {&w, &ws, &L, &over, &window, &limit, &trace};
+        void* args[] = {&w, &ws, &L, &over, &window, &limit, &trace, &hc};
         kt.begin(K_WAVE);
         PSS_CUDA(cudaLaunchCooperativeKernel((const void*)k_wave, dim3(G), dim3(WAVE_THREADS), args,
                                              sizeof(WaveSmem), st));
@@ -630,8 +630,8 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
             hc[C_NSTR + cls] = n;
         }
     } else {
-        // k_one has written the host's counters itself
-        if (!one) PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
+        // the single launches have written the host's counters themselves
+        if (!one && !wave) PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
         PSS_CUDA(cudaStreamSynchronize(st));
         kt.collect();
     }
