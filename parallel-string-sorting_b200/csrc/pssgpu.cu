@@ -72,6 +72,21 @@ __global__ void k_roots(Work w, const uint64_t* __restrict__ inst, uint32_t nins
     }
 }
 
+// The end of a pass of parity cur (-1: of another step): the counters go to
+// the host's copy (mapped memory), and those that the next pass appends to
+// start at 0. One small launch instead of a copy and four memsets, whose gaps
+// are idle time between passes (2 M strings with LCPs: 510 -> 477 us, 613-instance batch
+// 465 -> 440).
+__global__ void k_publish(uint32_t* __restrict__ counters, uint32_t* host, int cur)
+{
+    const uint32_t t = threadIdx.x;
+    if (t >= (uint32_t)C_COUNT) return;
+    host[t] = counters[t];
+    const bool stat = t >= (uint32_t)C_P_FIRST && t <= (uint32_t)C_P_LAST;
+    if (cur >= 0 && (t / C_PAR == (uint32_t)cur || t == (uint32_t)(C_MULTI + cur) || t == (uint32_t)(C_DEEP + cur) || stat))
+        counters[t] = 0;
+}
+
 // Batch output: ids relative to their instance; the first LCP of every
 // instance is 0. One block per chunk of LOC_CHUNK positions (work follows
 // the strings, whether a batch holds many small instances or a few large
@@ -430,8 +445,8 @@ static int run_doubling(Ctx* c, Work& w, uint32_t ndbl, uint32_t* lcp, cudaStrea
         c->kstat[K_DBL].launches += k;
     };
     auto fetch = [&]() -> int {
+        k_publish<<<1, 64, 0, st>>>(w.counters, hc, -1);
         PSS_CUDA(cudaGetLastError());
-        PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
         PSS_CUDA(cudaStreamSynchronize(st));
         return PSSGPU_OK;
     };
@@ -631,7 +646,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         }
     } else {
         // the single launches have written the host's counters themselves
-        if (!one && !wave) PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
+        if (!one && !wave) k_publish<<<1, 64, 0, st>>>(w.counters, hc, -1);
         PSS_CUDA(cudaStreamSynchronize(st));
         kt.collect();
     }
@@ -686,16 +701,13 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
     // it; the limit turns a pass structure that stops making progress into
     // an error instead of an endless loop.
     constexpr uint32_t MAX_PASSES = 1u << 20;
+    const bool last_is_pass = !lcp && !suffix && (!d_inst || w.local);  // nothing comes behind the passes
     uint32_t npass = 0;
     while (!err && pending()) {
         if (++npass > MAX_PASSES) return fail(PSSGPU_ETIMEOUT, "pass limit exceeded");
         const int nxt = cur ^ 1;
         const uint32_t nbig = cnt[L_BIG];
         w.cur = cur;
-        PSS_CUDA(cudaMemsetAsync(w.counters + C_PAR * nxt, 0, 4 * C_PAR, st));
-        PSS_CUDA(cudaMemsetAsync(w.counters + C_MULTI + nxt, 0, 4, st));
-        PSS_CUDA(cudaMemsetAsync(w.counters + C_DEEP + nxt, 0, 4, st));
-        PSS_CUDA(cudaMemsetAsync(w.counters + C_P_FIRST, 0, 4 * (C_P_LAST - C_P_FIRST + 1), st));
         if (nbig && ntiles > c->cap.tile_cap) return fail(PSSGPU_ECUDA, "tile capacity exceeded");
         // small classes: on the side streams (after everything queued on st
         // so far), or serially on st in profile mode so that the per-class
@@ -800,8 +812,9 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         }
         for (int q = 0; q < 4; ++q)
             if (joined[q]) PSS_CUDA(cudaStreamWaitEvent(st, c->join_ev[q], 0));
+        if (last_is_pass) PSS_CUDA(cudaEventRecord(c->ev1, st));  // the end, when it was this one
+        k_publish<<<1, 64, 0, st>>>(w.counters, hc, cur);
         PSS_CUDA(cudaGetLastError());
-        PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
         PSS_CUDA(cudaStreamSynchronize(st));
         kt.collect();
         {
@@ -852,15 +865,16 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         err = hc[C_ERR];
         cur = nxt;
     }
+    bool more = false;  // steps behind the passes (or the single launch)
     if (!err && suffix && (hc[C_DBL] || lcp)) {
+        more = true;
         kt.begin(K_DBL);
         rc = run_doubling(c, w, std::min(hc[C_DBL], w.dbl_cap), lcp, st, stats, &err);
         kt.end(K_DBL);
         if (rc) return rc;
     }
-    // one launch was all there was to do
-    const bool whole = (one || wave) && npass == 0;
     if (!err && lcp && hc[C_NBND]) {
+        more = true;
         kt.begin(K_BOUNDARY);
         k_boundary_lcp<<<1184, 256, 0, st>>>(w);
         kt.end(K_BOUNDARY);
@@ -868,12 +882,13 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         stats.kernel_launches += 1;
     }
     if (!err && d_inst && !w.local) {
+        more = true;
         k_localize<<<std::max(1u, (n + LOC_CHUNK - 1) / LOC_CHUNK), 256, 0, st>>>(perm, lcp, d_inst, ninst, n);
         stats.kernel_launches += 1;
     }
-    if (!whole) {
+    if (more || (npass ? !last_is_pass : !one && !wave)) {
         PSS_CUDA(cudaEventRecord(c->ev1, st));
-        PSS_CUDA(cudaMemcpyAsync(hc, w.counters, 4 * C_COUNT, cudaMemcpyDeviceToHost, st));
+        k_publish<<<1, 64, 0, st>>>(w.counters, hc, -1);
         PSS_CUDA(cudaStreamSynchronize(st));
         kt.collect();
     }
