@@ -57,7 +57,7 @@ __global__ void k_tile_scan(Work w, uint32_t nbig)
     const Seg* big = w.list[L_BIG][w.cur];
     const uint32_t per = (nbig + blockDim.x - 1) / blockDim.x;
     const uint32_t lo = min(threadIdx.x * per, nbig), hi = min(lo + per, nbig);
-    auto tiles = [&](uint32_t i) { return (big[i].size + TILE - 1) / TILE; };
+    auto tiles = [&](uint32_t i) { return seg_tiles(w, big[i].size); };
     auto chunks = [&](uint32_t i) { return (tiles(i) + CHUNK - 1) / CHUNK; };
     uint32_t s = 0, sc = 0;
     for (uint32_t i = lo; i < hi; ++i) {
@@ -231,8 +231,8 @@ __global__ void __launch_bounds__(TILE_THREADS, 1536 / TILE_THREADS) k_classify(
     const uint32_t t = blockIdx.x;
     const int s = find_tile_seg(w.tile_start, nbig, t);
     const Seg sg = w.list[L_BIG][w.cur][s];
-    const uint32_t lo = sg.begin + (t - w.tile_start[s]) * TILE;
-    const uint32_t hi = min(lo + TILE, sg.begin + sg.size);
+    const uint32_t lo = sg.begin + ((t - w.tile_start[s]) << w.tshift);
+    const uint32_t hi = min(lo + (1u << w.tshift), sg.begin + sg.size);
     const int buf = sg.meta & META_BUF;
     if (sg.meta & META_FINAL) {
         for (uint32_t p = lo + threadIdx.x; p < hi; p += TILE_THREADS) {
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(512) k_bstart(Work w)
     }
 }
 
-// Segments of more than CHUNK tiles (rare: over CHUNK * TILE strings) scan
+// Segments of more than CHUNK tiles (rare: over CHUNK tiles' strings) scan
 // their (tile, bucket) counts in chunks of CHUNK tiles: chunk sums, their
 // scan per bucket, then the tiles inside each chunk. The kernels loop over
 // chunks / segments with a fixed grid and skip the short segments.
@@ -502,8 +502,8 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) k_scatter(Work w, uint32_t nb
     const Seg sg = w.list[L_BIG][w.cur][s];
     const uint8_t L = w.tree_bits[s];
     if (!classified(L) || w.bflags[s]) return;
-    const uint32_t lo = sg.begin + (t - w.tile_start[s]) * TILE;
-    const uint32_t hi = min(lo + TILE, sg.begin + sg.size);
+    const uint32_t lo = sg.begin + ((t - w.tile_start[s]) << w.tshift);
+    const uint32_t hi = min(lo + (1u << w.tshift), sg.begin + sg.size);
     const uint32_t cnt = hi - lo;
     const uint32_t B = seg_buckets(w, s);
     const int buf = sg.meta & META_BUF;
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(1024) k_children(Work w)
                     cls = seg_class(c);
                     slot = atomicAdd(&lcnt[cls], 1u);
                     if (cls == L_BIG) {
-                        const uint32_t tiles = (c + TILE - 1) / TILE;
+                        const uint32_t tiles = seg_tiles(w, c);
                         atomicAdd(&ltiles, tiles);
                         if (tiles > (uint32_t)CHUNK) atomicAdd(&lmulti, 1u);
                     } else {

@@ -147,7 +147,10 @@ static Sizes sizes_for(uint64_t n)
     s.cap[L_SMALLB] = s.n / 257 + 2;
     s.cap[L_SMALLA] = s.n / (WARP_GROUP_MAX + 1) + 2;
     s.cap[L_TINY] = s.n / 2 + 2;
-    s.tile_cap = s.n / TILE + s.cap[L_BIG] + 1;
+    // whole tiles of every n that this workspace serves (tile_shift), and one
+    // more per segment
+    s.tile_cap = std::max({s.n >> 13, std::min<uint64_t>(s.n, TILE_MID_N) >> 12,
+                           std::min<uint64_t>(s.n, TILE_SMALL_N) >> 11}) + s.cap[L_BIG] + 1;
     // deep groups hold 2..32 strings; a fuller list falls back to walking
     // the group inside the block sorter
     s.deep_cap = s.n / 32 + 64;
@@ -550,6 +553,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
     w.perm = perm;
     w.lcp = lcp;
     w.kbits = w.kchars = 8;
+    w.tshift = tile_shift(n);
     set_handle_format(w, c->indirect_handles);
     memcpy(w.tree_bits_by_size, c->tree_bits_by_size, sizeof(w.tree_bits_by_size));
     pssgpu_stats stats{};
@@ -636,7 +640,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
     if (known) {
         memset(hc, 0, 4 * C_COUNT);
         const int cls = seg_class(n);
-        const uint32_t tiles = (n + TILE - 1) / TILE;
+        const uint32_t tiles = seg_tiles(w, n);
         hc[cls] = 1;
         if (cls == L_BIG) {
             hc[C_NTILES] = tiles;

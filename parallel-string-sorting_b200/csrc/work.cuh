@@ -5,7 +5,7 @@
 
 namespace pssgpu {
 
-constexpr int TILE = 8192;          // strings per classify / scatter tile
+constexpr int TILE = 8192;          // most strings per classify / scatter tile (Work::tshift)
 constexpr int TILE_THREADS = 512;   // 16 strings per thread
 constexpr int MAX_TREE_BITS = 10;   // 1023 splitters, 2047 buckets (pS5's DefaultTreebits)
 constexpr int MAX_BKT = 2056;       // bucket slots per big segment: 2047 + the two prefix buckets
@@ -101,6 +101,7 @@ struct Work {
     uint32_t* tcount;       // [tile_cap][MAX_BKT]
     uint32_t* ccount;       // [tile_cap][MAX_BKT]: chunk sums, then chunk bases
     uint32_t tile_cap;
+    uint32_t tshift;        // strings per tile: 2^tshift, at most TILE (tile_shift)
     int cur;               // parity of the lists read in this pass
     // Deep groups: groups of at most 32 strings that a block sorter's warp
     // window found stuck on a long common prefix, handed to k_deep (one warp
@@ -132,6 +133,22 @@ struct Work {
 __device__ __forceinline__ uint32_t seg_buckets(const Work& w, int s)
 {
     return (2u << w.tree_bits[s]) - 1 + (w.jump[s] ? 2u : 0u);
+}
+
+__host__ __device__ __forceinline__ uint32_t seg_tiles(const Work& w, uint32_t size)
+{
+    return (size + (1u << w.tshift) - 1) >> w.tshift;
+}
+
+// Strings per tile in a sort of n: fewer where 8192 would leave a thread 16
+// strings to gather one after another while SMs idle, or one wave of tiles
+// just over full (classify 53 -> 26 us for 143 tiles; 1.3 M strings 326 -> 303 us,
+// 4.2 M prefix strings 909 -> 875 with 4096); 8192 where tiles are plenty, as every
+// tile pays for its buckets (5 M suffixes 940 us with 8192, 948 with 4096).
+constexpr uint64_t TILE_MID_N = 9u << 19, TILE_SMALL_N = 1u << 19;
+__host__ __device__ constexpr uint32_t tile_shift(uint64_t n)
+{
+    return n > TILE_MID_N ? 13 : n > TILE_SMALL_N ? 12 : 11;
 }
 
 // list class of a segment
@@ -248,7 +265,7 @@ __device__ __forceinline__ void push_seg(const Work& w, int nxt, Seg c)
     }
     w.list[cls][nxt][at] = c;
     if (cls == L_BIG) {
-        const uint32_t tiles = (c.size + TILE - 1) / TILE;
+        const uint32_t tiles = seg_tiles(w, c.size);
         atomicAdd(w.counters + C_PAR * nxt + C_NTILES, tiles);
         if (tiles > (uint32_t)CHUNK) atomicAdd(w.counters + C_MULTI + nxt, 1u);
     } else {
@@ -269,7 +286,7 @@ __device__ __forceinline__ void push_seg_warp(const Work& w, int nxt, bool push,
         const uint32_t m = __ballot_sync(0xffffffffu, cls == k);
         if (!m) continue;
         const int leader = __ffs(m) - 1;
-        const uint32_t tiles = cls == k && k == L_BIG ? (c.size + TILE - 1) / TILE : 0u;
+        const uint32_t tiles = cls == k && k == L_BIG ? seg_tiles(w, c.size) : 0u;
         const uint32_t amount = __reduce_add_sync(0xffffffffu, cls != k ? 0u : k == L_BIG ? tiles : c.size);
         const uint32_t multi = __reduce_add_sync(0xffffffffu, tiles > (uint32_t)CHUNK ? 1u : 0u);
         uint32_t base = 0;

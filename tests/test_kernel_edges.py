@@ -128,3 +128,16 @@ def test_suffix_alphabets(pkg, orc, sigma, with_lcp):
     finally:
         c.close()
     check(orc, chars, offs, perm, lcp)
+
+
+@pytest.mark.parametrize("n", [4097, 6143, 6144, 6145, 524288, 524289, 528385])
+def test_pass_loop_tiles(pkg, orc, n):
+    """The pass loop at the edges of its tile sizes (2048 strings up to 2^19,
+    4096 above) and with a last tile of one string."""
+    chars, offs, _ = pkg.workloads.random_strings(n, 0, 12, b"abcde", n)
+    c = pass_loop(pkg)
+    try:
+        perm, lcp = c.sort_host(chars, offs, lcp=True)
+    finally:
+        c.close()
+    check(orc, chars, offs, perm, lcp)
