@@ -1736,7 +1736,7 @@ static uint32_t merge_piece_for(uint64_t n, uint64_t wave)
 {
     const uint64_t per_wave = (uint64_t)MERGE_PIECE * wave;
     const uint64_t waves = std::max<uint64_t>(1, (n + per_wave - 1) / per_wave);
-    const uint64_t p = (n + waves * wave - 1) / (waves * wave);
+    const uint64_t p = ((n + waves * wave - 1) / (waves * wave) + 7) & ~7ull;
     return (uint32_t)std::min<uint64_t>(MERGE_PIECE, std::max<uint64_t>(MERGE_PIECE_MIN, p));
 }
 
