@@ -19,7 +19,8 @@
 //   k_segs<4>   257..1024 strings: a block of 4 warps
 //   k_segs<16>  1025..4096 strings: a block of 16 warps
 //
-// All are bound by instructions (12 to 17 warp instructions per string).
+// All are bound by instructions (26 warp instructions per string in k_segs<16>,
+// issue slots 60% busy) and, the smaller ones, by their fetch.
 // Measured in the 64 Mi prefix sort, 67 M strings: 27, 32, 32 and 62 ps per
 // string. Sample-sort steps in shared memory with a warp window per 32
 // strings took 30 ps (2..32 strings), 66 (33..256) and 67 (257..1024), and
@@ -38,9 +39,8 @@
 namespace pssgpu {
 
 // Order of two 64-bit words. WORD62: both are below 2^62, so that their bits
-// are non-negative finite doubles in the same order, and the compare is one
-// DSETP on the FP64 pipe instead of two ISETP on the ALU, which bounds the
-// warp sorts (75% busy in k_segs<16>): 1.16 -> 1.07 ms for the 27.7 M strings that
+// are non-negative finite doubles in the same order, and the compare runs on
+// the FP64 pipe instead of the integer ALU, which bounds the warp sorts (75% busy in k_segs<16>): 1.16 -> 1.07 ms for the 27.7 M strings that
 // kernel sorts of the 100k-instance batch.
 template <bool WORD62>
 __device__ __forceinline__ bool word_less(uint64_t a, uint64_t b)
@@ -131,11 +131,20 @@ __device__ __forceinline__ void group_sync()
 // Every merge starts by comparing positions with their mirror in the merged
 // block, so all compares are ascending. Partner distances below E stay
 // inside a thread, those inside a warp are shuffles, longer ones go through
-// xb (32 * E * G words of shared memory, G > 1 only).
+// xb (32 * E * G words of shared memory, G > 1 only). A merge with log2(E) or
+// more of the longer ones takes that many of them, the mirror first, in one
+// exchange: each thread loads the E words that meet in them, compares them in
+// registers and stores them in place. That is 4 accesses per word and 3
+// barriers instead of 2 and 2 per distance, and half the compares: the 27.7 M
+// strings that k_segs<16> sorts of the 100k-instance batch 1.08 -> 1.04 ms, the
+// batch 2.035 -> 1.994 ms. Exchanges in place of the shuffles, too, were slower
+// (2.153 ms): the two shuffles of a distance cost less than shared accesses.
 template <int E, int G, bool WORD62>
 __device__ __forceinline__ void group_sort(uint64_t (&x)[E], uint64_t* xb)
 {
     constexpr uint32_t T = 32 * G;
+    constexpr int FB = E == 8 ? 3 : E == 4 ? 2 : 1;  // log2(E)
+    constexpr bool FUSED = E >= 4 && G >= E;
     const uint32_t t = G == 1 ? threadIdx.x & 31 : threadIdx.x;
     auto inner = [&](int j) {  // distances j, j/2, .., 1 inside the threads
 #pragma unroll
@@ -163,7 +172,44 @@ __device__ __forceinline__ void group_sort(uint64_t (&x)[E], uint64_t* xb)
 #pragma unroll 1
     for (uint32_t k = 2; k <= T; k <<= 1) {
         const bool lower = (t & (k >> 1)) == 0;
-        if (G == 1 || k <= 32) {
+        uint32_t j = k >> 2;
+        bool in_xb = false;  // xb holds x
+        if (FUSED && k >= 32 * E) {
+            // thread bits low .. low + FB - 1; the mirrors' order is the reverse
+            const int low = __ffs(k) - 1 - FB;  // at least 5
+            const uint32_t e = (t >> 5) & (E - 1), rest = t >> (5 + FB);
+            const uint32_t below = rest & ((1u << (low - 5)) - 1u);
+            const uint32_t r = (t & 31u) | (below << 5) | ((rest >> (low - 5)) << (low + FB));
+            uint64_t lo[E / 2], hi[E / 2];
+            publish();
+#pragma unroll
+            for (uint32_t v = 0; v < E / 2; ++v) {
+                const uint32_t p = r | (v << low);
+                lo[v] = xb[e * T + p];
+                hi[v] = xb[(E - 1 - e) * T + (p ^ (k - 1))];
+                cmp_exchange<WORD62>(lo[v], hi[v]);
+            }
+#pragma unroll
+            for (int d = E / 4; d > 0; d >>= 1) {
+#pragma unroll
+                for (int v = 0; v < E / 2; ++v)
+                    if (!(v & d)) {
+                        cmp_exchange<WORD62>(lo[v], lo[v + d]);
+                        cmp_exchange<WORD62>(hi[v + d], hi[v]);
+                    }
+            }
+#pragma unroll
+            for (uint32_t v = 0; v < E / 2; ++v) {
+                const uint32_t p = r | (v << low);
+                xb[e * T + p] = lo[v];
+                xb[(E - 1 - e) * T + (p ^ (k - 1))] = hi[v];
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < E; ++i) x[i] = xb[i * T + t];
+            j = k >> (FB + 1);
+            in_xb = true;
+        } else if (G == 1 || k <= 32) {
 #pragma unroll
             for (int e = 0; e < E / 2; ++e) {
                 const uint64_t y0 = __shfl_xor_sync(0xFFFFFFFFu, x[E - 1 - e], k - 1);
@@ -179,12 +225,12 @@ __device__ __forceinline__ void group_sort(uint64_t (&x)[E], uint64_t* xb)
                 if (word_less<WORD62>(y, x[e]) == lower) x[e] = y;
             }
         }
-        uint32_t j = k >> 2;
         if (G > 1) {
 #pragma unroll 1
             for (; j >= 32; j >>= 1) {
                 const bool low = (t & j) == 0;
-                publish();
+                if (!in_xb) publish();
+                in_xb = false;
 #pragma unroll
                 for (int e = 0; e < E; ++e) {
                     const uint64_t y = xb[e * T + (t ^ j)];
