@@ -105,9 +105,11 @@ int pssgpu_ctx_kernel_stats(pssgpu_ctx* ctx, pssgpu_kernel_stats* out, int max);
  * outputs one GPU thread merges in each round of pssgpu_merge_lcp_device.
  * PSSGPU_OPT_SUFFIX_DOUBLING (default 1): when the strings of a sort are all
  * suffixes of one text (n == nchars, offs[i] == i, no NUL before the last
- * char: psstest --suffix, src/psstest.cpp:502-518), groups that share 8 or
- * more chars are finished by prefix doubling on suffix ranks instead of
- * deeper string passes; the output is the same. 0: sort them as strings. */
+ * char: psstest --suffix, src/psstest.cpp:502-518), the passes read the text
+ * packed at its alphabet's bits per char, and groups that still share a whole
+ * 64-bit key are finished from the ranks of their members' later suffixes
+ * instead of deeper string passes; the output is the same. 0: sort them as
+ * strings. */
 #define PSSGPU_OPT_PROFILE 1
 #define PSSGPU_OPT_INDIRECT_HANDLES 2
 #define PSSGPU_OPT_SINGLE_LAUNCH 3

@@ -1,5 +1,6 @@
 // kernels_block.cuh -- block sample sort for segments of 33..MAXN strings: the
-// last phase of k_wave and the allocation-free entry point.
+// allocation-free entry point, whose one block has no workspace for lists of
+// leftover ties (the leaf sorters of kernels_leaf.cuh hand theirs on).
 //
 // One block runs pS5's sequential sample-sort step (SeqSampleSortStep,
 // src/parallel/bingmann-parallel_sample_sort.hpp:565-676) on its segment in

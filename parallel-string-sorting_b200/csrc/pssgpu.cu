@@ -5,7 +5,8 @@
 // level-synchronous passes: every pass runs one sample-sort step over all
 // segments larger than SMALL_MAX strings (kernels_big.cuh) and finishes all
 // smaller segments in registers (kernels_leaf.cuh).
-// One device-to-host read of the counters per pass sizes the next grids.
+// At the end of a pass k_publish writes the counters to the host's mapped copy,
+// which sizes the next grids.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -242,10 +243,10 @@ struct Ctx {
     // outputs one thread merges in a round of pssgpu_merge_lcp_device (0:
     // chosen per merge, merge_piece_for)
     uint32_t merge_piece = 0;
-    // suffix sets finish their deep groups by rank doubling (off: the string
-    // passes sort them like any strings)
+    // suffix sets sort on packed chars and finish their deep groups from suffix
+    // ranks (off: the string passes sort them like any strings)
     bool suffix_doubling = true;
-    // the list of groups the passes hand to rank doubling (allocated on the
+    // the list of groups the passes hand to run_doubling (allocated on the
     // first suffix-set sort)
     unsigned char* sfx = nullptr;
     uint64_t sfx_bytes = 0;
@@ -1732,6 +1733,8 @@ int pssgpu_sort_text_host(pssgpu_ctx* ctx, const uint8_t* text, uint64_t size, i
 // most MERGE_PIECE, and as few waves of `wave` pieces (the piece-merge
 // threads the GPU holds at once) as that allows, filled evenly, so that no
 // wave runs part-empty; at least MERGE_PIECE_MIN (every piece costs a split).
+// Rounded up to 8 outputs, so that all pieces of a pair start at the same place
+// in a 32-byte output sector: 8 runs of 2 Mi strings 2.30 -> 2.25 ms.
 static uint32_t merge_piece_for(uint64_t n, uint64_t wave)
 {
     const uint64_t per_wave = (uint64_t)MERGE_PIECE * wave;

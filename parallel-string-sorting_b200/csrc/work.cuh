@@ -15,7 +15,7 @@ constexpr int SMALL_THREADS = 256;
 constexpr int WARP_GROUP_MAX = 32;  // groups this small are finished by one warp
 constexpr int FINAL_INLINE = 64;    // equal-string buckets this small are copied inline
 constexpr int CHUNK = 32;           // tiles per chunk of the destination scan
-constexpr uint32_t DBL_MAX = 4096;  // largest group a suffix sort hands to rank doubling
+constexpr uint32_t DBL_MAX = 4096;  // largest group a suffix sort hands to the rounds of kernels_suffix.cuh
 
 // segment list classes
 // (at most 32, 256, 1024 and SMALL_MAX strings; L_BIG above)
@@ -42,9 +42,9 @@ enum : int {
     C_MULTI = 30,     // + parity: big segments of more than CHUNK tiles in the list
     C_DEEP = 32,      // + parity: length of the deep-group list
     C_SFX = 34,       // suffix-set check: nonzero when the input is not all suffixes of a text
-    C_DBL = 35,       // groups handed to rank doubling by the passes
-    C_DBL_CNT = 36,   // + 3 * parity + class: rank-doubling round lists
-    C_DBL_MEMB = 42,  // 64-bit (42, 43): members of the rank-doubling groups, summed over rounds
+    C_DBL = 35,       // suffix groups the passes hand to the rounds of kernels_suffix.cuh
+    C_DBL_CNT = 36,   // + 3 * parity + class: lists of a suffix round
+    C_DBL_MEMB = 42,  // 64-bit (42, 43): members of those groups, summed over rounds
     C_ALPHA = 44,     // suffix-set check: which of the 256 chars occur (8 words)
     C_COUNT = 52
 };
@@ -117,8 +117,8 @@ struct Work {
     // chars numbered from 1 in their order, 0 past the end), so a key holds
     // kchars chars, 21 of a 4-letter text where bytes hold 8, and most
     // suffixes are told apart by their first key. Groups of at most DBL_MAX
-    // that share a key go to the list dbl, which is finished by text rounds
-    // and rank doubling (kernels_suffix.cuh). No LCPs are written before that.
+    // that share a key go to the list dbl, which is finished by the rounds of
+    // kernels_suffix.cuh. No LCPs are written before that.
     // kchars is 8 and kbits 8 otherwise.
     const uint64_t* ptext;
     uint64_t kmask;  // the kchars * kbits top bits
