@@ -56,10 +56,10 @@ __global__ void k_roots(Work w, const uint64_t* __restrict__ inst, uint32_t nins
         if (blockIdx.x == 0 && threadIdx.x == 0) push_seg(w, 0, Seg{0u, w.n, 0u, META_ROOT});
         return;
     }
-    // warp-uniform trips, so that the list appends aggregate per warp
-    for (uint32_t k0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); k0 < ninst;
-         k0 += gridDim.x * blockDim.x) {
-        const uint32_t k = k0 + (threadIdx.x & 31);
+    __shared__ PushBlock sm;
+    // block-uniform trips: the list appends aggregate per block
+    for (uint32_t k0 = blockIdx.x * blockDim.x; k0 < ninst; k0 += gridDim.x * blockDim.x) {
+        const uint32_t k = k0 + threadIdx.x;
         uint32_t b = 0, e = 0;
         if (k < ninst) {
             b = (uint32_t)inst[k];
@@ -69,7 +69,7 @@ __global__ void k_roots(Work w, const uint64_t* __restrict__ inst, uint32_t nins
             if (__ldg(w.offs + b) >= w.nchars) set_error(w.counters + C_ERR, ERR_OFFSET);
             w.perm[b] = w.local ? 0u : b;
         }
-        push_seg_warp(w, 0, e - b >= 2, Seg{b, e - b, 0u, META_ROOT});
+        push_seg_block(w, sm, 0, e - b >= 2, Seg{b, e - b, 0u, META_ROOT});
     }
 }
 
@@ -617,7 +617,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         PSS_CUDA(cudaMemsetAsync(w.counters, 0, 4 * C_COUNT, st));
         kt.begin(K_INIT);
         w.local = d_inst && !lcp && w.packed;
-        k_roots<<<d_inst ? std::max(1u, std::min((ninst + 255) / 256, 148u * 16u)) : 1u, 256, 0, st>>>(
+        k_roots<<<d_inst ? std::max(1u, std::min((ninst + 511) / 512, 148u * 4u)) : 1u, 512, 0, st>>>(
             w, d_inst, ninst);
         // every string a suffix of one text (n == nchars is necessary)?
         if (suffix_try) k_suffix_check<<<1184, 256, 0, st>>>(chars, offs, n, w.counters + C_SFX, w.counters + C_ALPHA);

@@ -308,4 +308,49 @@ __device__ __forceinline__ void push_seg_warp(const Work& w, int nxt, bool push,
     }
 }
 
+// push_seg for a whole block (every thread calls it): one reservation per class
+// and block, for launches whose warps all push to several classes. The roots
+// of a 100k-instance batch: 35 us per warp, 9 per block of 512 (batch 2.005 -> 1.979 ms).
+struct PushBlock {
+    uint32_t count[L_NCLASS], amount[L_NCLASS], base[L_NCLASS], multi;
+};
+__device__ __forceinline__ void push_seg_block(const Work& w, PushBlock& sm, int nxt, bool push, const Seg& c)
+{
+    const uint32_t t = threadIdx.x, lane = t & 31;
+    if (t < (uint32_t)L_NCLASS) sm.count[t] = sm.amount[t] = 0;
+    if (t == 0) sm.multi = 0;
+    __syncthreads();
+    const int cls = push ? seg_class(c.size) : -1;
+    const uint32_t tiles = cls == L_BIG ? seg_tiles(w, c.size) : 0u;
+    uint32_t at = 0;  // in the block's share of the class
+#pragma unroll
+    for (int k = 0; k < L_NCLASS; ++k) {
+        const uint32_t m = __ballot_sync(0xffffffffu, cls == k);
+        if (!m) continue;
+        const int leader = __ffs(m) - 1;
+        const uint32_t amount = __reduce_add_sync(0xffffffffu, cls != k ? 0u : k == L_BIG ? tiles : c.size);
+        uint32_t base = 0;
+        if (lane == (uint32_t)leader) {
+            base = atomicAdd(&sm.count[k], (uint32_t)__popc(m));
+            atomicAdd(&sm.amount[k], amount);
+        }
+        base = __shfl_sync(0xffffffffu, base, leader);
+        if (cls == k) at = base + __popc(m & ((1u << lane) - 1u));
+    }
+    if (tiles > (uint32_t)CHUNK) atomicAdd(&sm.multi, 1u);
+    __syncthreads();
+    if (t < (uint32_t)L_NCLASS && sm.count[t]) {
+        sm.base[t] = atomicAdd(w.counters + C_PAR * nxt + t, sm.count[t]);
+        atomicAdd(w.counters + C_PAR * nxt + (t == L_BIG ? C_NTILES : C_NSTR + t), sm.amount[t]);
+        if (t == L_BIG && sm.multi) atomicAdd(w.counters + C_MULTI + nxt, sm.multi);
+    }
+    __syncthreads();
+    if (push) {
+        at += sm.base[cls];
+        if (at >= w.cap[cls]) set_error(w.counters + C_ERR, ERR_OVERFLOW);
+        else w.list[cls][nxt][at] = c;
+    }
+    __syncthreads();  // sm is free
+}
+
 }  // namespace pssgpu

@@ -141,3 +141,28 @@ def test_pass_loop_tiles(pkg, orc, n):
     finally:
         c.close()
     check(orc, chars, offs, perm, lcp)
+
+
+@pytest.mark.parametrize("ninst", [1, 31, 511, 512, 513, 1025, 310000])
+def test_batch_roots(pkg, ninst):
+    """Root segments of a batch, appended to the lists per block of 512
+    instances and, beyond 592 blocks, by blocks in turn: every size class in
+    one block, the last block part-filled."""
+    rng = np.random.default_rng(ninst)
+    sizes = rng.choice([1, 2, 32, 33, 300, 1500, 5000], ninst) if ninst < 2000 else rng.integers(1, 4, ninst)
+    inst = np.zeros(ninst + 1, dtype=np.uint64)
+    np.cumsum(sizes, out=inst[1:])
+    n = int(inst[-1])
+    text = np.zeros((n, 10), np.uint8)  # distinct: the string's number, shuffled, in base 16
+    number = rng.permutation(n)
+    for j in range(8):
+        text[:, 7 - j] = 97 + ((number >> (4 * j)) & 15)
+    offs = np.arange(n, dtype=np.uint64) * 10
+    c = pkg.Context(0)
+    try:
+        perm, _ = c.sort_batch_host(text.reshape(-1), offs, inst, lcp=False)
+    finally:
+        c.close()
+    of = np.repeat(np.arange(ninst), sizes)
+    want = np.lexsort((number, of)) - inst[of].astype(np.int64)
+    assert np.array_equal(perm.astype(np.int64), want)
