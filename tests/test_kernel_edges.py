@@ -166,3 +166,21 @@ def test_batch_roots(pkg, ninst):
     of = np.repeat(np.arange(ninst), sizes)
     want = np.lexsort((number, of)) - inst[of].astype(np.int64)
     assert np.array_equal(perm.astype(np.int64), want)
+
+
+@pytest.mark.parametrize("with_lcp", [True, False])
+@pytest.mark.parametrize("length", [3, 8, 13])
+def test_equal_buckets(pkg, orc, length, with_lcp):
+    """Equal strings in buckets of their own, of 8 to 40 strings: around the 16
+    that are copied out inline and the 32 of the smallest segments."""
+    rng = np.random.default_rng(length)
+    copies = np.tile(np.arange(8, 41), 50)
+    values = [bytes(rng.integers(97, 123, length).astype(np.uint8)) for _ in copies]
+    strings = [v for v, c in zip(values, copies) for _ in range(c)]
+    chars, offs = pkg.pack_strings([strings[i] for i in rng.permutation(len(strings))])
+    c = pass_loop(pkg)
+    try:
+        perm, lcp = c.sort_host(chars, offs, lcp=with_lcp)
+    finally:
+        c.close()
+    check(orc, chars, offs, perm, lcp if with_lcp else None)
