@@ -123,6 +123,11 @@ int pssgpu_ctx_set_option(pssgpu_ctx* ctx, int option, int64_t value);
  * ends at its first NUL, which must lie inside the arena (chars[nchars-1]
  * must be 0). Outputs: perm[r] = id of the r-th smallest string; lcp (may be
  * NULL) as in the LCP convention above (lcp[0] untouched).
+ * An offset outside the arena, or a last char that is not 0, returns
+ * PSSGPU_EINVAL. The device entry points (pssgpu_sort_device and
+ * pssgpu_sort_batch_device) find either one in the first pass, so after an
+ * error the contents of d_perm and d_lcp are unspecified; the host entry
+ * points leave perm and lcp as they were.
  *
  * pssgpu_sort_host: host buffers; the call copies the arena and offsets to
  * the device, sorts, and copies perm/lcp back. Replaces the body of a

@@ -64,14 +64,41 @@ __device__ __forceinline__ uint64_t load_key(const uint8_t* __restrict__ chars,
     return bswap64(raw);
 }
 
+// What load_raw_chunks reads for cnt windows at position p: 16-byte blocks from
+// the 16-byte boundary at or below chars + p on (an absolute address, so the
+// arena needs no more than its 8-byte alignment), as many as the windows need
+// and only those that hold a char of the arena, which start at positions -15 to
+// nchars - 1. Counted from -15 the test is one unsigned compare, so a string
+// offset outside the arena (it is refused, but only behind the pass that reads
+// it first) leads to no other read, however large it is: a signed test took
+// offsets from 2^63 on for positions in front of the arena.
+struct RawRange {
+    uint64_t at15;  // position of the first block, + 15
+    unsigned need;  // bytes of words used, from there
+    __host__ __device__ __forceinline__ RawRange(uintptr_t chars, uint64_t p, uint32_t cnt)
+    {
+        const unsigned off = (unsigned)(chars + p) & 15u;
+        at15 = ((chars + p) & ~(uintptr_t)15) - chars + 15;
+        need = 8u * ((off >> 3) + cnt + 1);
+    }
+    __host__ __device__ __forceinline__ bool reads(int i, uint64_t nchars) const
+    {
+        return (unsigned)(16 * i) < need && at15 + 16 * i < nchars + 15;
+    }
+    // bytes from such a block's start to the arena's end
+    __host__ __device__ __forceinline__ uint64_t left(int i, uint64_t nchars) const
+    {
+        return nchars + 15 - (at15 + 16 * i);
+    }
+};
+
 // The raw little-endian 8-char windows at p, p + 8, ... (cnt <= NB of them)
 // into raw[0, cnt); raw[cnt, NB) are left 0 and chars at or beyond nchars
 // read as 0. The words come from 16-byte loads at the 16-byte boundary at or
-// below chars + p (an absolute address, so the arena needs no more than its
-// 8-byte alignment): every vector lies in a 16-byte block that holds a char
-// of the arena or of its padding, and at most ceil((NB + 2) / 2) are read,
-// where byte-wise 8-byte loads would take NB + 1 (a string's loads are one
-// L1 request per lane each, which bounds the common-prefix pass). A window
+// below chars + p: every vector lies in a 16-byte block that holds a char of
+// the arena (RawRange), and at most ceil((NB + 2) / 2) are read, where
+// byte-wise 8-byte loads would take NB + 1 (a string's loads are one L1
+// request per lane each, which bounds the common-prefix pass). A window
 // becomes load_key's value through finish_key.
 template <int NB>
 __device__ __forceinline__ void load_raw_chunks(const uint8_t* __restrict__ chars, uint64_t nchars,
@@ -83,18 +110,16 @@ __device__ __forceinline__ void load_raw_chunks(const uint8_t* __restrict__ char
     const unsigned off = (unsigned)(ab - a16);  // 0..15
     const unsigned sh = (off & 7u) * 8u;
     const bool upper = off >= 8;                // the first window starts in the upper word
-    const unsigned need = 8u * ((off >> 3) + cnt + 1);  // bytes of words used, from a16
-    const int64_t base = (int64_t)(a16 - reinterpret_cast<uintptr_t>(chars));
+    const RawRange range(reinterpret_cast<uintptr_t>(chars), p, cnt);
     uint64_t wd[2 * NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-        const int64_t r = base + 16 * i;  // arena position of the vector's first byte
         uint64_t x = 0, y = 0;
-        if ((unsigned)(16 * i) < need && r < (int64_t)nchars) {
+        if (range.reads(i, nchars)) {
             const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(a16 + 16 * i));
             x = v.x;
             y = v.y;
-            const int64_t left = (int64_t)nchars - r;  // its bytes inside the arena
+            const uint64_t left = range.left(i, nchars);
             if (left < 16) {
                 if (left <= 8) {
                     x &= ~0ull >> (64u - 8u * (unsigned)left);

@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1536 / TILE_THREADS) k_classify(
         const uint64_t x = __ldg(hs + p);
         if (!root) return h_off(w, x);
         bad |= x >= w.nchars;
-        return x;
+        return min(x, w.nchars);  // an offset outside the arena reads as an empty string
     };
     for (uint32_t p = lo + threadIdx.x; p < hi; p += TILE_THREADS) {
         uint64_t key = 0;
