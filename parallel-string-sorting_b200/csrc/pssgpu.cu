@@ -450,6 +450,7 @@ static int run_doubling(Ctx* c, Work& w, uint32_t ndbl, uint32_t* lcp, cudaStrea
     };
     auto fetch = [&]() -> int {
         k_publish<<<1, 64, 0, st>>>(w.counters, hc, -1);
+        stats.kernel_launches += 1;
         PSS_CUDA(cudaGetLastError());
         PSS_CUDA(cudaStreamSynchronize(st));
         return PSSGPU_OK;
@@ -622,8 +623,8 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         // every string a suffix of one text (n == nchars is necessary)?
         if (suffix_try) k_suffix_check<<<1184, 256, 0, st>>>(chars, offs, n, w.counters + C_SFX, w.counters + C_ALPHA);
         kt.end(K_INIT);
-        c->kstat[K_INIT].launches += 1;
-        stats.kernel_launches += 1;
+        c->kstat[K_INIT].launches += suffix_try ? 2 : 1;
+        stats.kernel_launches += suffix_try ? 2 : 1;
     }
     if (one || wave) {
         c->kstat[K_WAVE].launches += 1;
@@ -651,7 +652,10 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         }
     } else {
         // the single launches have written the host's counters themselves
-        if (!one && !wave) k_publish<<<1, 64, 0, st>>>(w.counters, hc, -1);
+        if (!one && !wave) {
+            k_publish<<<1, 64, 0, st>>>(w.counters, hc, -1);
+            stats.kernel_launches += 1;
+        }
         PSS_CUDA(cudaStreamSynchronize(st));
         kt.collect();
     }
@@ -819,6 +823,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
             if (joined[q]) PSS_CUDA(cudaStreamWaitEvent(st, c->join_ev[q], 0));
         if (last_is_pass) PSS_CUDA(cudaEventRecord(c->ev1, st));  // the end, when it was this one
         k_publish<<<1, 64, 0, st>>>(w.counters, hc, cur);
+        stats.kernel_launches += 1;
         PSS_CUDA(cudaGetLastError());
         PSS_CUDA(cudaStreamSynchronize(st));
         kt.collect();
@@ -894,6 +899,7 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
     if (more || (npass ? !last_is_pass : !one && !wave)) {
         PSS_CUDA(cudaEventRecord(c->ev1, st));
         k_publish<<<1, 64, 0, st>>>(w.counters, hc, -1);
+        stats.kernel_launches += 1;
         PSS_CUDA(cudaStreamSynchronize(st));
         kt.collect();
     }
