@@ -75,8 +75,11 @@ int pssgpu_ctx_stats(pssgpu_ctx* ctx, pssgpu_stats* out);
 /* Per-kernel-class figures of the last sort: launches, strings processed,
  * algorithmic bytes (per-string model: key gather 4 id + 8 chars + 8 key,
  * classify 8 key, scatter 12 + 12, base case 12 + output) and, in profile
- * mode, summed device time from CUDA events around each class. Returns the
- * number of entries written (at most max), or a negative status. */
+ * mode, summed device time from CUDA events around each class. The last five
+ * entries count, in `launches` alone, parts of "doubling" (the rounds that
+ * finish a suffix set): its chain rounds, its rank rounds, and the launches
+ * that sorted groups of at most 32, 1024 and 4096 suffixes. Returns the number
+ * of entries written (at most max; there are 19), or a negative status. */
 typedef struct pssgpu_kernel_stats {
     char name[16];
     uint32_t launches;

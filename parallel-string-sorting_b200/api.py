@@ -88,8 +88,8 @@ class Context:
         _check(_native.gpu().pssgpu_ctx_set_option(self._h, option, value))
 
     def kernel_stats(self) -> list:
-        arr = (PssKernelStats * 16)()
-        k = _native.gpu().pssgpu_ctx_kernel_stats(self._h, arr, 16)
+        arr = (PssKernelStats * 32)()
+        k = _native.gpu().pssgpu_ctx_kernel_stats(self._h, arr, 32)
         if k < 0:
             _check(-k)
         return [{"name": arr[i].name.decode(), "launches": arr[i].launches,

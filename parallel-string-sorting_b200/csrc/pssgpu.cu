@@ -183,12 +183,16 @@ static uint64_t workspace_bytes(const Sizes& s)
     return b;
 }
 
-// Kernel classes reported by pssgpu_ctx_kernel_stats.
+// Kernel classes reported by pssgpu_ctx_kernel_stats. The ones behind K_DBL
+// count parts of it (KStat::launches only): its chain and rank rounds, and the
+// launches that sorted groups of at most 32, DBL_MID and DBL_MAX members.
 enum KClass { K_INIT = 0, K_SAMPLE, K_CLASSIFY, K_BSTART, K_SCATTER, K_CHILDREN, K_TINY,
-              K_SMALLA, K_SMALLB, K_SMALLC, K_DEEP, K_BOUNDARY, K_WAVE, K_DBL, K_NCLASS };
+              K_SMALLA, K_SMALLB, K_SMALLC, K_DEEP, K_BOUNDARY, K_WAVE, K_DBL,
+              K_CHAINS, K_RANKS, K_GROUPS, K_NCLASS = K_GROUPS + 3 };
 static const char* const kclass_name[K_NCLASS] = {
     "init", "sample", "classify", "bstart", "scatter", "children", "tiny",
-    "small256", "small1024", "small4096", "deep", "boundary", "wave", "doubling"};
+    "small256", "small1024", "small4096", "deep", "boundary", "wave", "doubling",
+    "chain_rounds", "rank_rounds", "groups32", "groups1024", "groups4096"};
 
 struct KStat {
     uint32_t launches = 0;
@@ -411,13 +415,12 @@ static int ensure_buf(unsigned char** buf, uint64_t* have, uint64_t bytes)
     return PSSGPU_OK;
 }
 
-// Finish the ndbl groups the passes handed over (a suffix set): chain rounds
-// while they leave less than three quarters of the groups, then rank
-// doubling; with LCP output, the LCP array.
+// Finish the ndbl groups (at least 1) the passes handed over (a suffix set):
+// chain rounds while they leave less than three quarters of the groups, then
+// rank doubling.
 // Works in the workspace's key, handle and bucket arrays, which the passes no
 // longer need. Caller holds c->mu; *err receives the device error bits.
-static int run_doubling(Ctx* c, Work& w, uint32_t ndbl, uint32_t* lcp, cudaStream_t st, pssgpu_stats& stats,
-                        uint32_t* err)
+static int run_doubling(Ctx* c, Work& w, uint32_t ndbl, cudaStream_t st, pssgpu_stats& stats, uint32_t* err)
 {
     const uint32_t n = w.n;
     const uint64_t capn = c->cap.n;
@@ -458,11 +461,9 @@ static int run_doubling(Ctx* c, Work& w, uint32_t ndbl, uint32_t* lcp, cudaStrea
     int rc, par = 0;
     c->kstat[K_DBL].strings += n;
     PSS_CUDA(cudaMemsetAsync(w.counters + C_DBL_CNT, 0, 4 * (C_DBL_MEMB + 2 - C_DBL_CNT), st));
-    if (ndbl) {
-        PSS_CUDA(cudaMemsetAsync(a.isa, 0xFF, 4ull * n, st));
-        k_dbl_init<<<(ndbl + 255) / 256, 256, 0, st>>>(w, w.dbl, ndbl, a, members);
-        launched(1);
-    }
+    PSS_CUDA(cudaMemsetAsync(a.isa, 0xFF, 4ull * n, st));
+    k_dbl_init<<<(ndbl + 255) / 256, 256, 0, st>>>(w, w.dbl, ndbl, a, members);
+    launched(1);
     if ((rc = fetch())) return rc;
     // the depth of every group at least doubles per rank round (n <= 2^32
     // chars): a loop beyond this many rounds is an internal error
@@ -480,6 +481,8 @@ static int run_doubling(Ctx* c, Work& w, uint32_t ndbl, uint32_t* lcp, cudaStrea
         if (fill) chain = false;
         groups = total;
         const uint32_t classes = (cnt[0] != 0) + (cnt[1] != 0) + (cnt[2] != 0);
+        for (int k = 0; k < 3; ++k) c->kstat[K_GROUPS + k].launches += cnt[k] != 0;
+        c->kstat[chain ? K_CHAINS : K_RANKS].launches += 1;
         if (chain) {
             PSS_CUDA(cudaMemsetAsync(a.chain[0], 0, 4ull * a.clen[0], st));
             for (int k = 0; k < 3; ++k)
@@ -525,17 +528,11 @@ static int run_doubling(Ctx* c, Work& w, uint32_t ndbl, uint32_t* lcp, cudaStrea
         par ^= 1;
     }
     *err = hc[C_ERR];
-    // algorithmic bytes: per group member and round its id and the chars or
-    // the rank `depth` further read, its id and new rank written
+    // algorithmic bytes: per group member handed over, and per member and rank
+    // round, its id and the chars or the rank `depth` further read, its id and
+    // new rank written
     const uint64_t memb = (uint64_t)hc[C_DBL_MEMB] | ((uint64_t)hc[C_DBL_MEMB + 1] << 32);
-    c->kstat[K_DBL].alg_bytes += 16ull * memb + (lcp ? 16ull * n : 0);
-    if (!*err && lcp) {
-        k_dbl_fill<<<1184, 256, 0, st>>>(w.perm, n, a.isa, 1);
-        k_dbl_lcp<<<(unsigned)std::min<uint64_t>(((uint64_t)n + 255) / 256, 148ull * 16), 256, 0, st>>>(
-            w.chars, w.nchars, w.perm, a.isa, lcp, n);
-        launched(2);
-        PSS_CUDA(cudaGetLastError());
-    }
+    c->kstat[K_DBL].alg_bytes += 16ull * memb;
     return PSSGPU_OK;
 }
 
@@ -696,11 +693,11 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         uint64_t* pt = reinterpret_cast<uint64_t*>(c->sfx + 16 * cap);
         w.ptext = pt;
         w.lcp = nullptr;  // the LCPs come last, in text order
-        kt.begin(K_DBL);
+        kt.begin(K_INIT);
         k_pack_text<<<(unsigned)std::min<uint64_t>((words + 255) / 256, 148ull * 16), 256, 0, st>>>(
             chars, nchars, w.kbits, map, pt, words);
-        kt.end(K_DBL);
-        c->kstat[K_DBL].launches += 1;
+        kt.end(K_INIT);
+        c->kstat[K_INIT].launches += 1;
         stats.kernel_launches += 1;
     }
     auto pending = [&]() {
@@ -876,12 +873,26 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         cur = nxt;
     }
     bool more = false;  // steps behind the passes (or the single launch)
-    if (!err && suffix && (hc[C_DBL] || lcp)) {
+    if (!err && suffix && hc[C_DBL]) {
         more = true;
         kt.begin(K_DBL);
-        rc = run_doubling(c, w, std::min(hc[C_DBL], w.dbl_cap), lcp, st, stats, &err);
+        rc = run_doubling(c, w, std::min(hc[C_DBL], w.dbl_cap), st, stats, &err);
         kt.end(K_DBL);
         if (rc) return rc;
+    }
+    if (!err && suffix && lcp) {
+        more = true;
+        // every suffix's position, in the key array that the passes are done with
+        uint32_t* isa = reinterpret_cast<uint32_t*>(w.keys[0]);
+        kt.begin(K_BOUNDARY);
+        k_dbl_fill<<<1184, 256, 0, st>>>(perm, n, isa, 1);
+        k_dbl_lcp<<<(unsigned)std::min<uint64_t>(((uint64_t)n + 255) / 256, 148ull * 16), 256, 0, st>>>(
+            chars, nchars, perm, isa, lcp, n);
+        kt.end(K_BOUNDARY);
+        c->kstat[K_BOUNDARY].launches += 2;
+        c->kstat[K_BOUNDARY].strings += n;
+        c->kstat[K_BOUNDARY].alg_bytes += 16ull * n;
+        stats.kernel_launches += 2;
     }
     if (!err && lcp && hc[C_NBND]) {
         more = true;

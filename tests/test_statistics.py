@@ -24,3 +24,58 @@ def test_kernel_launches_counts_every_kernel(pkg, batch, lcp, single, want):
         assert c.stats()["kernel_launches"] == want
     finally:
         c.close()
+
+
+def suffix_sort_launches(pkg, orc, text):
+    """The launches per kernel class of the sort of all suffixes of a text,
+    whose result is checked."""
+    chars = np.concatenate([text, np.zeros(1, np.uint8)])
+    offs = np.arange(chars.shape[0], dtype=np.uint64)
+    c = pkg.Context(0)
+    try:
+        c.set_option(c.OPT_SINGLE_LAUNCH, 0)
+        perm, lcp = c.sort_host(chars, offs, lcp=True)
+        used = {k["name"]: k["launches"] for k in c.kernel_stats()}
+    finally:
+        c.close()
+    ids, want = orc.sort_ids_lcp(chars, offs)  # suffixes are distinct: one order
+    assert np.array_equal(perm, ids)
+    assert np.array_equal(lcp[1:].astype(np.uint64), want[1:])
+    return used
+
+
+def test_suffix_rounds_by_text(pkg, orc):
+    """Which rounds finish a suffix set: none where all suffixes part within a
+    key, chain rounds alone for copied blocks, rank rounds for a periodic
+    text, whose groups part one member at a time."""
+    rng = np.random.default_rng(5)
+    letters = rng.choice(np.frombuffer(b"ACGT", np.uint8), 6000)
+    used = suffix_sort_launches(pkg, orc, letters)
+    assert used["doubling"] == used["chain_rounds"] == used["rank_rounds"] == 0
+
+    copies = letters.copy()
+    copies[4000:4500] = copies[100:600]
+    used = suffix_sort_launches(pkg, orc, copies)
+    assert used["chain_rounds"] > 0 and used["rank_rounds"] == 0
+    assert used["groups32"] > 0 and used["groups1024"] == used["groups4096"] == 0
+
+    periodic = np.tile(np.frombuffer(b"abcab", np.uint8), 2000)
+    used = suffix_sort_launches(pkg, orc, periodic)
+    assert used["chain_rounds"] > 0 and used["rank_rounds"] > 0 and used["groups4096"] > 0
+
+
+@pytest.mark.parametrize("copies,groups", [(32, "groups32"), (33, "groups1024"), (1024, "groups1024"),
+                                           (1025, "groups4096"), (4000, "groups4096")])
+def test_suffix_group_classes(pkg, orc, copies, groups):
+    """Groups at the edges of the three group sorts: that many copies of one
+    word of 40 letters, each behind and before random ones."""
+    rng = np.random.default_rng(copies)
+    letters = np.frombuffer(b"ACGT", np.uint8)
+    word = rng.choice(letters, 40)
+    text = np.concatenate([x for _ in range(copies) for x in (word, rng.choice(letters, 25))] + [rng.choice(letters, 5000)])
+    used = suffix_sort_launches(pkg, orc, text)
+    assert used[groups] > 0
+    if groups != "groups4096":
+        assert used["groups4096"] == 0
+    if groups == "groups32":
+        assert used["groups1024"] == 0
