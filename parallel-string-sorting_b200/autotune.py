@@ -23,16 +23,18 @@ from . import workloads
 from .api import Context
 
 TABLE_PATH = Path(__file__).resolve().parent / "tuning_b200.json"
-CLASSES = range(10, 21)  # big segments: more than 1024 strings
+LEAF_MAX = 4096  # larger segments are big (SMALL_MAX): only their classes have a tree
+CLASSES = range(12, 21)
 
 
 def _class_batch(k: int, strings: int, seed: int):
-    """Instances of 2^k..2^(k+1)-1 strings, about `strings` in total."""
+    """Instances of 2^k..2^(k+1)-1 strings, more than LEAF_MAX each, about
+    `strings` in total."""
     rng = np.random.default_rng(seed + k)
     sizes = []
     total = 0
     while total < strings:
-        s = int(rng.integers(1 << k, 1 << (k + 1)))
+        s = int(rng.integers(max(1 << k, LEAF_MAX + 1), 1 << (k + 1)))
         sizes.append(s)
         total += s
     inst = np.zeros(len(sizes) + 1, dtype=np.uint64)
