@@ -56,7 +56,7 @@ constexpr int WINDOW_STEPS = 8;
 // the key at mydep when has_key. Returns the handle that sorts into this
 // lane's slot; LCPs inside groups are written to lcp[mypos]. scratch is 32
 // words of shared memory private to the warp.
-// With defer_hnd set (the block sorters), groups that stall on a long common
+// With defer_hnd set (the leaf sorters), groups that stall on a long common
 // prefix are not walked here: their handles go to defer_hnd[mypos] and the
 // group to the deep-group list (segment meta defer_meta), and k_deep finishes
 // them in the next pass, one warp per group, while this block moves on; the
@@ -298,7 +298,7 @@ __device__ __forceinline__ void warp_seg_windows(const Seg* __restrict__ L, uint
     }
 }
 
-// Deep groups handed over by the block sorters: one warp per group, which
+// Deep groups handed over by the leaf sorters: one warp per group, which
 // starts with the common-prefix jump and then sorts the group to the end.
 constexpr int DEEP_WARPS = 8;
 __global__ void __launch_bounds__(32 * DEEP_WARPS) k_deep(Work w, const Seg* list, uint32_t count)

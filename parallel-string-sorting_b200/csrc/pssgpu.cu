@@ -153,7 +153,7 @@ static Sizes sizes_for(uint64_t n)
     s.tile_cap = std::max({s.n >> 13, std::min<uint64_t>(s.n, TILE_MID_N) >> 12,
                            std::min<uint64_t>(s.n, TILE_SMALL_N) >> 11}) + s.cap[L_BIG] + 1;
     // deep groups hold 2..32 strings; a fuller list falls back to walking
-    // the group inside the block sorter
+    // the group inside the leaf sorter
     s.deep_cap = s.n / 32 + 64;
     return s;
 }
@@ -756,8 +756,8 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
             stats.kernel_launches += 1;
         }
         if (ndeep) {
-            // groups the previous pass's block sorters handed over; the same
-            // stream as the block sorters, which add to the other list
+            // groups the previous pass's leaf sorters handed over; the same
+            // stream as k_segs_b, which adds to the other list
             cudaStream_t s = small_stream(2);
             kt.begin(K_DEEP);
             constexpr uint32_t per_block = DEEP_WARPS;
@@ -2105,7 +2105,7 @@ void pssgpu_sort_strings_out(unsigned char** strings, unsigned char** output, si
 // Allocation-free entry point.
 //
 // pssgpu_sort_device_noalloc sorts at most PSSGPU_NOALLOC_MAX_STRINGS strings
-// with the small-segment kernel and allocates nothing. Its scratch -- the
+// with the block sorter (k_block) and allocates nothing. Its scratch -- the
 // string-handle buffer, the one segment descriptor and the counters that
 // kernel uses -- is the file-scope array below (16,608 bytes), which every
 // device that loads this library holds until the process exits. In host code
@@ -2114,6 +2114,8 @@ void pssgpu_sort_strings_out(unsigned char** strings, unsigned char** output, si
 // that device current. Device code may name the array directly
 // (k_noalloc_prep does).
 namespace pssgpu {
+
+static_assert(PSSGPU_NOALLOC_MAX_STRINGS == BLK_N, "one block sorts them");
 
 struct NoAllocScratch {
     uint64_t hnd[PSSGPU_NOALLOC_MAX_STRINGS];
@@ -2166,8 +2168,8 @@ extern "C" int pssgpu_sort_device_noalloc(const uint8_t* d_chars, uint64_t nchar
             void* p = nullptr;
             if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || !p)
                 return fail(PSSGPU_ECUDA, "symbol lookup");
-            if (cudaFuncSetAttribute(K_BLOCK_NOALLOC, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(BlockSmem<2048>)) != cudaSuccess)
+            if (cudaFuncSetAttribute(k_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(BlockSmem)) != cudaSuccess)
                 return fail(PSSGPU_ECUDA, "smem limit");
             g_noalloc_addr[dev] = static_cast<NoAllocScratch*>(p);
         }
@@ -2191,8 +2193,8 @@ extern "C" int pssgpu_sort_device_noalloc(const uint8_t* d_chars, uint64_t nchar
     w.counters = scratch->counters;
     w.cur = 0;
     set_handle_format(w, false);
-    k_noalloc_prep<<<1, SMALL_THREADS, 0, st>>>(w);
-    K_BLOCK_NOALLOC<<<1, 256, sizeof(BlockSmem<2048>), st>>>(w, &scratch->seg);
+    k_noalloc_prep<<<1, BLK_THREADS, 0, st>>>(w);
+    k_block<<<1, BLK_THREADS, sizeof(BlockSmem), st>>>(w, &scratch->seg);
     uint32_t err = 0;
     if (cudaGetLastError() != cudaSuccess ||
         cudaMemcpyAsync(&err, scratch->counters + C_ERR, 4, cudaMemcpyDeviceToHost, st) !=

@@ -11,7 +11,6 @@ constexpr int MAX_TREE_BITS = 10;   // 1023 splitters, 2047 buckets (pS5's Defau
 constexpr int MAX_BKT = 2056;       // bucket slots per big segment: 2047 + the two prefix buckets
 constexpr int JMAX_CHUNKS = 32;     // common-prefix jump of one pass: at most 32 8-byte chunks
 constexpr int SMALL_MAX = 4096;     // largest segment the leaf sorters take
-constexpr int SMALL_THREADS = 256;
 constexpr int WARP_GROUP_MAX = 32;  // groups this small are finished by one warp
 // equal-string buckets this small are copied out by one thread of k_children
 // (1.95 M strings over 4 letters with LCPs: 480 us at 64, 472 at 16, 476 at 4)
@@ -29,9 +28,7 @@ enum : int {
     C_NTILES = 5,     // + C_PAR * parity: tiles of the big list
     C_NSTR = 5,       // + C_PAR * parity + class (1..4): strings in the small lists
     C_NBND = 20,      // boundary list length
-    C_SPARE = 21,
     C_ERR = 22,       // error bits
-    C_SMALLSEGS = 23, // statistics: segments finished by the leaf sorters
     // per-pass statistics, reset every pass
     C_P_BIG = 24,     // strings in big sample-sort segments
     C_P_STALE = 25,   // of those, strings whose key was gathered this pass
@@ -105,7 +102,7 @@ struct Work {
     uint32_t tile_cap;
     uint32_t tshift;        // strings per tile: 2^tshift, at most TILE (tile_shift)
     int cur;               // parity of the lists read in this pass
-    // Deep groups: groups of at most 32 strings that a block sorter's warp
+    // Deep groups: groups of at most 32 strings that a leaf sorter's warp
     // window found stuck on a long common prefix, handed to k_deep (one warp
     // each) in the next pass; double-buffered by pass parity, null when not
     // allocated
