@@ -83,8 +83,8 @@ __global__ void k_tile_scan(Work w, uint32_t nbig)
 // segments and each block's latency is the pass's).
 __global__ void __launch_bounds__(1024) k_sample(Work w)
 {
-    __shared__ uint64_t samp[2 << MAX_TREE_BITS];
-    __shared__ uint64_t shnd[2 << MAX_TREE_BITS];
+    __shared__ uint64_t samp[1 << MAX_TREE_BITS];
+    __shared__ uint64_t shnd[1 << MAX_TREE_BITS];
     __shared__ uint64_t smin, smax;
     __shared__ uint32_t jrun;
     const int s = blockIdx.x;
