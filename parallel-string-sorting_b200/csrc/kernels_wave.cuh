@@ -184,6 +184,35 @@ __device__ __forceinline__ void wave_sort_run(const Work& w, WaveState* ws, Wave
     __syncthreads();
 }
 
+// Phase D: bucket b, of more than `window` strings.
+__device__ __forceinline__ void wave_large_bucket(const Work& w, WaveState* ws, WaveSmem& sm, uint32_t B,
+                                                  uint32_t b, uint64_t* red)
+{
+    const uint32_t P = sm.start[b], c = sm.start[b + 1] - P;
+    const uint64_t s = (b & 1) ? __ldcg(ws->spl + (b >> 1)) : 0ull;
+    const bool equal = (b & 1) && key_terminated(s);
+    if (!equal && c <= (uint32_t)SMALL_MAX) {
+        wave_sort_run(w, ws, sm, B, P, c, red);
+        return;
+    }
+    if (w.lcp) {
+        if (!(b & 1)) {
+            wave_note_run(w, ws, sm.start, B, P, c, red);
+        } else if (threadIdx.x == 0) {  // all of its keys are the splitter
+            ws->bmin[b] = ws->bmax[b] = s;
+            if (P) ws->run[atomicAdd(&ws->nruns, 1u)] = (uint16_t)b;
+        }
+    }
+    if (equal) {
+        for (uint32_t q = threadIdx.x; q < c; q += WAVE_THREADS) {
+            w.perm[P + q] = h_id(w, __ldcg(w.hnd[1] + P + q));
+            if (w.lcp && q) w.lcp[P + q] = lcp_key_depth(s);
+        }
+    } else if (threadIdx.x == 0) {
+        push_seg(w, 1, (b & 1) ? Seg{P, c, 8u, 1u} : Seg{P, c, 0u, 1u | META_VALID});
+    }
+}
+
 // Draw and sort S samples (at most E * WAVE_THREADS) into samp, the same ones
 // in every block.
 template <int E>
@@ -332,22 +361,8 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
 
     // ---- D: buckets over `window` strings, one block each ----------------------
     for (uint32_t b = blockIdx.x; b < B; b += G) {
-        const uint32_t P = sm.start[b], c = sm.start[b + 1] - P;
-        if (c <= window) continue;
-        const uint64_t s = (b & 1) ? __ldcg(ws->spl + (b >> 1)) : 0ull;
-        if ((b & 1) && key_terminated(s)) {
-            if (w.lcp) wave_note_run(w, ws, sm.start, B, P, c, red);
-            for (uint32_t q = threadIdx.x; q < c; q += WAVE_THREADS) {
-                w.perm[P + q] = h_id(w, __ldcg(w.hnd[1] + P + q));
-                if (w.lcp && q) w.lcp[P + q] = lcp_key_depth(s);
-            }
-        } else if (c <= (uint32_t)SMALL_MAX) {
-            wave_sort_run(w, ws, sm, B, P, c, red);
-        } else {
-            if (w.lcp) wave_note_run(w, ws, sm.start, B, P, c, red);
-            if (threadIdx.x == 0)
-                push_seg(w, 1, (b & 1) ? Seg{P, c, 8u, 1u} : Seg{P, c, 0u, 1u | META_VALID});
-        }
+        if (sm.start[b + 1] - sm.start[b] <= window) continue;
+        wave_large_bucket(w, ws, sm, B, b, red);
         __syncthreads();
     }
     // ---- D: windows of small buckets ---------------------------------------
