@@ -19,10 +19,10 @@
 //   D  a dynamic queue of windows of `window` positions: the runs of buckets
 //      of at most `window` strings that start in a window are finished by the
 //      leaf sorter as one segment (sort_segment, the SmallsortJob
-//      counterpart); larger buckets are finished alone (up to SMALL_MAX
-//      strings), copied out when their strings are all equal, or handed to
-//      the level-synchronous passes as a segment (distribute_finished,
-//      hpp:1492-1584). With LCP output a third barrier precedes the LCPs at
+//      counterpart); larger buckets, which come first, are finished alone (up
+//      to SMALL_MAX strings), copied out when their strings are all equal, or
+//      handed to the level-synchronous passes as a segment
+//      (distribute_finished, hpp:1492-1584). With LCP output a third barrier precedes the LCPs at
 //      the first positions of the runs, which come from the neighbouring
 //      buckets' key ranges (sample_sort_lcp, hpp:311-396).
 // Latency-bound: dependent gathers, the sorts' chains and the barriers.
@@ -51,7 +51,7 @@ constexpr uint32_t WAVE_TILE_MAX = (uint32_t)WAVE_THREADS * WAVE_PER;
 // splitters is zeroed by the host before the launch.
 struct WaveState {
     uint32_t bar;        // grid barrier arrivals
-    uint32_t next_task;  // phase-D windows taken
+    uint32_t next_task;  // phase-D tasks taken behind the blocks' first ones
     uint32_t nruns;      // runs recorded (LCP output only)
     uint32_t done;       // blocks that have ended
     uint32_t pad[2];
@@ -359,33 +359,39 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
     if (!wave_barrier(ws, 2, err, limit)) return leave();
     lap(3);
 
-    // ---- D: buckets over `window` strings, one block each ----------------------
-    for (uint32_t b = blockIdx.x; b < B; b += G) {
-        if (sm.start[b + 1] - sm.start[b] <= window) continue;
-        wave_large_bucket(w, ws, sm, B, b, red);
-        __syncthreads();
-    }
-    // ---- D: windows of small buckets ---------------------------------------
+    // ---- D: buckets over `window` strings, then the windows of small buckets ----
+    // One queue, whose first G tasks are the blocks' own: a window's large
+    // bucket (at most one starts in it) is one task, its small buckets another,
+    // behind all the large ones. Large buckets by b modulo G left a block with
+    // four of them while others had none (700 k strings over 2 letters, 256
+    // buckets: 530 us, 234 from the queue).
     const uint32_t ntask = (n + window - 1) / window;
-    while (true) {
+    uint32_t large = 0;  // tasks of large buckets
+    for (uint32_t b = threadIdx.x; b < B; b += WAVE_THREADS)
+        if (sm.start[b + 1] - sm.start[b] > window) large = ntask;
+    if (threadIdx.x == 0) big_at = B;
+    large = __syncthreads_or((int)large) ? ntask : 0u;
+    for (uint32_t t = blockIdx.x; t < large + ntask; t = task) {
+        const uint32_t lo = (t < large ? t : t - large) * window, hi = min(lo + window, n);
+        const uint32_t b_lo = wave_lower(sm.start, B, lo);
+        const uint32_t b_hi = wave_lower(sm.start, B, hi);
+        if (large)
+            for (uint32_t b = b_lo + threadIdx.x; b < b_hi; b += WAVE_THREADS)
+                if (sm.start[b + 1] - sm.start[b] > window) atomicMin(&big_at, b);
+        __syncthreads();
+        const uint32_t bb = min(big_at, b_hi);
+        if (t >= large) {
+            wave_sort_run(w, ws, sm, B, sm.start[b_lo], sm.start[bb] - sm.start[b_lo], red);
+            if (bb < b_hi) wave_sort_run(w, ws, sm, B, sm.start[bb + 1], sm.start[b_hi] - sm.start[bb + 1], red);
+        } else if (bb < b_hi) {
+            wave_large_bucket(w, ws, sm, B, bb, red);
+        }
+        __syncthreads();
         if (threadIdx.x == 0) {
-            task = atomicAdd(&ws->next_task, 1u);
+            task = G + atomicAdd(&ws->next_task, 1u);
             big_at = B;
         }
         __syncthreads();
-        const uint32_t t = task;
-        if (t >= ntask) break;
-        const uint32_t lo = t * window, hi = min(lo + window, n);
-        const uint32_t b_lo = wave_lower(sm.start, B, lo);
-        const uint32_t b_hi = wave_lower(sm.start, B, hi);
-        // at most one bucket over `window` strings starts in a window
-        for (uint32_t b = b_lo + threadIdx.x; b < b_hi; b += WAVE_THREADS)
-            if (sm.start[b + 1] - sm.start[b] > window) atomicMin(&big_at, b);
-        __syncthreads();
-        const uint32_t bb = min(big_at, b_hi);
-        wave_sort_run(w, ws, sm, B, sm.start[b_lo], sm.start[bb] - sm.start[b_lo], red);
-        if (bb < b_hi) wave_sort_run(w, ws, sm, B, sm.start[bb + 1], sm.start[b_hi] - sm.start[bb + 1], red);
-        __syncthreads();  // task and big_at are rewritten next round
     }
     if (!w.lcp) {
         lap(4);
