@@ -147,7 +147,29 @@ __device__ __forceinline__ void dbl_push_warp(DblArrays& a, uint32_t* counters, 
     }
 }
 
-// fn(s, lane, first, step) over the members of a warp's 32 list entries (s
+// A warp's share of a list: `per` consecutive entries, one per lane (at: the
+// first; size 0: none).
+__device__ __forceinline__ Seg dbl_entry(const Seg* __restrict__ list, uint32_t count, uint32_t per, uint32_t* at)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    *at = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per;
+    const uint32_t g = *at + lane;
+    return lane < per && g < count ? list[g] : Seg{0u, 0u, 0u, 0u};
+}
+
+// Entries per warp of a list that may hold groups over 32 members: its warp
+// takes those one after another, so few of them get a warp each (suffixes of a
+// Fibonacci word of 200,000 chars, 89 groups of 2000 on average: 3.80 ms with
+// 32 per warp, 1.24 with one).
+inline uint32_t dbl_per(uint32_t count)
+{
+    uint32_t per = 32;
+    while (per > 1 && count < per * 2368u) per >>= 1;  // 8 warps on each of 2 x 148 blocks
+    return per;
+}
+inline uint32_t dbl_blocks(uint32_t count, uint32_t per) { return (count + 8 * per - 1) / (8 * per); }
+
+// fn(s, lane, first, step) over the members of a warp's list entries (s
 // and its lane): small groups by their own lane (first 0, step 1), larger ones
 // by the whole warp.
 template <typename Fn>
@@ -169,10 +191,10 @@ __device__ __forceinline__ void dbl_each_group(const Seg& s, Fn fn)
 // The groups the passes handed over: their ids into perm (unless they are
 // there), their members' isa, their depths, and the round lists of parity 0.
 __global__ void __launch_bounds__(256) k_dbl_init(Work w, const Seg* __restrict__ list, uint32_t count,
-                                                  DblArrays a, unsigned long long* members)
+                                                  uint32_t per, DblArrays a, unsigned long long* members)
 {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    const Seg s = g < count ? list[g] : Seg{0u, 0u, 0u, 0u};
+    uint32_t at;
+    const Seg s = dbl_entry(list, count, per, &at);
     const uint32_t m = __reduce_add_sync(0xFFFFFFFFu, s.size);
     if ((threadIdx.x & 31) == 0 && m) atomicAdd(members, (unsigned long long)m);
     dbl_each_group(s, [&](const Seg& q, uint32_t, uint32_t first, uint32_t step) {
@@ -194,11 +216,11 @@ __global__ void __launch_bounds__(256) k_dbl_init(Work w, const Seg* __restrict_
 
 // Chain bits of every member: set when the successors of its group's members
 // lie in one group. (Members share a char, so x + 1 is a suffix.)
-__global__ void __launch_bounds__(256) k_dbl_link(const Seg* __restrict__ list, uint32_t count,
+__global__ void __launch_bounds__(256) k_dbl_link(const Seg* __restrict__ list, uint32_t count, uint32_t per,
                                                   const uint32_t* __restrict__ perm, DblArrays a)
 {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    const Seg s = g < count ? list[g] : Seg{0u, 0u, 0u, 0u};
+    uint32_t at;
+    const Seg s = dbl_entry(list, count, per, &at);
     dbl_each_group(s, [&](const Seg& q, uint32_t, uint32_t first, uint32_t step) {
         if (!q.size) return;
         const uint32_t b = a.isa[perm[q.begin] + 1];
@@ -261,11 +283,11 @@ __device__ __forceinline__ uint32_t chain_end(const DblArrays& a, uint32_t x)
 // the ranks dist + 1 chars further, where all have one, else the text at the
 // depth the chain's end shares. isa and gd are read as the last round left
 // them.
-__global__ void __launch_bounds__(256) k_dbl_chain_keys(Seg* __restrict__ list, uint32_t count,
+__global__ void __launch_bounds__(256) k_dbl_chain_keys(Seg* __restrict__ list, uint32_t count, uint32_t per,
                                                         const uint32_t* __restrict__ perm, DblArrays a, int par)
 {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    const Seg s = g < count ? list[g] : Seg{0u, 0u, 0u, 0u};
+    uint32_t at;
+    const Seg s = dbl_entry(list, count, per, &at);
     dbl_each_group(s, [&](const Seg& q, uint32_t f, uint32_t first, uint32_t step) {
         if (!q.size) return;
         const uint32_t x = perm[q.begin];
@@ -281,7 +303,7 @@ __global__ void __launch_bounds__(256) k_dbl_chain_keys(Seg* __restrict__ list, 
         if (first) return;
         const uint32_t b = a.isa[e];
         const uint32_t d = ranks || b == DBL_NONE ? q.depth : max(q.depth, e - x + a.gd[par][b]);
-        list[(g & ~31u) + f] = Seg{q.begin, q.size, ranks ? off : d, ranks ? DBL_BY_RANK : 0u};
+        list[at + f] = Seg{q.begin, q.size, ranks ? off : d, ranks ? DBL_BY_RANK : 0u};
     });
 }
 

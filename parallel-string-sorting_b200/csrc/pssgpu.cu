@@ -462,7 +462,8 @@ static int run_doubling(Ctx* c, Work& w, uint32_t ndbl, cudaStream_t st, pssgpu_
     c->kstat[K_DBL].strings += n;
     PSS_CUDA(cudaMemsetAsync(w.counters + C_DBL_CNT, 0, 4 * (C_DBL_MEMB + 2 - C_DBL_CNT), st));
     PSS_CUDA(cudaMemsetAsync(a.isa, 0xFF, 4ull * n, st));
-    k_dbl_init<<<(ndbl + 255) / 256, 256, 0, st>>>(w, w.dbl, ndbl, a, members);
+    const uint32_t init_per = dbl_per(ndbl);
+    k_dbl_init<<<dbl_blocks(ndbl, init_per), 256, 0, st>>>(w, w.dbl, ndbl, init_per, a, members);
     launched(1);
     if ((rc = fetch())) return rc;
     // the depth of every group at least doubles per rank round (n <= 2^32
@@ -484,16 +485,18 @@ static int run_doubling(Ctx* c, Work& w, uint32_t ndbl, cudaStream_t st, pssgpu_
         for (int k = 0; k < 3; ++k) c->kstat[K_GROUPS + k].launches += cnt[k] != 0;
         c->kstat[chain ? K_CHAINS : K_RANKS].launches += 1;
         if (chain) {
+            uint32_t per[3];
+            for (int k = 0; k < 3; ++k) per[k] = k ? dbl_per(cnt[k]) : 32u;
             PSS_CUDA(cudaMemsetAsync(a.chain[0], 0, 4ull * a.clen[0], st));
             for (int k = 0; k < 3; ++k)
                 if (cnt[k])
-                    k_dbl_link<<<(cnt[k] + 255) / 256, 256, 0, st>>>(a.list[k][par], cnt[k], w.perm, a);
+                    k_dbl_link<<<dbl_blocks(cnt[k], per[k]), 256, 0, st>>>(a.list[k][par], cnt[k], per[k], w.perm, a);
             for (int lv = 1; lv < CHAIN_LEVELS; ++lv)
                 k_chain_level<<<std::min<uint32_t>((a.clen[lv] + 7) / 8, 1184u), 256, 0, st>>>(
                     a.chain[lv - 1], a.clen[lv - 1], a.chain[lv], a.clen[lv]);
             for (int k = 0; k < 3; ++k)
                 if (cnt[k])
-                    k_dbl_chain_keys<<<(cnt[k] + 255) / 256, 256, 0, st>>>(a.list[k][par], cnt[k], w.perm, a, par);
+                    k_dbl_chain_keys<<<dbl_blocks(cnt[k], per[k]), 256, 0, st>>>(a.list[k][par], cnt[k], per[k], w.perm, a, par);
             launched(CHAIN_LEVELS - 1 + 2 * classes);
         } else {
             if (fill) {

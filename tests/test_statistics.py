@@ -79,3 +79,16 @@ def test_suffix_group_classes(pkg, orc, copies, groups):
         assert used["groups4096"] == 0
     if groups == "groups32":
         assert used["groups1024"] == 0
+
+
+@pytest.mark.parametrize("words,copies", [(100, 33), (600, 33), (1500, 40)])
+def test_suffix_many_larger_groups(pkg, orc, words, copies):
+    """Lists of about 2,000, 12,000 and 30,000 groups over 32 members, of which
+    a warp takes one, two and eight."""
+    rng = np.random.default_rng(words)
+    letters = np.frombuffer(b"ACGT", np.uint8)
+    word = rng.choice(letters, (words, 40))
+    text = np.concatenate([np.concatenate([word, rng.choice(letters, (words, 25))], 1).reshape(-1)
+                           for _ in range(copies)])
+    used = suffix_sort_launches(pkg, orc, text)
+    assert used["groups1024"] > 0
