@@ -89,3 +89,39 @@ def test_tiles_in_descending_sizes(pkg, orc, indirect):
                 assert pkg.workloads.check_sorted(chars, chars.shape[0], offs, perm) == -1
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("indirect", [0, 1])
+@pytest.mark.parametrize("width", [7, 8, 9, 31, 32, 39, 40, 41, 100])
+def test_small_segments_behind_whole_keys(pkg, orc, width, indirect):
+    """Instances of 2 to 32 strings that share whole 8-char keys: all equal, in
+    two halves, or apart behind `width` chars, beside instances of random
+    strings (the turns of k_tiny, around their last one)."""
+    rng = np.random.default_rng(width)
+    strings, sizes = [], []
+    for n in list(range(2, 33)) * 3:
+        head = bytes(rng.integers(97, 123, width).astype(np.uint8))
+        kind = int(rng.integers(4))
+        if kind == 0:
+            s = [head] * n
+        elif kind == 1:
+            s = [head] * (n // 2) + [head[:-1] + b"~"] * (n - n // 2)
+        elif kind == 2:
+            s = [head + bytes(rng.integers(97, 100, int(rng.integers(0, 4))).astype(np.uint8)) for _ in range(n)]
+        else:
+            s = [bytes(rng.integers(97, 123, int(rng.integers(0, 12))).astype(np.uint8)) for _ in range(n)]
+        strings += [s[i] for i in rng.permutation(n)]
+        sizes.append(n)
+    chars, offs = pkg.pack_strings(strings)
+    inst = np.zeros(len(sizes) + 1, dtype=np.uint64)
+    np.cumsum(sizes, out=inst[1:])
+    c = pkg.Context(0)
+    try:
+        c.set_option(c.OPT_INDIRECT_HANDLES, indirect)
+        for with_lcp in (True, False):
+            perm, lcp = c.sort_batch_host(chars, offs, inst, lcp=with_lcp)
+            for k in range(len(sizes)):
+                b, e = int(inst[k]), int(inst[k + 1])
+                check(orc, chars, offs[b:e], perm[b:e], lcp[b:e] if with_lcp else None)
+    finally:
+        c.close()
