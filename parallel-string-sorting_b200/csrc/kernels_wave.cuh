@@ -360,31 +360,39 @@ __global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws,
     lap(3);
 
     // ---- D: buckets over `window` strings, then the windows of small buckets ----
-    // One queue, whose first G tasks are the blocks' own: a window's large
-    // bucket (at most one starts in it) is one task, its small buckets another,
-    // behind all the large ones. Large buckets by b modulo G left a block with
-    // four of them while others had none (700 k strings over 2 letters, 256
-    // buckets: 530 us, 234 from the queue).
+    // One queue, whose first G tasks are the blocks' own: the large buckets, then
+    // the windows. Large buckets by b modulo G left a block with four of them
+    // while others had none (700 k strings over 2 letters, 256 buckets: 530 us,
+    // 236 from the queue). They are numbered by the threads that find them, in
+    // every block alike.
     const uint32_t ntask = (n + window - 1) / window;
-    uint32_t large = 0;  // tasks of large buckets
-    for (uint32_t b = threadIdx.x; b < B; b += WAVE_THREADS)
-        if (sm.start[b + 1] - sm.start[b] > window) large = ntask;
+    uint32_t flags = 0;  // bit q: bucket threadIdx.x + q * WAVE_THREADS is large
+    for (uint32_t b = threadIdx.x, q = 0; b < B; b += WAVE_THREADS, ++q)
+        if (sm.start[b + 1] - sm.start[b] > window) flags |= 1u << q;
+    uint32_t large;
+    const uint32_t before = block_excl_sum<WAVE_THREADS>(__popc(flags), tmp, &large);
     if (threadIdx.x == 0) big_at = B;
-    large = __syncthreads_or((int)large) ? ntask : 0u;
+    __syncthreads();
     for (uint32_t t = blockIdx.x; t < large + ntask; t = task) {
-        const uint32_t lo = (t < large ? t : t - large) * window, hi = min(lo + window, n);
-        const uint32_t b_lo = wave_lower(sm.start, B, lo);
-        const uint32_t b_hi = wave_lower(sm.start, B, hi);
-        if (large)
-            for (uint32_t b = b_lo + threadIdx.x; b < b_hi; b += WAVE_THREADS)
-                if (sm.start[b + 1] - sm.start[b] > window) atomicMin(&big_at, b);
-        __syncthreads();
-        const uint32_t bb = min(big_at, b_hi);
-        if (t >= large) {
+        if (t < large) {
+            if (t - before < (uint32_t)__popc(flags)) {
+                uint32_t m = flags;
+                for (uint32_t q = t - before; q; --q) m &= m - 1;
+                big_at = threadIdx.x + (__ffs(m) - 1) * WAVE_THREADS;
+            }
+            __syncthreads();
+            wave_large_bucket(w, ws, sm, B, big_at, red);
+        } else {
+            const uint32_t lo = (t - large) * window, hi = min(lo + window, n);
+            const uint32_t b_lo = wave_lower(sm.start, B, lo);
+            const uint32_t b_hi = wave_lower(sm.start, B, hi);
+            if (large)  // at most one starts in a window
+                for (uint32_t b = b_lo + threadIdx.x; b < b_hi; b += WAVE_THREADS)
+                    if (sm.start[b + 1] - sm.start[b] > window) atomicMin(&big_at, b);
+            __syncthreads();
+            const uint32_t bb = min(big_at, b_hi);
             wave_sort_run(w, ws, sm, B, sm.start[b_lo], sm.start[bb] - sm.start[b_lo], red);
             if (bb < b_hi) wave_sort_run(w, ws, sm, B, sm.start[bb + 1], sm.start[b_hi] - sm.start[bb + 1], red);
-        } else if (bb < b_hi) {
-            wave_large_bucket(w, ws, sm, B, bb, red);
         }
         __syncthreads();
         if (threadIdx.x == 0) {
