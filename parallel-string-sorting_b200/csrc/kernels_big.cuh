@@ -51,6 +51,30 @@ __device__ __forceinline__ uint32_t tree_bits_for(const Work& w, uint32_t m)
     return (uint32_t)min(MAX_TREE_BITS, max(1, lg - 7));
 }
 
+// The levels of a segment whose keys are shared by SHARED_KEY_STRINGS or more
+// strings each: about 8 strings per bucket, so that most of these keys get an
+// '=' bucket of their own, whose strings the leaf sorters read at the next depth
+// at once instead of sorting them by this one first. Its samples show it by
+// repeating; when they repeat much (a third of all neighbours equal), they
+// cover the keys as they are. From 2^21 strings on: a second set of samples is
+// on the pass's path (2 M ACGT strings 450 us without, 470 with). 3 M strings over
+// 2 letters 850 -> 729 us (714 before the leaf sorters), 8 M 1780 -> 1333
+// (1340), 4.2 M over 4 letters 784 -> 677; prefixes, batches and 3 letters as
+// before.
+constexpr uint32_t SHARED_KEY_STRINGS = 24, SHARED_KEY_MIN_N = 1u << 21;
+__device__ __forceinline__ uint32_t tree_bits_fine(const Work& w, uint32_t m)
+{
+    const int lg = 31 - __clz((int)m);
+    return w.n < SHARED_KEY_MIN_N || w.tree_bits_by_size[lg] || w.suffix ? 0u : (uint32_t)min(MAX_TREE_BITS, max(1, lg - 3));
+}
+
+// Position of sample i of a segment.
+__device__ __forceinline__ uint32_t sample_pos(const Seg& sg, uint32_t i)
+{
+    const uint64_t h = mix64(((uint64_t)sg.begin << 32) ^ ((uint64_t)sg.depth << 12) ^ i);
+    return sg.begin + (uint32_t)(((h >> 32) * sg.size) >> 32);
+}
+
 __global__ void k_tile_scan(Work w, uint32_t nbig)
 {
     __shared__ uint32_t tmp[32];
@@ -99,21 +123,19 @@ __global__ void __launch_bounds__(1024) k_sample(Work w)
         }
         return;
     }
-    const uint32_t L = tree_bits_for(w, sg.size);
-    const uint32_t k = (1u << L) - 1;
+    uint32_t L = tree_bits_for(w, sg.size);
     // one sample per bucket slot: 2^L sorted samples, the splitters are all
     // but the first. pS5 oversamples by 2 (hpp:1388); here half the
     // samples halve the bitonic sort, which is most of this kernel's work,
-    // while '<' buckets still hold about 8 strings on average
-    const uint32_t S = 1u << L;
+    // while '<' buckets still hold about 128 strings on average
+    uint32_t S = 1u << L;
     const int buf = sg.meta & META_BUF;
     const bool valid = sg.meta & META_VALID;
     // handles (and cached keys) of the samples, then the keys of stale ones:
     // every load of a round is independent
 #pragma unroll 8
     for (uint32_t i = threadIdx.x; i < S; i += blockDim.x) {
-        const uint64_t h = mix64(((uint64_t)sg.begin << 32) ^ ((uint64_t)sg.depth << 12) ^ i);
-        const uint32_t r = sg.begin + (uint32_t)(((h >> 32) * sg.size) >> 32);
+        const uint32_t r = sample_pos(sg, i);
         shnd[i] = handle_at(w, sg.meta, sg.begin, r);
         if (valid) samp[i] = w.keys[buf][r];
     }
@@ -192,7 +214,27 @@ __global__ void __launch_bounds__(1024) k_sample(Work w)
             samp[i] = h_key(w, shnd[i], sg.depth + K * J);
         __syncthreads();
     }
-    bitonic_sort_block(samp, S);
+    const uint32_t fine = tree_bits_fine(w, sg.size);
+    while (true) {
+        bitonic_sort_block(samp, S);
+        if (L >= fine) break;
+        uint32_t same = 0;  // equal neighbours among the samples
+        for (uint32_t i0 = 0; i0 + 1 < S; i0 += blockDim.x) {
+            const uint32_t i = i0 + threadIdx.x;
+            same += __syncthreads_count(i + 1 < S && samp[i] == samp[i + 1] && !key_ends(w, samp[i]));
+        }
+        // 2 same size / S^2 strings per key, as the samples show it
+        if ((uint64_t)same * sg.size * 2 < (uint64_t)SHARED_KEY_STRINGS * S * S || 3 * same >= S) break;
+        L = fine;
+        S = 1u << L;
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x; i < S; i += blockDim.x) {
+            const uint32_t r = sample_pos(sg, i);
+            samp[i] = valid && !J ? w.keys[buf][r] : h_key(w, handle_at(w, sg.meta, sg.begin, r), sg.depth + K * J);
+        }
+        __syncthreads();
+    }
+    const uint32_t k = (1u << L) - 1;
     if (threadIdx.x == 0) {
         w.jump[s] = K * J;
         atomicAdd(w.counters + C_P_BIG, sg.size);

@@ -63,3 +63,20 @@ def test_copies_in_large_sorts(pkg, orc, n):
     finally:
         c.close()
     check(orc, text.reshape(-1), offs, perm, lcp)
+
+
+@pytest.mark.parametrize("sigma,width,n", [(2, 24, (1 << 21) - 1), (2, 24, 1 << 21), (2, 24, 2800000),
+                                           (4, 20, 3000000), (2, 7, 2200000)])
+def test_shared_keys_in_the_pass_loop(pkg, orc, sigma, width, n):
+    """Segments of few distinct keys, around the size from which they are
+    sampled again for a finer tree; keys that end are not counted."""
+    rng = np.random.default_rng(sigma + width)
+    text = np.zeros((n, width + 1), np.uint8)
+    text[:, :width] = rng.integers(97, 97 + sigma, (n, width))
+    offs = np.arange(n, dtype=np.uint64) * (width + 1)
+    c = pkg.Context(0)
+    try:
+        perm, lcp = c.sort_host(text.reshape(-1), offs, lcp=True)
+    finally:
+        c.close()
+    check(orc, text.reshape(-1), offs, perm, lcp)
