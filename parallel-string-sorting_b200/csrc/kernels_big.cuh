@@ -65,7 +65,8 @@ constexpr uint32_t SHARED_KEY_STRINGS = 24, SHARED_KEY_MIN_N = 1u << 21;
 __device__ __forceinline__ uint32_t tree_bits_fine(const Work& w, uint32_t m)
 {
     const int lg = 31 - __clz((int)m);
-    return w.n < SHARED_KEY_MIN_N || w.tree_bits_by_size[lg] || w.suffix ? 0u : (uint32_t)min(MAX_TREE_BITS, max(1, lg - 3));
+    if (w.n < SHARED_KEY_MIN_N || w.tree_bits_by_size[lg] || w.suffix) return 0;
+    return (uint32_t)min(MAX_TREE_BITS, max(1, lg - 3));
 }
 
 // Position of sample i of a segment.

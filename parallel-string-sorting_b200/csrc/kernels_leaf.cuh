@@ -27,9 +27,11 @@
 // segments of 1025..4096 strings one more sample-sort pass (about 42 ps)
 // before them: 9.29 -> 7.42 ms per sort; 100k-instance batch 3.86 -> 2.48 ms.
 //
-// Strings whose whole words tie and do not end go to warp windows
-// (kernels_small.cuh), up to 32 strings of several groups at a time; larger
-// tied groups are sorted again by their warp, behind their common prefix.
+// Strings whose whole words tie and do not end are sorted on together by their
+// next chars, end as copies of one string (equal_runs), or go to warp windows
+// (kernels_small.cuh), up to 32 strings of several groups at a time, or to the
+// next pass; larger tied groups are sorted again by their warps, behind their
+// common prefix.
 #pragma once
 
 #include <utility>
@@ -40,8 +42,9 @@ namespace pssgpu {
 
 // Order of two 64-bit words. WORD62: both are below 2^62, so that their bits
 // are non-negative finite doubles in the same order, and the compare runs on
-// the FP64 pipe instead of the integer ALU, which bounds the warp sorts (75% busy in k_segs<16>): 1.16 -> 1.07 ms for the 27.7 M strings that
-// kernel sorts of the 100k-instance batch.
+// the FP64 pipe instead of the integer ALU, which bounds the warp sorts (75%
+// busy in k_segs<16>): 1.16 -> 1.07 ms for the 27.7 M strings that kernel sorts
+// of the 100k-instance batch.
 template <bool WORD62>
 __device__ __forceinline__ bool word_less(uint64_t a, uint64_t b)
 {
@@ -357,6 +360,9 @@ struct TinyWarp {
 // The warp's segments, one per lane (sg.size 0: none; packed from lane
 // `first` on), `total` strings from row entries `off`; N the network. Sorts
 // and writes them.
+// Segments of equal strings (META_FINAL, 17..32 of them from k_children) need no
+// case of their own: their depth is the strings' length and no key is cached,
+// so every key reads the NUL, 0, all tie, and the LCPs are the depth.
 template <int N, bool SFX>
 __device__ __forceinline__ void tiny_warp_sort(const Work& w, TinyWarp& sm, Seg sg, uint32_t first,
                                                uint32_t off, uint32_t total)
@@ -426,7 +432,6 @@ __device__ __forceinline__ void tiny_warp_sort(const Work& w, TinyWarp& sm, Seg 
         }
         __syncwarp();
     }
-    const uint64_t key0 = key[0];
     const int cp = __clzll((long long)(diff | 1));  // equal keys: any shift does
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -505,7 +510,8 @@ __device__ __forceinline__ void tiny_warp_sort(const Work& w, TinyWarp& sm, Seg 
             push_dbl_warp(w, has, Seg{sg.begin + start, len, sg.depth + w.kchars, META_PERM});
             has = has && next_run(start, len);
         }
-    } else
+        return;
+    }
     tie_windows(
         sm.scratch, next_run,
         [&](uint32_t owner, uint32_t start, uint32_t gs) {
@@ -708,7 +714,7 @@ __device__ __forceinline__ uint32_t sort_group(const Work& w, SegState<G>& sm, u
             for (uint32_t j = t; j < c; j += T) w.perm[begin + s + j] = h_id(w, sm.hnd[sm.idx[idx_at(s + j)]]);
             if (t == 0) push_dbl(w, Seg{begin + s, c, d + w.kchars, META_PERM});
             return 0;
-        } else {
+        }
         if (key_terminated(key0)) {  // all equal: any order
             for (uint32_t j = t; j < c; j += T) {
                 w.perm[begin + s + j] = h_id(w, sm.hnd[sm.idx[idx_at(s + j)]]);
@@ -730,7 +736,6 @@ __device__ __forceinline__ uint32_t sort_group(const Work& w, SegState<G>& sm, u
             sm.g_dep[at] = d + 8u * sm.jump;
         }
         return 0;
-        }
     }
     const WordForm<IB, SFX> form(w, key0, diff);
 #pragma unroll
@@ -989,8 +994,9 @@ __device__ __forceinline__ bool equal_runs(const Work& w, SegState<G>& sm, uint3
 }
 
 // The nt ties left in the group of c strings at offset s, whose runs share
-// `dep` chars: to the list dbl (a suffix set), to the next pass when there are many, else runs of up to 32
-// strings to warp windows and longer ones to the stack.
+// `dep` chars: to the list dbl (a suffix set), to the next pass when there are
+// many, else runs of up to 32 strings to warp windows and longer ones to the
+// stack.
 template <int G, bool SFX>
 __device__ __forceinline__ void finish_ties(const Work& w, SegState<G>& sm, uint32_t begin, int buf, uint32_t s,
                                             uint32_t c, uint32_t dep, uint32_t nt)
@@ -1038,7 +1044,8 @@ __device__ __forceinline__ void finish_ties(const Work& w, SegState<G>& sm, uint
             push_dbl_warp(w, has, Seg{begin + s + start, len, dep, META_PERM});
             has = has && next_run(start, len);
         }
-    } else {
+        return;
+    }
     if (pass_on) {
         // the next pass sorts the runs as segments of their own size, from the
         // segment's handles in the order reached here
@@ -1059,7 +1066,6 @@ __device__ __forceinline__ void finish_ties(const Work& w, SegState<G>& sm, uint
         const uint64_t r = warp_window(w, h, gs, dep, begin + q, false, 0ull, sm.scratch[warp], defer, (uint32_t)buf);
         if (real) w.perm[begin + q] = h_id(w, r);
     });
-    }
 }
 
 // Sort the segment of m strings at position begin by its group of G warps:
@@ -1098,7 +1104,8 @@ __device__ __forceinline__ void sort_segment(const Work& w, SegState<G>& sm, uns
             if (!chars) {
                 uint32_t k2 = k;
                 const bool copies = k <= runs * (uint32_t)WARP_GROUP_MAX;
-                for (int q = 0; copies && q < LEAF_EQUAL_TURNS && nt && equal_runs<G>(w, sm, begin, s, k2, dep, &nt); ++q) {
+                for (int q = 0; copies && q < LEAF_EQUAL_TURNS && nt; ++q) {
+                    if (!equal_runs<G>(w, sm, begin, s, k2, dep, &nt)) break;
                     dep += 32;
                     if (nt) k2 = collect_ties<G>(sm, c, &runs);
                 }

@@ -236,8 +236,9 @@ __device__ __forceinline__ void wave_samples(const Work& w, uint32_t S, uint64_t
 // L: levels of the splitter tree, over: samples per splitter (1 or 2).
 // w.cur must be 0: the wave's leftovers (big segments, tied runs, deep
 // groups) go to the lists of parity 1, with their strings in buffer 1.
-__global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws, uint32_t L, uint32_t over, uint32_t window,
-                                                          uint32_t limit, int trace, uint32_t* host_counters)
+__global__ void __launch_bounds__(WAVE_THREADS, 2) k_wave(Work w, WaveState* ws, uint32_t L, uint32_t over,
+                                                          uint32_t window, uint32_t limit, int trace,
+                                                          uint32_t* host_counters)
 {
     long long cl = clock64();
     auto lap = [&](int k) {  // phase k ended here (tracing only)

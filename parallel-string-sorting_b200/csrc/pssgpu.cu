@@ -76,16 +76,16 @@ __global__ void k_roots(Work w, const uint64_t* __restrict__ inst, uint32_t nins
 // The end of a pass of parity cur (-1: of another step): the counters go to
 // the host's copy (mapped memory), and those that the next pass appends to
 // start at 0. One small launch instead of a copy and four memsets, whose gaps
-// are idle time between passes (2 M strings with LCPs: 510 -> 477 us, 613-instance batch
-// 465 -> 440).
+// are idle time between passes (2 M strings with LCPs: 510 -> 477 us,
+// 613-instance batch 465 -> 440).
 __global__ void k_publish(uint32_t* __restrict__ counters, uint32_t* host, int cur)
 {
     const uint32_t t = threadIdx.x;
     if (t >= (uint32_t)C_COUNT) return;
     host[t] = counters[t];
     const bool stat = t >= (uint32_t)C_P_FIRST && t <= (uint32_t)C_P_LAST;
-    if (cur >= 0 && (t / C_PAR == (uint32_t)cur || t == (uint32_t)(C_MULTI + cur) || t == (uint32_t)(C_DEEP + cur) || stat))
-        counters[t] = 0;
+    const bool of_pass = t / C_PAR == (uint32_t)cur || t == (uint32_t)(C_MULTI + cur) || t == (uint32_t)(C_DEEP + cur);
+    if (cur >= 0 && (of_pass || stat)) counters[t] = 0;
 }
 
 // Batch output: ids relative to their instance; the first LCP of every
@@ -496,7 +496,8 @@ static int run_doubling(Ctx* c, Work& w, uint32_t ndbl, cudaStream_t st, pssgpu_
                     a.chain[lv - 1], a.clen[lv - 1], a.chain[lv], a.clen[lv]);
             for (int k = 0; k < 3; ++k)
                 if (cnt[k])
-                    k_dbl_chain_keys<<<dbl_blocks(cnt[k], per[k]), 256, 0, st>>>(a.list[k][par], cnt[k], per[k], w.perm, a, par);
+                    k_dbl_chain_keys<<<dbl_blocks(cnt[k], per[k]), 256, 0, st>>>(a.list[k][par], cnt[k], per[k],
+                                                                                 w.perm, a, par);
             launched(CHAIN_LEVELS - 1 + 2 * classes);
         } else {
             if (fill) {
@@ -621,7 +622,8 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         k_roots<<<d_inst ? std::max(1u, std::min((ninst + 511) / 512, 148u * 4u)) : 1u, 512, 0, st>>>(
             w, d_inst, ninst);
         // every string a suffix of one text (n == nchars is necessary)?
-        if (suffix_try) k_suffix_check<<<1184, 256, 0, st>>>(chars, offs, n, w.counters + C_SFX, w.counters + C_ALPHA);
+        if (suffix_try)
+            k_suffix_check<<<1184, 256, 0, st>>>(chars, offs, n, w.counters + C_SFX, w.counters + C_ALPHA);
         kt.end(K_INIT);
         c->kstat[K_INIT].launches += suffix_try ? 2 : 1;
         stats.kernel_launches += suffix_try ? 2 : 1;
@@ -706,9 +708,10 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
     auto pending = [&]() {
         return cnt[L_BIG] || cnt[L_TINY] || cnt[L_SMALLA] || cnt[L_SMALLB] || cnt[L_SMALLC] || ndeep;
     };
-    // Every pass takes each open segment at least 8 chars deeper or splits
-    // it; the limit turns a pass structure that stops making progress into
-    // an error instead of an endless loop.
+    // Every pass splits each open segment or takes it at least 4 chars deeper
+    // (tied runs of the leaf sorters; 8 for a tie of whole keys); the limit
+    // turns a pass structure that stops making progress into an error instead
+    // of an endless loop.
     constexpr uint32_t MAX_PASSES = 1u << 20;
     const bool last_is_pass = !lcp && !suffix && (!d_inst || w.local);  // nothing comes behind the passes
     uint32_t npass = 0;
@@ -734,7 +737,8 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         if (cnt[L_SMALLC]) {
             cudaStream_t s = small_stream(3);
             kt.begin(K_SMALLC);
-            (suffix ? k_segs_c<true> : k_segs_c<false>)<<<cnt[L_SMALLC], 512, segs_smem<16>(1, true), s>>>(w, w.list[L_SMALLC][cur], cnt[L_SMALLC]);
+            (suffix ? k_segs_c<true> : k_segs_c<false>)<<<cnt[L_SMALLC], 512, segs_smem<16>(1, true), s>>>(
+                w, w.list[L_SMALLC][cur], cnt[L_SMALLC]);
             kt.end(K_SMALLC);
             c->kstat[K_SMALLC].launches += 1;
             stats.kernel_launches += 1;
@@ -743,7 +747,8 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
             cudaStream_t s = small_stream(0);
             kt.begin(K_TINY);
             const uint32_t per = tiny_per(cnt[L_TINY]), per_block = per * (TINY_THREADS / 32);
-            (suffix ? k_tiny<true> : k_tiny<false>)<<<(cnt[L_TINY] + per_block - 1) / per_block, TINY_THREADS, TINY_SMEM, s>>>(
+            const uint32_t blocks = (cnt[L_TINY] + per_block - 1) / per_block;
+            (suffix ? k_tiny<true> : k_tiny<false>)<<<blocks, TINY_THREADS, TINY_SMEM, s>>>(
                 w, w.list[L_TINY][cur], cnt[L_TINY], per);
             kt.end(K_TINY);
             c->kstat[K_TINY].launches += 1;
@@ -752,8 +757,10 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         if (cnt[L_SMALLA]) {
             cudaStream_t s = small_stream(1);
             kt.begin(K_SMALLA);
-            (suffix ? k_segs_a<true> : k_segs_a<false>)<<<(cnt[L_SMALLA] + SEGS_A_WARPS - 1) / SEGS_A_WARPS, 32 * SEGS_A_WARPS,
-                       segs_smem<1>(SEGS_A_WARPS, w.lcp != nullptr), s>>>(w, w.list[L_SMALLA][cur], cnt[L_SMALLA]);
+            const uint32_t blocks = (cnt[L_SMALLA] + SEGS_A_WARPS - 1) / SEGS_A_WARPS;
+            const size_t smem = segs_smem<1>(SEGS_A_WARPS, w.lcp != nullptr);
+            (suffix ? k_segs_a<true> : k_segs_a<false>)<<<blocks, 32 * SEGS_A_WARPS, smem, s>>>(
+                w, w.list[L_SMALLA][cur], cnt[L_SMALLA]);
             kt.end(K_SMALLA);
             c->kstat[K_SMALLA].launches += 1;
             stats.kernel_launches += 1;
@@ -773,7 +780,8 @@ static int run_sort(Ctx* c, const uint8_t* chars, uint64_t nchars, const uint64_
         if (cnt[L_SMALLB]) {
             cudaStream_t s = small_stream(2);
             kt.begin(K_SMALLB);
-            (suffix ? k_segs_b<true> : k_segs_b<false>)<<<cnt[L_SMALLB], 128, segs_smem<4>(1, true), s>>>(w, w.list[L_SMALLB][cur], cnt[L_SMALLB]);
+            (suffix ? k_segs_b<true> : k_segs_b<false>)<<<cnt[L_SMALLB], 128, segs_smem<4>(1, true), s>>>(
+                w, w.list[L_SMALLB][cur], cnt[L_SMALLB]);
             kt.end(K_SMALLB);
             c->kstat[K_SMALLB].launches += 1;
             stats.kernel_launches += 1;

@@ -13,7 +13,8 @@ constexpr int JMAX_CHUNKS = 32;     // common-prefix jump of one pass: at most 3
 constexpr int SMALL_MAX = 4096;     // largest segment the leaf sorters take
 constexpr int WARP_GROUP_MAX = 32;  // groups this small are finished by one warp
 // equal-string buckets this small are copied out by one thread of k_children
-// (1.95 M strings over 4 letters with LCPs: 480 us at 64, 472 at 16, 476 at 4)
+// (1.95 M strings over 4 letters with LCPs: 480 us at 64, 472 at 16, 476 at 4);
+// larger ones become META_FINAL segments, whose depth is the strings' length
 constexpr int FINAL_INLINE = 16;
 constexpr int CHUNK = 32;           // tiles per chunk of the destination scan
 constexpr uint32_t DBL_MAX = 4096;  // largest group a suffix sort hands to the rounds of kernels_suffix.cuh
@@ -141,9 +142,13 @@ __host__ __device__ __forceinline__ uint32_t seg_tiles(const Work& w, uint32_t s
 
 // Strings per tile in a sort of n: fewer where 8192 would leave a thread 16
 // strings to gather one after another while SMs idle, or one wave of tiles
-// just over full (classify 53 -> 26 us for 143 tiles; 1.3 M strings 326 -> 303 us,
-// 4.2 M prefix strings 909 -> 875 with 4096); 8192 where tiles are plenty, as every
-// tile pays for its buckets (5 M suffixes 940 us with 8192, 948 with 4096).
+// just over full (classify 53 -> 26 us for 143 tiles; 1.3 M strings 326 -> 303
+// us); 8192 where tiles are plenty, as every tile pays for its buckets. With
+// 8192 and with 4096, in us, of 2, 4, 6, 8 and 12 Mi strings: prefixes 702 / 678,
+// 918 / 892, 1118 / 1100, 1314 / 1298, 1722 / 1736 (24 Mi: 2946 / 3067);
+// letters 335 / 340, 495 / 499, 634 / 653, 773 / 799; suffixes 498 / 496, 718 /
+// 727, 8 Mi 1093 / 1124, 16 Mi 1774 / 1856. The line lies where the one's gain
+// is 3% and the other's loss 1%; beyond it the loss grows.
 constexpr uint64_t TILE_MID_N = 9u << 19, TILE_SMALL_N = 1u << 19;
 __host__ __device__ constexpr uint32_t tile_shift(uint64_t n)
 {
