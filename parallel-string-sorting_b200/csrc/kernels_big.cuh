@@ -56,12 +56,13 @@ __device__ __forceinline__ uint32_t tree_bits_for(const Work& w, uint32_t m)
 // '=' bucket of their own, whose strings the leaf sorters read at the next depth
 // at once instead of sorting them by this one first. Its samples show it by
 // repeating; when they repeat much (a third of all neighbours equal), they
-// cover the keys as they are. From 2^21 strings on: a second set of samples is
-// on the pass's path (2 M ACGT strings 450 us without, 470 with). 3 M strings over
-// 2 letters 850 -> 729 us (714 before the leaf sorters), 8 M 1780 -> 1333
-// (1340), 4.2 M over 4 letters 784 -> 677; prefixes, batches and 3 letters as
-// before.
-constexpr uint32_t SHARED_KEY_STRINGS = 24, SHARED_KEY_MIN_N = 1u << 21;
+// cover the keys as they are. From 2.6 M strings on: a second set of samples is
+// on the pass's path (ACGT strings of up to 64 chars: 2.2 M 475 us without, 486
+// with; 2.8 M 576 / 551; 3.4 M 667 / 592). 3 M strings over 2 letters 850 -> 729
+// us (714 before the leaf sorters), 8 M 1780 -> 1333 (1340), 4.2 M over 4
+// letters 784 -> 677; prefixes, batches and 3 letters as before, random letters
+// 0.6% slower (looking at the samples).
+constexpr uint32_t SHARED_KEY_STRINGS = 24, SHARED_KEY_MIN_N = 5u << 19;
 __device__ __forceinline__ uint32_t tree_bits_fine(const Work& w, uint32_t m)
 {
     const int lg = 31 - __clz((int)m);

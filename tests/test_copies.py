@@ -65,8 +65,8 @@ def test_copies_in_large_sorts(pkg, orc, n):
     check(orc, text.reshape(-1), offs, perm, lcp)
 
 
-@pytest.mark.parametrize("sigma,width,n", [(2, 24, (1 << 21) - 1), (2, 24, 1 << 21), (2, 24, 2800000),
-                                           (4, 20, 3000000), (2, 7, 2200000)])
+@pytest.mark.parametrize("sigma,width,n", [(2, 24, (5 << 19) - 1), (2, 24, 5 << 19), (2, 24, 3200000),
+                                           (4, 20, 3000000), (2, 7, 2700000)])
 def test_shared_keys_in_the_pass_loop(pkg, orc, sigma, width, n):
     """Segments of few distinct keys, around the size from which they are
     sampled again for a finer tree; keys that end are not counted."""
